@@ -127,6 +127,7 @@ void release_pack_buffers(brr_ctx &c)
     drop_dev(c.d_eps);
     drop_dev(c.d_eps_hi);
     drop_dev(c.d_eps_lo);
+    drop_dev(c.d_emax);
     drop_host(c.h_order);
     drop_host(c.h_stats);
     drop_host(c.h_part);
@@ -179,6 +180,15 @@ void free_all(brr_ctx *c)
     cudaFree(c->d_gstage);
     cudaFree(c->d_brec);
     cudaFree(c->d_bdf);
+    cudaFree(c->d_rrec);
+    cudaFree(c->d_rnz);
+    cudaFree(c->d_psum);
+    cudaFree(c->d_rgram);
+    cudaFree(c->d_num);
+    cudaFree(c->d_emax);
+    cudaFree(c->d_eps2);
+    cudaFree(c->d_eps_hi2);
+    cudaFree(c->d_eps_lo2);
     cudaFreeHost(c->h_order);
     cudaFreeHost(c->h_stats);
     cudaFreeHost(c->h_part);
@@ -340,6 +350,81 @@ int build_ragged_lists(brr_ctx &c)
 
 }  // namespace
 
+// Whether the whole-round sweep fits this chain's slices at its round width
+// (the widest that does when none was asked for), and whether FP32C chains can
+// take pair-resolved rounds.
+void brr::choose_round(brr_ctx &c)
+{
+    const brr_config &cf = c.cfg;
+    SweepArgs a{};
+    a.n_groups = cf.n_groups;
+    a.slice_max = c.slice_max;
+    a.cluster = cf.cluster > 0 && c.G > 1 ? c.G : 0;
+    a.rmode = kRoundPairs;
+    a.has_missing = 1;
+    const int asked = cf.spec_width || cf.async_batch ? c.B : (cf.form == BRR_FORM_FP64 ? 64 : 32);
+    c.round_ok = false;
+    for (int B = asked; B >= 8 && !c.round_ok && !c.no_round; B /= 2) {
+        a.B = B;
+        const size_t smem = round_smem_bytes(a);
+        const int fit = smem <= kMaxRoundSmem ? round_fits(c.G, smem, a.cluster > 0) : 0;
+        c.round_ok = a.cluster > 0 ? fit >= 1 : (int64_t)fit * c.sms >= c.G;
+        c.RB = B;
+        if (cf.spec_width || cf.async_batch)
+            break;
+    }
+    c.pair_rounds = cf.form == BRR_FORM_FP32C && !c.eigen && c.round_ok && c.RB <= 32 && cf.pair_rounds >= 0 &&
+                    a.cluster == 0 && cf.async_batch == 0 && cf.N < (1 << 24);
+}
+
+namespace {
+
+// Buffers of the whole-round sweep; without memory for the pair products the
+// FP64 form ends its rounds at their first change.
+int prepare_round(brr_ctx *c)
+{
+    if (!c->use_round())
+        return BRR_OK;
+    const brr_config &cf = c->cfg;
+    const size_t N = (size_t)cf.N, M = (size_t)cf.M;
+    if (!c->d_rrec && (dalloc(&c->d_rrec, M) != cudaSuccess || dalloc(&c->d_rnz, (M + 255) / 256 * 8 + 2) != cudaSuccess || dalloc(&c->d_num, M) != cudaSuccess ||
+                       (cf.form == BRR_FORM_FP64
+                            ? dalloc(&c->d_eps2, N) != cudaSuccess
+                            : dalloc(&c->d_eps_hi2, N) != cudaSuccess || dalloc(&c->d_eps_lo2, N) != cudaSuccess))) {
+        cudaGetLastError();
+        drop_dev(c->d_rrec);
+        drop_dev(c->d_rnz);
+        drop_dev(c->d_num);
+        drop_dev(c->d_eps2);
+        drop_dev(c->d_eps_hi2);
+        drop_dev(c->d_eps_lo2);
+        c->round_ok = false;   // the restart sweep needs no more memory
+        c->pair_rounds = false;
+        return BRR_OK;
+    }
+    if (cf.async_batch > 0 || (cf.form == BRR_FORM_FP32C && !c->pair_rounds && !c->always_pairs))
+        return BRR_OK;
+    size_t words = 0, doubles = 0;
+    round_pair_sizes(cf.M, c->RB, round_pair_modes(c->kind, c->eigen ? 1 : 0, c->has_missing ? 1 : 0), &words, &doubles);
+    if (words > c->psum_words || doubles > c->rgram_doubles) {
+        drop_dev(c->d_psum);
+        drop_dev(c->d_rgram);
+        c->psum_words = c->rgram_doubles = 0;
+        if (dalloc(&c->d_psum, words) != cudaSuccess || dalloc(&c->d_rgram, doubles) != cudaSuccess) {
+            cudaGetLastError();
+            drop_dev(c->d_psum);
+            drop_dev(c->d_rgram);
+            c->pair_rounds = false;
+            return BRR_OK;
+        }
+        c->psum_words = words;
+        c->rgram_doubles = doubles;
+    }
+    return BRR_OK;
+}
+
+}  // namespace
+
 // New slicing (G CTAs) and round width B of a packed chain; the residual and
 // the chain state are per individual and marker, so they carry over.
 int brr::reslice(brr_ctx *c, int G, int B)
@@ -367,7 +452,8 @@ int brr::reslice(brr_ctx *c, int G, int B)
             return rc;
     }
     BRR_CUDA(cudaStreamSynchronize(c->st));
-    return BRR_OK;
+    choose_round(*c);
+    return c->inited ? prepare_round(c) : BRR_OK;
 }
 
 // The sampler constants of the current sigmaE, sigmaG and pi into the pinned
@@ -381,6 +467,38 @@ void brr::sweep_stage(brr_ctx *c)
     std::memcpy(c->h_gK, gK.data(), sizeof(int32_t) * gK.size());
 }
 
+// FP32C sweeps choose between pair-resolved rounds and rounds that end at their
+// first change by the chain's state after the last sweep (a deterministic
+// function of the chain, which keeps it reproducible): a pair-resolved sweep
+// also forms the pair products of its rounds, a restart sweep pays one round
+// per residual-changing marker.
+static bool use_pair_rounds(const brr_ctx *c)
+{
+    if (!c->pair_rounds || c->blocked)
+        return false;
+    if (c->cfg.pair_rounds > 0)
+        return true;
+    return c->kind != BRR_KIND_DENSE && (c->last_nnz < 0 || c->last_nnz * 40 > c->cfg.M);
+}
+
+// How the whole-round sweep ends its rounds.
+static RoundMode round_mode(const brr_ctx *c)
+{
+    if (c->cfg.async_batch > 0)
+        return kRoundAsync;
+    if (c->cfg.form == BRR_FORM_FP64 || c->always_pairs)
+        return c->d_rgram ? kRoundPairs : kRoundRestart;
+    return use_pair_rounds(c) ? kRoundPairs : kRoundRestart;
+}
+
+// Whether a sweep forms the pair products of every marker of a round or only of
+// those sure or likely to change (a change without them ends its round, about one
+// round in forty): all of them while their sums take a fraction of the sweep.
+static int round_all_rows(const brr_ctx *c)
+{
+    return (double)c->cfg.N * (double)c->cfg.M < 5e8 ? 1 : 0;
+}
+
 // Device work before the sweep, on stream st: the staged constants, the records
 // in sweep order (order in d_order, draws in d_u/d_z), cleared accumulators.
 int brr::sweep_enqueue_inputs(brr_ctx *c, double eps_total, cudaStream_t st)
@@ -389,34 +507,36 @@ int brr::sweep_enqueue_inputs(brr_ctx *c, double eps_total, cudaStream_t st)
     const size_t ng = (size_t)cf.n_groups;
     BRR_CUDA(cudaMemcpyAsync(c->d_gconst, c->h_gc, sizeof(double) * ng * kMaxK * 4, cudaMemcpyHostToDevice, st));
     BRR_CUDA(cudaMemcpyAsync(c->d_gK, c->h_gK, sizeof(int32_t) * ng, cudaMemcpyHostToDevice, st));
-    if (c->blocked)
+    if (c->use_round()) {
+        int kmax = 0;
+        for (int g = 0; g < cf.n_groups; ++g)
+            kmax = std::max(kmax, cf.K[g]);
+        // num of a marker without effect has variance about (N - 1) sigmaE: 2.5
+        // standard deviations
+        const float likely = (float)(6.25 * (double)cf.N * c->sigmaE);
+        BRR_CUDA(launch_round_gather(c->d_order, cf.M, cf.N, c->kind, kmax, c->d_table, c->d_scale, c->d_counts, c->d_beta,
+                                     c->d_u, c->d_z, c->d_group, c->d_gconst, c->d_gK, likely, c->d_rrec,
+                                     c->d_rnz, st));
+        if (round_mode(c) == kRoundPairs)
+            BRR_CUDA(launch_round_pairs(c->d_order, cf.M, cf.N, c->RB, c->kind, c->eigen ? 1 : 0,
+                                        c->has_missing ? 1 : 0, c->d_codes, c->col_stride, c->d_table, c->d_scale,
+                                        c->d_counts, c->d_rnz, round_all_rows(c), c->d_psum, c->d_rgram, c->sms, st));
+    } else if (c->blocked)
         BRR_CUDA(launch_gather_block(c->d_order, cf.M, cf.N, c->d_table, c->d_scale, c->d_beta, c->d_u, c->d_z,
                                      c->d_group, eps_total, c->d_brec, st));
     else
         BRR_CUDA(launch_gather(cf.form, c->kind, c->d_order, cf.M, c->d_table, c->d_scale, c->d_beta, c->d_u,
                                c->d_z, c->d_group, c->d_colsum, c->d_rec, st));
+    return sweep_reset(c, st);
+}
+
+// Clears the sweep's accumulators, barrier counters and status, on stream st.
+int brr::sweep_reset(brr_ctx *c, cudaStream_t st)
+{
     BRR_CUDA(cudaMemsetAsync(c->d_acc, 0, sizeof(unsigned long long) * (kAccWords + kCounterWords), st));
     BRR_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
     BRR_CUDA(cudaMemsetAsync(c->d_prof, 0, sizeof(long long) * 16, st));
     return BRR_OK;
-}
-
-// Pair-resolved rounds pay a fixed cost per round of 32 markers; restart
-// rounds pay one round per residual-changing marker.  Measured on ragged
-// markers (N = 20,000, M = 50,000) the pair-resolved sweep is faster while more
-// than about one marker in forty carries a non-zero effect, so the choice
-// follows the chain's state after the last sweep (a deterministic function of
-// the chain, which keeps it reproducible).  Dense pair terms (population counts
-// over every code word of the slice for each pair) grow with the square of the
-// round width and cost more than the dot products on large slices, so dense
-// markers take them only when asked (pair_rounds = 1, as every kind does).
-static bool use_pair_rounds(const brr_ctx *c)
-{
-    if (!c->pair_rounds || c->blocked)
-        return false;
-    if (c->cfg.pair_rounds > 0)
-        return true;
-    return c->kind != BRR_KIND_DENSE && (c->last_nnz < 0 || c->last_nnz * 40 > c->cfg.M);
 }
 
 // The sweep kernel's arguments and shared memory.
@@ -467,8 +587,7 @@ void brr::sweep_args(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, 
     a.tline = c->profile && c->timeline && c->G <= c->sms ? c->d_tline : nullptr;
     a.async_batch = cf.async_batch;
     a.cluster = cf.cluster > 0 && c->G > 1 ? c->G : 0;
-    a.pairs = use_pair_rounds(c) ? c->d_acc + kPairOffset : nullptr;
-    c->last_pair = a.pairs != nullptr;
+    c->last_pair = cf.form == BRR_FORM_FP32C && use_pair_rounds(c);
     a.timeout_ns = c->wait_limit_ns;
     a.phantom = c->phantom;
     a.gram = c->d_gram;
@@ -478,6 +597,25 @@ void brr::sweep_args(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, 
     a.order = c->d_order;
     a.beta_df = c->d_bdf;
     a.acum_df = c->d_bdf ? c->d_bdf + cf.M : nullptr;
+    a.form = cf.form;
+    a.rkind = c->kind;
+    if (c->use_round()) {
+        a.B = c->RB;
+        a.rmode = round_mode(c);
+        a.n_emax = kPartBlocks;
+        a.emax = c->d_emax;
+        a.rrec = c->d_rrec;
+        a.rgram = c->d_rgram;
+        a.rnz = c->d_rnz;
+        a.rall = round_all_rows(c);
+        a.u = c->d_u;
+        a.num_out = c->d_num;
+        a.eps_out = c->d_eps2;
+        a.eps_hi_out = c->d_eps_hi2;
+        a.eps_lo_out = c->d_eps_lo2;
+        smem = round_smem_bytes(a);
+        return;
+    }
     smem = c->blocked ? sweep_block_smem_bytes(a) : sweep_smem_bytes(cf.form, c->kind, a);
 }
 
@@ -541,6 +679,11 @@ int brr::sweep_collect(brr_ctx *c, brr_sweep_out *out)
     out->eps_sum = s1;
     out->eps_sqnorm = s2;
     out->rounds = rounds;
+    if (c->use_round()) {
+        std::swap(c->d_eps, c->d_eps2);
+        std::swap(c->d_eps_hi, c->d_eps_hi2);
+        std::swap(c->d_eps_lo, c->d_eps_lo2);
+    }
     if (c->kind == BRR_KIND_RAGGED)
         c->epsSum = c->h_stats[0];
     c->sweeps += 1;
@@ -563,6 +706,28 @@ int brr::sweep_finish(brr_ctx *c, brr_sweep_out *out)
     return sweep_collect(c, out);
 }
 
+// The whole-round sweep of the prepared inputs and its statistics.  A residual
+// that outgrows its fixed-point grid leaves the buffers of the last sweep as
+// they were (the records hold the old effects), and the sweep runs again on a
+// grid 12 bits coarser, four times at most.
+int brr::round_sweep(brr_ctx *c, SweepArgs a, size_t smem, brr_sweep_out *out)
+{
+    for (;;) {
+        BRR_CUDA(launch_round(a, smem, c->st));
+        BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
+        if (a.async_batch == 0)
+            BRR_CUDA(launch_round_finish(a.M, a.form, a.kmax, c->d_num, c->d_u, c->d_group, c->d_gconst, c->d_gK,
+                                         c->d_acum, c->st));
+        const int rc = sweep_finish(c, out);
+        if (rc != BRR_ERR_RANGE || a.headroom >= 48)
+            return rc;
+        a.headroom += 12;
+        const int rr = sweep_reset(c, c->st);
+        if (rr)
+            return rr;
+    }
+}
+
 namespace {
 
 // One sweep over the order already in d_order with draws in d_u/d_z.
@@ -571,9 +736,17 @@ int run_sweep(brr_ctx *c, double mu_new, double eps_total, brr_sweep_out *out, f
     const brr_config &cf = c->cfg;
     SweepArgs a{};
     size_t smem = 0;
+    BRR_CUDA(cudaEventRecord(c->ev[0], c->st));
     int rc = sweep_prepare(c, mu_new, eps_total, a, smem);
     if (rc)
         return rc;
+    if (c->use_round()) {
+        rc = round_sweep(c, a, smem, out);
+        if (rc)
+            return rc;
+        BRR_CUDA(cudaEventElapsedTime(sweep_ms, c->ev[0], c->ev[1]));
+        return BRR_OK;
+    }
     BRR_CUDA(cudaEventRecord(c->ev[0], c->st));
     if (c->blocked)
         BRR_CUDA(launch_sweep_block(a, smem, c->st));
@@ -767,7 +940,7 @@ int brr::iter_pre_dev(brr_ctx &c, uint32_t it)
         if (rc)
             return rc;
     }
-    BRR_CUDA(launch_mu_prep(cf.form, cf.N, c.mu, c.d_eps, c.d_eps_hi, c.d_eps_lo, c.d_part, kPartBlocks, c.st));
+    BRR_CUDA(launch_mu_prep(cf.form, cf.N, c.mu, c.d_eps, c.d_eps_hi, c.d_eps_lo, c.d_part, c.d_emax, kPartBlocks, c.st));
     if (cf.kind == BRR_KIND_DENSE)
         BRR_CUDA(cudaMemcpyAsync(c.h_part, c.d_part, sizeof(double) * kPartBlocks, cudaMemcpyDeviceToHost, c.st));
     return BRR_OK;
@@ -956,7 +1129,7 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
             dalloc(&c.d_stats, (size_t)cf.n_groups * kMaxK + cf.n_groups + 1) ||
             dalloc(&c.d_part, (size_t)std::max(2 * c.G, kPartBlocks)) || dalloc(&c.d_err, 1) ||
             dalloc(&c.d_rounds, 1) || dalloc(&c.d_prof, 16) || dalloc(&c.d_gstage, sweep_block_stage_bytes(kMaxSpec) / sizeof(double)) || dalloc(&c.d_group, (size_t)M) || dalloc(&c.d_ystd, (size_t)cf.N) ||
-            dalloc(&c.d_nzj, (size_t)M) || dalloc(&c.d_nzb, (size_t)M)) {
+            dalloc(&c.d_nzj, (size_t)M) || dalloc(&c.d_nzb, (size_t)M) || dalloc(&c.d_emax, (size_t)kPartBlocks)) {
             release_pack_buffers(c);
             return fail(BRR_ERR_OOM, "device allocation failed");
         }
@@ -1023,6 +1196,13 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
             return rc;
     }
     BRR_CUDA(cudaStreamSynchronize(c.st));
+    if (c.always_pairs) {
+        choose_round(c);
+        if (!c.round_ok)
+            return fail(BRR_ERR_ARG, "the sweep kernel does not fit " + std::to_string(c.G) + " co-resident CTAs");
+        c.packed = true;
+        return BRR_OK;
+    }
     // the sweep kernel must fit one CTA per slice on the GPU at once
     SweepArgs a{};
     a.B = c.B;
@@ -1030,24 +1210,12 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
     a.slice_max = c.slice_max;
     a.slot_bytes = c.slot_bytes;
     a.cluster = cf.cluster > 0 && c.G > 1 ? c.G : 0;
-    // FP32C restart sweeps resolve whole rounds with pair terms when the round
-    // is one warp wide and the slice's code map or masks fit beside the ring
-    c.pair_rounds = cf.form == BRR_FORM_FP32C && !c.eigen && c.B <= 32 && cf.pair_rounds >= 0 && a.cluster == 0 &&
-                    cf.async_batch == 0 && cf.N < (1 << 24);
-    if (c.pair_rounds) {
-        a.pairs = c.d_acc + kPairOffset;
-        const size_t sp = sweep_smem_bytes(cf.form, c.kind, a);
-        const int per = sp <= (size_t)200 * 1024 ? sweep_max_ctas_per_sm(cf.form, c.kind, sp, true) : 0;
-        if (per < 1 || (int64_t)per * c.sms < c.G) {
-            c.pair_rounds = false;
-            a.pairs = nullptr;
-        }
-    }
     const size_t smem = sweep_smem_bytes(cf.form, c.kind, a);
     if (a.cluster > 0) {
         if (sweep_cluster_fits(cf.form, c.kind, c.G, smem) < 1)
             return fail(BRR_ERR_ARG, "a cluster of " + std::to_string(c.G) + " CTAs with " + std::to_string(smem) +
                                          " bytes of shared memory each cannot be scheduled");
+        choose_round(c);
         c.packed = true;
         return BRR_OK;
     }
@@ -1055,6 +1223,7 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
     if (per_sm < 1 || (int64_t)per_sm * c.sms < c.G)
         return fail(BRR_ERR_ARG, "the sweep kernel does not fit " + std::to_string(c.G) +
                                      " co-resident CTAs (shared memory " + std::to_string(smem) + " bytes)");
+    choose_round(c);
     c.packed = true;
     return BRR_OK;
 }
@@ -1174,6 +1343,8 @@ int brr_init_chain(brr_ctx *ctx)
     if (rc)
         return rc;
     rc = prepare_blocked(&c);
+    if (!rc)
+        rc = prepare_round(&c);
     if (rc)
         return rc;
     c.iteration = 0;
@@ -1239,9 +1410,9 @@ int brr_sweep(brr_ctx *ctx, const uint32_t *order, const double *u, const double
     BRR_CUDA(cudaEventRecord(c.ev[2], c.st));
     std::memset(c.phase, 0, sizeof(c.phase));
     double esum = 0.0;
-    if (c.cfg.kind == BRR_KIND_DENSE) {
-        // current residual total (adding zero leaves the residual unchanged)
-        BRR_CUDA(launch_mu_prep(c.cfg.form, c.cfg.N, 0.0, c.d_eps, c.d_eps_hi, c.d_eps_lo, c.d_part, kPartBlocks, c.st));
+    if (c.cfg.kind == BRR_KIND_DENSE || c.use_round()) {
+        // current residual total and magnitude (adding zero leaves the residual unchanged)
+        BRR_CUDA(launch_mu_prep(c.cfg.form, c.cfg.N, 0.0, c.d_eps, c.d_eps_hi, c.d_eps_lo, c.d_part, c.d_emax, kPartBlocks, c.st));
         BRR_CUDA(cudaMemcpyAsync(c.h_part, c.d_part, sizeof(double) * kPartBlocks, cudaMemcpyDeviceToHost, c.st));
         BRR_CUDA(cudaStreamSynchronize(c.st));
         for (int b = 0; b < kPartBlocks; ++b)
@@ -1308,7 +1479,9 @@ int brr_set_state(brr_ctx *ctx, const brr_state *st)
     std::memcpy(c.pi, st->pi, sizeof(c.pi));
     c.iteration = st->iteration;
     c.last_nnz = -1;
-    const int rb = prepare_blocked(&c);
+    int rb = prepare_blocked(&c);
+    if (!rb)
+        rb = prepare_round(&c);
     if (rb)
         return rb;
     c.inited = true;

@@ -60,8 +60,22 @@ struct brr_ctx {
     brr::BlockRec *d_brec = nullptr;         // blocked FP32C: records in sweep order
     float2 *d_bdf = nullptr;            // blocked FP32C: [2][M] new beta, acum (double-float)
     bool blocked = false;
-    bool pair_rounds = false;   // FP32C restart sweep: pair-resolved rounds available (pair terms in
-                                // d_acc + kPairOffset)
+    // whole-round sweep (brr_round.cu): taken by every chain it fits but the Gram-blocked ones
+    bool round_ok = false;
+    bool no_round = false;              // an instance of a multi-instance run on the restart sweep
+    bool always_pairs = false;          // an instance of a multi-instance run: pair-resolved rounds in every form
+    int RB = 64;                        // markers per round
+    brr::RoundRec *d_rrec = nullptr;    // records in sweep order
+    uint32_t *d_rnz = nullptr;          // one bit per sweep position: old effect not zero
+    int *d_psum = nullptr;              // integer pair sums of a sweep's rounds
+    double *d_rgram = nullptr;          // pair products of a sweep's rounds
+    size_t psum_words = 0, rgram_doubles = 0;
+    double *d_num = nullptr;            // the num every marker was decided on
+    double *d_emax = nullptr;           // [kPartBlocks] partial maxima of |eps|
+    double *d_eps2 = nullptr;           // the residual a sweep writes, swapped with d_eps when it ended well
+    float *d_eps_hi2 = nullptr, *d_eps_lo2 = nullptr;
+    bool use_round() const { return round_ok && !blocked; }
+    bool pair_rounds = false;   // FP32C without the marker Gram: pair-resolved rounds available
     bool last_pair = false;     // the last sweep took pair-resolved rounds
     int gram_bits = 0;          // element bits of the marker Gram's GEMM operands (FP4, FP8 or BF16)
     int64_t last_nnz = -1;      // markers in a non-zero component after the last sweep (-1: not known)
@@ -111,10 +125,7 @@ namespace brr {
 
 constexpr size_t kAccWords = 8 * 8 * kMaxSpec * 4;
 constexpr size_t kCounterWords = 2 * 8 * 16;
-// The restart sweep's accumulators take the first 3 x kMaxSpec x 4 words; the
-// pair terms of pair-resolved rounds (3 x 2048 words) follow.
-constexpr size_t kPairOffset = 4096;
-static_assert(kPairOffset + 3 * 2048 <= kAccWords, "pair terms must fit the accumulator block");
+constexpr size_t kMaxRoundSmem = 220 * 1024;   // dynamic shared memory of the whole-round sweep, beside its static arrays
 constexpr int kPartBlocks = 608;   // 4 x 152 SMs for the updateMu reduction
 
 // Phases of one iteration of a chain (BayesRBase::runGibbs loop body,
@@ -137,10 +148,13 @@ int sweep_prepare(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, siz
 void sweep_stage(brr_ctx *c);
 int sweep_enqueue_inputs(brr_ctx *c, double eps_total, cudaStream_t st);
 void sweep_args(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, size_t &smem);
+int sweep_reset(brr_ctx *c, cudaStream_t st);
 int sweep_finish(brr_ctx *c, brr_sweep_out *out);
 int sweep_enqueue_outputs(brr_ctx *c, cudaStream_t st);
 int sweep_collect(brr_ctx *c, brr_sweep_out *out);
 int iter_post(brr_ctx &c, const brr_sweep_out &so, uint32_t it);
+void choose_round(brr_ctx &c);
+int round_sweep(brr_ctx *c, SweepArgs a, size_t smem, brr_sweep_out *out);
 // New slicing (G CTAs) and, if B > 0, round width of a packed chain.
 int reslice(brr_ctx *c, int G, int B);
 

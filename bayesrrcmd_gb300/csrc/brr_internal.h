@@ -50,6 +50,29 @@ struct alignas(16) BlockRec {
 };
 static_assert(sizeof(BlockRec) == 128, "BlockRec must be 128 bytes");
 
+// Record of the whole-round sweep (brr_round.cu, k_round_gather), in sweep order:
+// num = c + s S + am Sm + at T with S the sum of genotype x residual, Sm the residual
+// over the missing genotypes and T the residual total (dense) or the running sum
+// (sparse kinds); c = beta_old (N - 1).
+struct alignas(16) RoundRec {
+    double s;            // dense: sigma; sparse kinds: 1 / sd
+    double m;            // dense: column mean; sparse kinds: mean
+    double x;            // dense: value of a missing genotype; sparse kinds: Zsum
+    double beta_old, z;
+    float sf[2], atf[2], cf[2], amf[2];   // s, at, c, am as float pairs
+    float uf;            // u rounded to FP32 (certified samplers)
+    float s0;            // num^2 up to which component 0 is certain (negative: never)
+    uint32_t j;
+    uint32_t gm;         // group, and the missing count << 8
+    uint32_t n2, n1;     // individuals with genotype 2 and 1
+};
+static_assert(sizeof(RoundRec) == 96, "RoundRec must be 96 bytes");
+
+// How a round of the whole-round sweep ends: at its first change (the next
+// round starts after it), with every marker resolved through the pair
+// products, or with every marker decided on the residual before the round.
+enum RoundMode { kRoundRestart = 0, kRoundPairs = 1, kRoundAsync = 2 };
+
 struct SweepArgs {
     int64_t N, M;
     int G;                       // CTAs (slices of individuals)
@@ -97,11 +120,23 @@ struct SweepArgs {
     int async_batch;             // restart sweep: 0 synchronous; T > 0 asynchronous batches of T markers
     int cluster;                 // restart sweep: 0 grid-wide exchange; G: the G CTAs are one thread-block
                                  // cluster exchanging through distributed shared memory
-    unsigned long long *pairs;   // pair-resolved ragged rounds: [3][32][32] integer pair terms of the
-                                 // round's markers, A in the low and Bm in the high word (zero at
-                                 // launch), else null
     unsigned long long *tline;   // blocked sweep, counting variant, optional: per-CTA event timeline
                                  // [kTimelineIters][G][kTimelineEvents] of global-timer stamps (ns)
+    // whole-round sweep (brr_round.cu)
+    int form;                    // BRR_FORM_*: how the residual is stored between sweeps
+    int rkind;                   // BRR_KIND_DENSE, or any other value for the sparse kinds
+    int rmode;                   // RoundMode
+    int headroom;                // bits of headroom of the fixed-point residual beyond the default 3
+    int n_emax;
+    const double *emax;          // [n_emax] partial maxima of |eps| before mu_new is subtracted
+    const RoundRec *rrec;        // M records in sweep order
+    const double *rgram;         // [blocks of B][B (B-1) / 2] pair products in sweep order (pairs only)
+    const double *u;             // M: the markers' uniforms, by marker id
+    const uint32_t *rnz;         // one bit per sweep position: the marker is sure or likely to change
+    int rall;                    // the products of every row are formed, not only those of rnz
+    double *num_out;             // M: the num each marker was decided on
+    double *eps_out;             // the residual after the sweep (not the input buffers)
+    float *eps_hi_out, *eps_lo_out;
 };
 // Event timeline of the counting variant of the blocked sweep: iterations
 // nblk/2 - 32 .. nblk/2 + 31 (or all, fewer blocks), per CTA: 0 the others'
@@ -206,6 +241,8 @@ struct MultiSweepArgs {
 };
 int sweep_multi_max_ctas_per_sm(int form, int kmax, size_t smem);
 size_t sweep_multi_static_smem(int form, int kmax);
+int round_multi_ctas_per_sm(int kmax, size_t smem);
+cudaError_t launch_round_multi(int kmax, const MultiSweepArgs &m, size_t smem, cudaStream_t st);
 cudaError_t launch_sweep_multi(int form, int kmax, const MultiSweepArgs &m, size_t smem, cudaStream_t st);
 
 // Kernel launchers (defined in brr_pack.cu / brr_sweep.cu).
@@ -230,7 +267,7 @@ cudaError_t launch_gather(int form, int kind, const uint32_t *order, int64_t M, 
 cudaError_t launch_sweep_stats(int64_t M, const int32_t *group, const int32_t *comp, const uint8_t *chosen,
                                const double *beta, int n_groups, unsigned long long *out, cudaStream_t st);
 cudaError_t launch_mu_prep(int form, int64_t N, double mu_old, double *eps, float *eps_hi,
-                           float *eps_lo, double *part, int nblocks, cudaStream_t st);
+                           float *eps_lo, double *part, double *emax, int nblocks, cudaStream_t st);
 cudaError_t launch_refresh(int form, int kind, int64_t N, const double *ystd, double mu,
                            const uint8_t *codes, int64_t col_stride, const double *table,
                            const uint32_t *nz_j, const double *nz_beta, int64_t n_nz, double *eps,
@@ -247,9 +284,27 @@ bool noalloc_check_output(int dev, const void *d_out, size_t bytes, std::string 
 // Whether p is device or managed memory of device dev with `bytes` bytes to the
 // end of its allocation (no allocation, no launch); the message names `name`.
 bool device_range_check(int dev, const void *p, size_t bytes, const char *name, std::string &why);
-int sweep_max_ctas_per_sm(int form, int kind, size_t smem, bool pair_rounds = false);
+int sweep_max_ctas_per_sm(int form, int kind, size_t smem);
 // Clusters of G CTAs of the cluster sweep that can be resident at once (0: none).
 int sweep_cluster_fits(int form, int kind, int G, size_t smem);
+// Whole-round sweep (brr_round.cu).
+size_t round_smem_bytes(const SweepArgs &a);
+int round_fits(int G, size_t smem, bool cluster);
+cudaError_t launch_round(const SweepArgs &a, size_t smem, cudaStream_t st);
+// nz: room for M bits rounded up to 256.
+cudaError_t launch_round_gather(const uint32_t *order, int64_t M, int64_t N, int kind, int kmax, const double *table,
+                                const double *scale, const int64_t *counts, const double *beta, const double *u,
+                                const double *z, const int32_t *group, const double *gconst, const int32_t *gK,
+                                float likely, RoundRec *rec, uint32_t *nz, cudaStream_t st);
+// Integer pair sums (modes products, see k_pair_sums) and pair products of every round.
+int round_pair_modes(int kind, int eigen, int missing);
+void round_pair_sizes(int64_t M, int B, int modes, size_t *sum_words, size_t *gram_doubles);
+cudaError_t launch_round_pairs(const uint32_t *order, int64_t M, int64_t N, int B, int kind, int eigen, int missing,
+                               const uint8_t *codes, int64_t col_stride, const double *table, const double *scale,
+                               const int64_t *counts, const uint32_t *nz, int all, int *sums, double *gram, int sms,
+                               cudaStream_t st);
+cudaError_t launch_round_finish(int64_t M, int form, int kmax, const double *num, const double *u, const int32_t *group,
+                                const double *gconst, const int32_t *gK, double *acum, cudaStream_t st);
 size_t sweep_block_smem_bytes(const SweepArgs &a);
 cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, const double *table,
                                 const double *scale, const double *beta, const double *u, const double *z,

@@ -42,6 +42,7 @@ constexpr int kChunkInd = 64;   // individuals per slice chunk (16 bytes of code
 
 struct brr_multi {
     int n = 0, form = 0, dev = 0, sms = 0, kmax = 2;
+    bool round = false;                      // the whole-round sweep (every instance's slices fit it)
     size_t smem_limit = 0;
     cudaStream_t st = nullptr;
     cudaEvent_t ev[4] = {};
@@ -78,8 +79,9 @@ void free_multi(brr_multi *m)
         cudaStreamDestroy(m->st);
 }
 
-// Shared memory of an instance's sweep over G slices with round width B.
-size_t inst_smem(const brr_ctx *c, int G, int B)
+// Shared memory of an instance's sweep over G slices with round width B: the
+// whole-round sweep, or the restart sweep.
+size_t inst_smem(const brr_ctx *c, int G, int B, bool round)
 {
     const int64_t chunks = (c->cfg.N + kChunkInd - 1) / kChunkInd;
     const int64_t maxch = (chunks + G - 1) / G;
@@ -88,15 +90,20 @@ size_t inst_smem(const brr_ctx *c, int G, int B)
     a.n_groups = c->cfg.n_groups;
     a.slice_max = (int)(maxch * kChunkInd);
     a.slot_bytes = (int)(maxch * 16);
+    if (round) {
+        a.rmode = kRoundPairs;
+        a.has_missing = 1;
+        return round_smem_bytes(a);
+    }
     return sweep_smem_bytes(c->cfg.form, c->kind, a);
 }
 
 // Fewest CTAs whose slices fit the shared memory limit (0: none does).
-int min_ctas(const brr_ctx *c, int B, size_t limit)
+int min_ctas(const brr_ctx *c, int B, size_t limit, bool round)
 {
     const int64_t chunks = (c->cfg.N + kChunkInd - 1) / kChunkInd;
     for (int G = 1; G <= chunks && G <= 4096; ++G)
-        if (inst_smem(c, G, B) <= limit && (c->kind != BRR_KIND_RAGGED || (chunks + G - 1) / G * kChunkInd <= 65536))
+        if (inst_smem(c, G, B, round) <= limit && (c->kind != BRR_KIND_RAGGED || (chunks + G - 1) / G * kChunkInd <= 65536))
             return G;
     return 0;
 }
@@ -182,7 +189,8 @@ int run_iteration(brr_multi *m)
         ma.inst[i] = args[i];
     }
     // occupancy check; also sets the kernel's shared-memory attribute outside the capture
-    const int per_sm = sweep_multi_max_ctas_per_sm(m->form, m->kmax, smem);
+    const int per_sm = m->round ? round_multi_ctas_per_sm(m->kmax, smem)
+                                : sweep_multi_max_ctas_per_sm(m->form, m->kmax, smem);
     if (per_sm < 1 || (int64_t)per_sm * m->sms < ma.cta_start[n])
         return api_fail(BRR_ERR_ARG, "the instances need " + std::to_string(ma.cta_start[n]) +
                                          " co-resident CTAs with " + std::to_string(smem) + " bytes of shared memory");
@@ -195,7 +203,13 @@ int run_iteration(brr_multi *m)
         if (rc)
             return abandon_capture(m, rc);
     }
-    cudaError_t e = launch_sweep_multi(m->form, m->kmax, ma, smem, m->st);
+    cudaError_t e = m->round ? launch_round_multi(m->kmax, ma, smem, m->st)
+                             : launch_sweep_multi(m->form, m->kmax, ma, smem, m->st);
+    for (int i = 0; m->round && i < n && e == cudaSuccess; ++i) {
+        const brr_ctx &c = *m->inst[i];
+        e = launch_round_finish(c.cfg.M, c.cfg.form, args[i].kmax, c.d_num, c.d_u, c.d_group, c.d_gconst, c.d_gK,
+                                c.d_acum, m->st);
+    }
     if (e != cudaSuccess)
         return abandon_capture(m, api_fail(BRR_ERR_CUDA, std::string("multi-instance sweep: ") + cudaGetErrorString(e)));
     for (int i = 0; i < n; ++i) {
@@ -229,6 +243,13 @@ int run_iteration(brr_multi *m)
     for (int i = 0; i < n; ++i) {
         brr_ctx &c = *m->inst[i];
         int rc = sweep_collect(&c, &so[i]);
+        if (rc == BRR_ERR_RANGE && m->round) {
+            // the residual outgrew its fixed-point grid: this instance's sweep again, alone, on a coarser one
+            args[i].headroom += 12;
+            rc = sweep_reset(&c, c.st);
+            if (!rc)
+                rc = round_sweep(&c, args[i], smem, &so[i]);
+        }
         if (rc)
             return rc;
         rc = iter_post(c, so[i], its[i]);
@@ -290,30 +311,34 @@ int brr_multi_create(const brr_config *cfgs, int32_t n, brr_multi **out)
         for (int g = 0; g < c.n_groups; ++g)
             m->kmax = std::max(m->kmax, c.K[g]);
     }
-    // dynamic shared memory: what a CTA may use beside the kernel's static arrays
-    m->smem_limit = prop.sharedMemPerBlockOptin - sweep_multi_static_smem(m->form, m->kmax);
-    // first split of the SMs: at least what the slices need, the rest by N*M;
+    // first split of the SMs: at least what the slices need, the rest by N*M.
+    // The whole-round sweep where every instance fits it, else the restart sweep;
     // when the default round widths need more CTAs than there are SMs, every
     // instance starts at the narrowest width (the smallest code ring)
     std::vector<double> work(n);
     std::vector<int> mins(n), maxs(n), G, widths(n);
     const int narrowest = 8;
-    for (int pass = 0; pass < 2; ++pass) {
-        int need = 0;
+    bool split = false;
+    for (int pass = 0; pass < 4 && !split; ++pass) {
+        m->round = pass < 2;
+        // dynamic shared memory: what a CTA may use beside the kernel's static arrays
+        m->smem_limit = m->round ? kMaxRoundSmem
+                                 : prop.sharedMemPerBlockOptin - sweep_multi_static_smem(m->form, m->kmax);
+        split = true;
         for (int i = 0; i < n; ++i) {
             const brr_ctx *c = m->inst[i];
-            widths[i] = pass == 0 ? c->B : narrowest;
+            const int def = c->cfg.spec_width || !m->round ? c->B : 64;
+            widths[i] = pass % 2 == 0 ? def : narrowest;
             work[i] = (double)c->cfg.N * (double)c->cfg.M;
-            mins[i] = min_ctas(c, widths[i], m->smem_limit);
+            mins[i] = min_ctas(c, widths[i], m->smem_limit, m->round);
             maxs[i] = (int)((c->cfg.N + kChunkInd - 1) / kChunkInd);
-            if (mins[i] == 0)
+            if (mins[i] == 0 && pass == 3)
                 return bail(api_fail(BRR_ERR_ARG, "instance " + std::to_string(i) + " does not fit shared memory"));
-            need += mins[i];
+            split = split && mins[i] > 0;
         }
-        if (need <= m->sms)
-            break;
+        split = split && allocate(work, mins, maxs, m->sms, G);
     }
-    if (!allocate(work, mins, maxs, m->sms, G))
+    if (!split)
         return bail(api_fail(BRR_ERR_ARG, "the instances need more CTAs than the GPU has SMs"));
     for (int i = 0; i < n; ++i) {
         brr_ctx *c = m->inst[i];
@@ -326,6 +351,8 @@ int brr_multi_create(const brr_config *cfgs, int32_t n, brr_multi **out)
         m->inst[i] = x;
         if (rc)
             return bail(rc);
+        x->no_round = !m->round;
+        x->always_pairs = m->round;
     }
     cudaError_t e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
     for (int i = 0; i < 4 && e == cudaSuccess; ++i)
@@ -429,7 +456,7 @@ int brr_multi_tune(brr_multi *m, int32_t rounds)
     for (int b : cand) {
         for (int i = 0; i < n; ++i) {
             brr_ctx *c = m->inst[i];
-            const int B = inst_smem(c, c->G, b) <= m->smem_limit ? b : c->B;
+            const int B = inst_smem(c, c->G, b, m->round) <= m->smem_limit ? b : c->B;
             const int rc = reslice(c, c->G, B);
             if (rc)
                 return rc;
@@ -459,7 +486,7 @@ int brr_multi_tune(brr_multi *m, int32_t rounds)
         for (int i = 0; i < n; ++i) {
             brr_ctx *c = m->inst[i];
             work[i] = std::max(m->inst_ms[i], 1e-3) * c->G;
-            mins[i] = min_ctas(c, c->B, m->smem_limit);
+            mins[i] = min_ctas(c, c->B, m->smem_limit, m->round);
             maxs[i] = (int)((c->cfg.N + kChunkInd - 1) / kChunkInd);
         }
         if (!allocate(work, mins, maxs, m->sms, G))

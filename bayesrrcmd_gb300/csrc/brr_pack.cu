@@ -28,10 +28,12 @@ __global__ void __launch_bounds__(kThreads) k_pack_counts(const uint8_t *__restr
         int c0 = 0, c1 = 0, c2 = 0, c3 = 0;
         for (int64_t b = threadIdx.x; b < col_stride; b += blockDim.x) {
             if (b < cb) {
-                const unsigned v = src[b];
-                dst[b] = (uint8_t)v;
+                unsigned v = src[b];
                 const int64_t i0 = b * 4;
                 const int nvalid = (int)imin64(4, N - i0);
+                if (nvalid < 4)   // the payload's own padding bits: missing codes, as past the last byte
+                    v = (v & ((1u << (2 * nvalid)) - 1u)) | (0x55u & ~((1u << (2 * nvalid)) - 1u));
+                dst[b] = (uint8_t)v;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (k < nvalid) {

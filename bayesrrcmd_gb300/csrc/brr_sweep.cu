@@ -1,4 +1,9 @@
-// Persistent Gibbs-sweep kernel and its per-iteration helpers (sm_103a).
+// Restart Gibbs sweep and the per-iteration helpers of every sweep (sm_103a).
+//
+// The whole-round sweep of brr_round.cu takes every chain whose slices fit it;
+// this one remains for the largest slices of individuals (it holds 8 bytes of
+// residual per individual and a ring of codes, the other 24 and two rounds of
+// codes).
 //
 // Replaces BayesRBase::processColumn (src/BayesRBase.cpp:287-392) driven once
 // per marker by AnalysisGraph::exec (src/sequential.cpp:23-26,
@@ -18,19 +23,11 @@
 // the next round starts right after it.  Every sampled marker therefore sees
 // exactly the residual of the sequential chain.
 //
-// Pair-resolved ragged rounds (FP32C, ragged markers): a round resolves all its
-// B <= 32 markers.  Besides the dot products, every CTA sums over its slice the
-// integer pair terms A[p][t] = sum_i g_p(i) g_t(i) and Bm[p][t] = sum over the
-// individuals missing at p of g_t(i) for p < t, by population counts of the
-// markers' bit masks (ones, twos, missing) over the slice; after a change at marker p the
-// later markers' num move by the exact linear correction these terms give, and
-// every changing marker's residual update is applied in order at the end of the
-// round.
-//
 // The cluster variant runs the same sweep as one thread-block cluster of up to
 // 16 CTAs: each CTA stores its partial sums straight into every CTA's shared
 // memory (distributed shared memory, st.async completing on the receiver's
 // mbarrier), so a round needs no global atomics and no grid-wide barrier.
+#include "brr_cluster.cuh"
 #include "brr_device.cuh"
 #include "brr_internal.h"
 #include "brr_pick.cuh"
@@ -89,12 +86,12 @@ __global__ void k_gather(int form, int kind, const uint32_t *__restrict__ order,
     rec[q] = r;
 }
 
-// updateMu, first half: eps += mu_old, and per-block sum(eps) (src/DenseBayesRRmz.cpp:38-39).
+// updateMu, first half: eps += mu_old, and per-block sum(eps) and max |eps| (src/DenseBayesRRmz.cpp:38-39).
 __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, double mu_old, double *eps,
-                                                      float *eps_hi, float *eps_lo, double *part)
+                                                      float *eps_hi, float *eps_lo, double *part, double *emax)
 {
-    __shared__ double red[kThreads / 32];
-    double s = 0.0;
+    __shared__ double red[kThreads / 32][2];
+    double s = 0.0, mx = 0.0;
     float mh, ml;
     df_from_double(mu_old, mh, ml);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
@@ -102,25 +99,34 @@ __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, doubl
             const double e = __dadd_rn(eps[i], mu_old);
             eps[i] = e;
             s += e;
+            mx = fmax(mx, fabs(e));
         } else {
             float h = eps_hi[i], l = eps_lo[i];
             df_add(h, l, mh, ml);
             eps_hi[i] = h;
             eps_lo[i] = l;
             s += (double)h + (double)l;
+            mx = fmax(mx, fabs((double)h) + fabs((double)l));
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = s;
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5][0] = s;
+        red[threadIdx.x >> 5][1] = mx;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q)
-            t += red[q];
+        double t = 0.0, m = 0.0;
+        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
+            t += red[q][0];
+            m = fmax(m, red[q][1]);
+        }
         part[blockIdx.x] = t;
+        emax[blockIdx.x] = m;
     }
 }
 
@@ -195,18 +201,13 @@ struct SmemPlan {
     size_t gcf;             // FP32C: FP32 sampler constants, n_groups x kMaxK x 2 floats
     size_t gtab;            // FP32C dense: 256 float4 + 256 bytes
     size_t xch;             // cluster: [2][cluster][B] exchange records of 32 bytes
-    size_t gmap;            // pair-resolved ragged rounds: [slice_max][32] codes of the round's markers
-    size_t bmask;           // pair-resolved rounds: [3][words][32] bit masks of the round's markers
-    size_t pterm;           // pair-resolved rounds: [2][32][32] pair terms of the round
-    size_t gdfo;            // pair-resolved rounds: n_groups x kMaxK x {sd_k, 1/den_k} double-float
     size_t total;
 };
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 __host__ __device__ inline SmemPlan make_plan(int form, int kind, int slice_max, int slot_bytes, int B, int n_groups,
-                                              int cluster = 0, bool pair_rounds = false,
-                                              size_t rec_bytes = sizeof(SweepRec))
+                                              int cluster = 0, size_t rec_bytes = sizeof(SweepRec))
 {
     SmemPlan p;
     const int R = 4 * B;
@@ -237,19 +238,6 @@ __host__ __device__ inline SmemPlan make_plan(int form, int kind, int slice_max,
     o = align16(o);
     p.xch = o;
     o += (size_t)2 * cluster * B * 32;
-    p.gmap = o;
-    if (pair_rounds && kind == kKindRagged)
-        o += align16((size_t)slice_max * 32);
-    p.bmask = o;
-    // ragged: a word holds 32 individuals; dense: a 32-bit code word, 16
-    if (pair_rounds)
-        o += align16((size_t)3 * 32 * (kind == kKindRagged ? slice_max / 32 : slot_bytes / 4) * sizeof(unsigned));
-    p.pterm = o;
-    if (pair_rounds)
-        o += 2 * 32 * 32 * sizeof(unsigned long long);
-    p.gdfo = o;
-    if (pair_rounds)
-        o += align16((size_t)n_groups * kMaxK * 4 * sizeof(float));
     p.total = align16(o);
     return p;
 }
@@ -291,77 +279,6 @@ __device__ __forceinline__ double lut_select(unsigned c, double l0, double l1, d
     return (c & 2u) ? ((c & 1u) ? l3 : l2) : ((c & 1u) ? l1 : l0);
 }
 
-// ---- thread-block-cluster primitives (distributed shared memory)
-__device__ __forceinline__ unsigned cl_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// Address of the same shared-memory location in CTA `rank` of the cluster.
-__device__ __forceinline__ unsigned cl_map(unsigned addr, unsigned rank)
-{
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-
-// 16-byte store into a CTA's shared memory that completes as 16 transaction
-// bytes on that CTA's mbarrier `rbar`.
-__device__ __forceinline__ void cl_push16(unsigned raddr, unsigned long long w0, unsigned long long w1, unsigned rbar)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(raddr),
-                 "l"(w0), "l"(w1), "r"(rbar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void cl_bar_init(uint64_t *m)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_addr(m)) : "memory");
-}
-
-// The receiver's own arrival of a round: one arrival plus the bytes it expects.
-__device__ __forceinline__ void cl_expect(uint64_t *m, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_addr(m)), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ bool cl_test(uint64_t *m, unsigned parity)
-{
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(cl_addr(m)), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-
-// Waits for phase `parity` of m at most timeout_ns; false on timeout.
-__device__ __forceinline__ bool cl_wait(uint64_t *m, unsigned parity, uint64_t timeout_ns)
-{
-    if (cl_test(m, parity))
-        return true;
-    const uint64_t t0 = global_timer_ns();
-    unsigned spins = 0;
-    while (!cl_test(m, parity)) {
-        if ((++spins & 63u) == 0 && global_timer_ns() - t0 > timeout_ns)
-            return false;
-    }
-    return true;
-}
-
-// All threads of all CTAs of the cluster (release / acquire at cluster scope).
-// Used once after the mbarriers are initialised and once before the CTAs
-// exit; every wait between the two is bounded, so every CTA reaches both.
-__device__ __forceinline__ void cl_sync_all()
-{
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
-__device__ __forceinline__ unsigned cl_rank()
-{
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
 __device__ __forceinline__ __int128 u128_join(unsigned long long lo, unsigned long long hi)
 {
     return (__int128)(((unsigned __int128)hi << 64) | (unsigned __int128)lo);
@@ -374,20 +291,14 @@ __device__ __forceinline__ __int128 u128_join(unsigned long long lo, unsigned lo
 // variant that counts phase cycles on the first CTA (the plain variant reads no
 // clock, whose reads would constrain the scheduling of every CTA's code).
 // CL: the G CTAs are one thread-block cluster and exchange the round's partial
-// sums through distributed shared memory (k_sweep_cl).  PR: pair-resolved
-// rounds of FP32C ragged markers (k_sweep_pr).
-template <int FORM, int KIND, int KM, bool PROF, bool CL = false, bool PR = false>
+// sums through distributed shared memory (k_sweep_cl).
+template <int FORM, int KIND, int KM, bool PROF, bool CL = false>
 __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double s_beta[kMaxSpec];
     __shared__ double s_acum[kMaxSpec];
     __shared__ int s_comp[kMaxSpec];
-    __shared__ int s_chg[kMaxSpec];       // pair-resolved rounds: the marker changes the residual
-    __shared__ float s_pdf[32][8];        // pair-resolved rounds: its residual deltas (ragged: ones, twos,
-                                          // missing; dense: per 2-bit code)
-    __shared__ float s_nf[32][2];         // pair-resolved rounds: the marker's final num (double-float)
-    __shared__ int s_fbd[32];             // pair-resolved rounds: the decision came from the FP64 sampler
     __shared__ int s_first;
     __shared__ int s_abort;
     __shared__ double s_scal[4];          // ragged: shift, epsSum; dense FP32C: residual total
@@ -410,7 +321,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
     const int ns = a.slice_lo[sidx + 1] - lo;
     const int nbytes = ((ns + kChunk - 1) / kChunk) * 16;
     const int64_t byte_lo = lo / 4;
-    const SmemPlan plan = make_plan(FORM, KIND, a.slice_max, a.slot_bytes, B, a.n_groups, CL ? a.G : 0, PR);
+    const SmemPlan plan = make_plan(FORM, KIND, a.slice_max, a.slot_bytes, B, a.n_groups, CL ? a.G : 0);
 
     double *eps64 = reinterpret_cast<double *>(smem + plan.eps0);
     float *eh = reinterpret_cast<float *>(smem + plan.eps0);
@@ -426,20 +337,6 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
     // cluster exchange records [round parity][source CTA][marker]: the partial
     // sum and the missing-genotype sum, each a 128-bit fixed-point integer
     ulonglong2 *xch = reinterpret_cast<ulonglong2 *>(smem + plan.xch);
-    // pair-resolved rounds.  Ragged: per individual of the slice the codes of
-    // the round's markers (0 absent, 1 or 2 listed genotype, 3 missing) and
-    // their bit masks over the slice [ones | twos | missing][word][marker];
-    // the round's pair terms [p][t] summed over the CTAs (A low, Bm high
-    // word).  Dense: bit masks of the code words [genotype >= 1 | genotype 2
-    // | missing][word][marker] at the even bit of each individual, and two
-    // words of pair terms [P | MM][p][t], [Gmp | Gmt][p][t], the diagonal
-    // holding each marker's genotype sum and missing count.
-    const int mw = KIND == kKindRagged ? a.slice_max / 32 : a.slot_bytes / 4;
-    uint8_t *gmap = smem + plan.gmap;
-    unsigned *bmask = reinterpret_cast<unsigned *>(smem + plan.bmask);
-    unsigned long long *s_pt = reinterpret_cast<unsigned long long *>(smem + plan.pterm);
-    float4 *gdf = reinterpret_cast<float4 *>(smem + plan.gdfo);
-
     // ---- prologue: residual slice, constants, tables
     float muh, mul;
     df_from_double(-a.mu_new, muh, mul);
@@ -563,7 +460,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
     const int team = tid >> lpm_log2;
     const double Nm1 = (double)(a.N - 1);
     const bool prof = PROF && sidx == 0 && tid == 0;
-    long long ph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    long long ph[5] = {0, 0, 0, 0, 0};
     long long tp = prof ? clock64() : 0;
     auto mark = [&](int k) {
         if (prof) {
@@ -584,21 +481,6 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
     };
     for (int i = tid; i < kMaxSpec * 4; i += kThreads)
         s_acc[i] = 0ull;
-    if (PR) {
-        if (KIND == kKindRagged)
-            for (int i = tid; i < a.slice_max * 2; i += kThreads)
-                reinterpret_cast<uint4 *>(gmap)[i] = make_uint4(0u, 0u, 0u, 0u);
-        // beta = z sd_k + num / den_k of a non-zero component in double-float
-        for (int i = tid; i < a.n_groups * kMaxK; i += kThreads) {
-            const int k = i % kMaxK;
-            const double *row = a.gconst + (size_t)(i / kMaxK) * kMaxK * 4;
-            float4 v;
-            df_from_double(row[4 * k + 3], v.x, v.y);
-            df_from_double(row[4 * k + 1], v.z, v.w);
-            gdf[i] = v;
-        }
-    }
-
     unsigned start = 0;
     long long r = 0;
     int rb = 0;   // r % 3
@@ -758,18 +640,11 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
                     for (int e = ro[0] + tm.lane; e < ro[1]; e += lpm) {
                         const int i = a.ridx[0][e];
                         df_add(h, l, eh[i], el[i]);
-                        if (PR)
-                            gmap[i * 32 + team] = 1;
                     }
                     for (int e = ro[2] + tm.lane; e < ro[3]; e += lpm) {
                         const int i = a.ridx[1][e];
                         df_add(h, l, 2.f * eh[i], 2.f * el[i]);
-                        if (PR)
-                            gmap[i * 32 + team] = 2;
                     }
-                    if (PR)
-                        for (int e = ro[4] + tm.lane; e < ro[5]; e += lpm)
-                            gmap[a.ridx[2][e] * 32 + team] = 3;
                     team_df_sum(h, l, tm, lpm);
                     float mh = 0.f, ml = 0.f;
                     if (a.eigen) {
@@ -802,113 +677,6 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
                 atomicCAS(a.err, kDevOk, kDevRange);
         }
         __syncthreads();
-        if (PR && KIND == kKindDense) {
-            mark(6);
-            // bit masks of the round's markers from their code words (16
-            // individuals each, code 0: genotype 2, 1: missing, 2: genotype 1,
-            // 3: genotype 0; individuals past the slice masked), one thread per
-            // (word, marker)
-            const int nwd = (ns + 15) / 16;
-            for (int e = tid; e < nwd * 32; e += kThreads) {
-                const int w = e >> 5, t = e & 31;
-                unsigned h = 0u, d = 0u, m = 0u;
-                if (t < nb) {
-                    const unsigned cw =
-                        reinterpret_cast<const unsigned *>(ring_codes + ((start + t) & Rm) * a.slot_bytes)[w];
-                    const int nv = ns - 16 * w;
-                    const unsigned vm = nv >= 16 ? 0x55555555u : (0x55555555u & ((1u << (2 * nv)) - 1u));
-                    h = ~cw & vm;
-                    d = ~cw & ~(cw >> 1) & vm;
-                    m = cw & ~(cw >> 1) & vm;
-                }
-                bmask[w * 32 + t] = h;
-                bmask[(mw + w) * 32 + t] = d;
-                bmask[(2 * mw + w) * 32 + t] = m;
-            }
-            __syncthreads();
-            // pair terms p <= t, a pair per thread: P = sum g_p g_t, MM =
-            // individuals missing at both, Gmp = sum of g_t over the
-            // individuals missing at p, Gmt = sum of g_p over those missing at
-            // t; on the diagonal the marker's genotype sum and missing count
-            // (g = [genotype >= 1] + [genotype 2])
-            unsigned long long *gp = a.pairs + (size_t)rb * 2048;
-            for (int e = tid; e < 1024; e += kThreads) {
-                const int p = e >> 5, t = e & 31;
-                if (p > t || t >= nb)
-                    continue;
-                unsigned w0a = 0u, w0b = 0u, w1a = 0u, w1b = 0u;
-                for (int w = 0; w < nwd; ++w) {
-                    const unsigned *hh = bmask + w * 32, *dd = bmask + (mw + w) * 32, *mm = bmask + (2 * mw + w) * 32;
-                    const unsigned hp = hh[p], dp = dd[p], mp = mm[p];
-                    if (p == t) {
-                        w0a += __popc(hp) + __popc(dp);
-                        w0b += __popc(mp);
-                    } else {
-                        const unsigned ht = hh[t], dt = dd[t], mt = mm[t];
-                        w0a += __popc(hp & ht) + __popc(hp & dt) + __popc(dp & ht) + __popc(dp & dt);
-                        if (a.has_missing) {
-                            w0b += __popc(mp & mt);
-                            w1a += __popc(mp & ht) + __popc(mp & dt);
-                            w1b += __popc(mt & hp) + __popc(mt & dp);
-                        }
-                    }
-                }
-                const unsigned long long v0 = (unsigned long long)w0a | ((unsigned long long)w0b << 32);
-                const unsigned long long v1 = (unsigned long long)w1a | ((unsigned long long)w1b << 32);
-                if (v0)
-                    red_add_u64(gp + e, v0);
-                if (v1)
-                    red_add_u64(gp + 1024 + e, v1);
-            }
-            __syncthreads();
-            mark(7);
-        } else if (PR) {
-            mark(6);
-            // bit masks of the round's markers over the slice, one thread per
-            // (word, marker): 32 consecutive individuals' codes of the marker
-            const int nwd = (ns + 31) / 32;
-            for (int e = tid; e < nwd * 32; e += kThreads) {
-                const int w = e >> 5, t = e & 31;
-                unsigned m1 = 0u, m2 = 0u, mm = 0u;
-                if (t < nb) {
-                    const int nj = min(32, ns - 32 * w);
-                    const uint8_t *col = gmap + (size_t)32 * w * 32 + t;
-                    for (int j = 0; j < nj; ++j) {
-                        const unsigned c = col[j * 32];
-                        m1 |= (c == 1u ? 1u : 0u) << j;
-                        m2 |= (c == 2u ? 1u : 0u) << j;
-                        mm |= (c == 3u ? 1u : 0u) << j;
-                    }
-                }
-                bmask[w * 32 + t] = m1;
-                bmask[(mw + w) * 32 + t] = m2;
-                bmask[(2 * mw + w) * 32 + t] = mm;
-            }
-            __syncthreads();
-            // pair terms p < t of the round's markers over the slice, a pair
-            // per thread: A[p][t] = sum g_p g_t over individuals listed in
-            // both, Bm[p][t] = sum of g_t over the individuals missing at p;
-            // published as exact integers (ordered before the barrier's
-            // release by the CTA barrier below)
-            unsigned long long *gp = a.pairs + (size_t)rb * 2048;
-            for (int e = tid; e < 1024; e += kThreads) {
-                const int p = e >> 5, t = e & 31;
-                if (p >= t || t >= nb)
-                    continue;
-                unsigned A = 0, Bm = 0;
-                for (int w = 0; w < nwd; ++w) {
-                    const unsigned *m1 = bmask + w * 32, *m2 = bmask + (mw + w) * 32, *mm = bmask + (2 * mw + w) * 32;
-                    const unsigned a1 = m1[p], a2 = m2[p], am = mm[p], b1 = m1[t], b2 = m2[t];
-                    A += __popc(a1 & b1) + 2u * (__popc(a1 & b2) + __popc(a2 & b1)) + 4u * __popc(a2 & b2);
-                    Bm += __popc(am & b1) + 2u * __popc(am & b2);
-                }
-                const unsigned long long v = (unsigned long long)A | ((unsigned long long)Bm << 32);
-                if (v)
-                    red_add_u64(gp + e, v);
-            }
-            __syncthreads();
-            mark(7);
-        }
         mark(1);
 
         // ---- grid barrier: one counter; release orders this CTA's
@@ -944,274 +712,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
         if (s_abort)
             break;
 
-        if (PR) {
-            // ---- pair-resolved round, identically in every CTA: lane t
-            // samples marker t; after the first change p the later markers'
-            // num move by dBeta_p isd_p isd_t (A[p][t] + mean_p Bm[p][t]
-            // - mean_t (Zsum_p - mean_p N) - mean_p Zsum_t), the change of
-            // x_t . eps that p's residual update, running sum and pending
-            // shift make (src/raggedbayesrkernel.cpp:10-35), and they are
-            // sampled again
-            const unsigned long long *gp = a.pairs + (size_t)rb * 2048;
-            for (int e = tid; e < (KIND == kKindDense ? 2048 : 1024); e += kThreads)
-                s_pt[e] = ld_relaxed_u64(gp + e);
-            __syncthreads();
-            if (tid < 32) {
-                const int t = tid;
-                const bool valid = t < nb;
-                const SweepRec &rc = ring_rec[(start + (valid ? t : 0)) & Rm];
-                // ragged: mean, 1/sd, sum of listed genotypes; dense: sigma,
-                // column mean, value of a missing genotype, sum of the column
-                const double mean = rc.t[0], isd = rc.t[2], Zsum = rc.t[3];
-                double num0 = 0.0;
-                if (valid) {
-                    const unsigned long long *acc = solo ? s_acc + t * 4 : a.acc + (rb * kMaxSpec + t) * 4;
-                    auto ldw = [&](int k) -> unsigned long long { return solo ? acc[k] : ld_relaxed_u64(acc + k); };
-                    const double tot = fx_join((long long)ldw(0), ldw(1));
-                    if (KIND == kKindDense) {
-                        const double sm = fx_join((long long)ldw(2), ldw(3));
-                        num0 = (rc.t[0] * (tot - rc.t[1] * (s_scal[2] - sm)) + rc.t[2] * sm) +
-                               rc.beta_old * ((double)a.N - 1.0);
-                    } else {
-                        num0 = (rc.beta_old * ((double)a.N - 1.0) - mean * s_scal[1] * isd) + (tot + s_scal[0] * Zsum) * isd;
-                    }
-                }
-                // num, the marker constants and the corrections in double-float
-                float nh, nl, mh, ml, ih, il;
-                df_from_double(num0, nh, nl);
-                df_from_double(mean, mh, ml);     // dense: sigma
-                df_from_double(isd, ih, il);      // dense: value of a missing genotype
-                const float Zf = (float)Zsum, Nf = (float)a.N;
-                // dense: column mean, sum of the column, sigma * colmean and
-                // sigma * colmean + the missing value, the marker's genotype sum
-                // and missing count (the diagonal of the pair terms)
-                float cmh = 0.f, cml = 0.f, csh = 0.f, csl = 0.f, sch = 0.f, scl = 0.f, sxh = 0.f, sxl = 0.f;
-                float Sg = 0.f, Nm = 0.f;
-                if (KIND == kKindDense) {
-                    df_from_double(rc.t[1], cmh, cml);
-                    df_from_double(rc.t[3], csh, csl);
-                    df_mul(mh, ml, cmh, cml, sch, scl);
-                    sxh = sch;
-                    sxl = scl;
-                    df_add(sxh, sxl, ih, il);
-                    const unsigned long long dg = s_pt[t * 32 + t];
-                    Sg = (float)(unsigned)dg;
-                    Nm = (float)(unsigned)(dg >> 32);
-                }
-                const int g = valid ? rc.group : 0;
-                const double *gcg = gconst + (size_t)g * kMaxK * 4;
-                const float *gcfg = gcf + (size_t)g * kMaxK * 2;
-                const int K = gk[g];
-                const float uf = __double2float_rn(rc.u);
-                // certified decisions with a stability margin in num^2: a marker
-                // is sampled again only when a correction moves num^2 beyond
-                // its margin (H: the spread of the group's h_k, h_0 = 0
-                // included); decisions the margin sampler cannot certify are
-                // taken by the guarded FP32 sampler, else in FP64
-                float H = 0.f;
-                {
-                    float hmax = 0.f, hmin = 0.f;
-                    for (int k = 1; k < K; ++k) {
-                        hmax = fmaxf(hmax, gcfg[2 * k + 1]);
-                        hmin = fminf(hmin, gcfg[2 * k + 1]);
-                    }
-                    H = (hmax - hmin) * 1.000001f;
-                }
-                bool done = !valid;
-                int comp = -1;
-                float sref = 0.f, wmar = -1.f;
-                bool fbd = false;
-                double fb_beta = rc.beta_old, fb_acum = 0.0;
-                float boh, bol, zh, zl;
-                df_from_double(rc.beta_old, boh, bol);
-                df_from_double(rc.z, zh, zl);
-                const float4 *gdfg = gdf + (size_t)g * kMaxK;
-                for (;;) {
-                    const float sx = __fmaf_rn(nh, nh, 2.f * nh * nl);
-                    const float delta = fabsf(sx - sref) * 1.000001f + 4e-7f * (sx + sref);
-                    if (!done && !(H * delta <= wmar)) {
-                        int cm;
-                        float w;
-                        fbd = false;
-                        if (pick_margin<KM>(sx, uf, gcfg, K, cm, w)) {
-                            comp = cm;
-                            sref = sx;
-                            wmar = w;
-                        } else {
-                            float a0;
-                            wmar = -1.f;
-                            if (!pick_f32<KM>(nh, nl, uf, gcfg, K, comp, a0)) {
-                                const Pick pk = pick_marker<true, KM>((double)nh + (double)nl, rc.u, rc.z, rc.beta_old,
-                                                                      gcg, K);
-                                comp = pk.comp;
-                                fb_beta = pk.beta;
-                                fb_acum = pk.acum0;
-                                fbd = true;
-                            }
-                        }
-                    }
-                    const bool chg = !done && (rc.beta_old != 0.0 || comp > 0);
-                    const unsigned mask = __ballot_sync(0xffffffffu, chg);
-                    const int p = mask ? __ffs(mask) - 1 : 32;
-                    float ch = 0.f, cl = 0.f;
-                    if (!done && t <= p) {
-                        // the decision of marker t is final (src/BayesRBase.cpp:346-366);
-                        // beta, acum and the residual deltas follow after the round
-                        s_nf[t][0] = nh;
-                        s_nf[t][1] = nl;
-                        s_comp[t] = comp;
-                        s_fbd[t] = fbd ? 1 : 0;
-                        s_chg[t] = t == p ? 1 : 0;
-                        if (fbd) {
-                            s_beta[t] = fb_beta;
-                            s_acum[t] = fb_acum;
-                        }
-                        if (t == p) {
-                            // dBeta isd of the change in double-float
-                            float bh = boh, bl = bol;
-                            if (fbd) {
-                                df_from_double(fb_beta, bh, bl);
-                            } else if (comp == 0) {
-                                bh = bl = 0.f;
-                            } else if (comp > 0) {
-                                const float4 k4 = gdfg[comp];
-                                float ah, al, xh, xl;
-                                df_mul(zh, zl, k4.x, k4.y, ah, al);
-                                df_mul(nh, nl, k4.z, k4.w, xh, xl);
-                                df_add(ah, al, xh, xl);
-                                bh = ah;
-                                bl = al;
-                            }
-                            float dh = boh, dl = bol;
-                            df_add(dh, dl, -bh, -bl);
-                            if (KIND == kKindDense) {
-                                ch = dh;
-                                cl = dl;
-                            } else {
-                                df_mul(dh, dl, ih, il, ch, cl);
-                            }
-                        }
-                        done = true;
-                    }
-                    if (!mask)
-                        break;
-                    if (KIND == kKindDense) {
-                        // x_p . x_t moves num_t by dBeta_p (sigma_t dT - sigma_t cm_t dE
-                        // + (sigma_t cm_t + xm_t) dSm): dT the change of the sum of
-                        // g_t eps over t's genotypes, dE of the residual total, dSm of
-                        // the residual over t's missing genotypes
-                        ch = __shfl_sync(0xffffffffu, ch, p);
-                        cl = __shfl_sync(0xffffffffu, cl, p);
-                        const float sph = __shfl_sync(0xffffffffu, mh, p), spl = __shfl_sync(0xffffffffu, ml, p);
-                        const float cph = __shfl_sync(0xffffffffu, cmh, p), cpl = __shfl_sync(0xffffffffu, cml, p);
-                        const float xph = __shfl_sync(0xffffffffu, ih, p), xpl = __shfl_sync(0xffffffffu, il, p);
-                        const float eph = __shfl_sync(0xffffffffu, csh, p), epl = __shfl_sync(0xffffffffu, csl, p);
-                        if (!done) {
-                            const unsigned long long v0 = s_pt[p * 32 + t], v1 = s_pt[1024 + p * 32 + t];
-                            const float P = (float)(unsigned)v0, MM = (float)(unsigned)(v0 >> 32);
-                            const float Gmp = (float)(unsigned)v1, Gmt = (float)(unsigned)(v1 >> 32);
-                            // dT = sigma_p (P - cm_p (S_t - Gmp)) + xm_p Gmp
-                            float th, tl, uh, ul;
-                            df_mul(cph, cpl, Sg - Gmp, 0.f, th, tl);
-                            th = -th;
-                            tl = -tl;
-                            df_add(th, tl, P, 0.f);
-                            df_mul(sph, spl, th, tl, uh, ul);
-                            df_mul(xph, xpl, Gmp, 0.f, th, tl);
-                            df_add(uh, ul, th, tl);
-                            // sigma_t dT - sigma_t cm_t dE
-                            float rh, rl, qh, ql;
-                            df_mul(mh, ml, uh, ul, rh, rl);
-                            df_mul(sch, scl, eph, epl, qh, ql);
-                            df_add(rh, rl, -qh, -ql);
-                            if (a.has_missing) {
-                                // dSm = sigma_p (Gmt - cm_p (nmiss_t - MM)) + xm_p MM
-                                df_mul(cph, cpl, Nm - MM, 0.f, th, tl);
-                                th = -th;
-                                tl = -tl;
-                                df_add(th, tl, Gmt, 0.f);
-                                df_mul(sph, spl, th, tl, uh, ul);
-                                df_mul(xph, xpl, MM, 0.f, th, tl);
-                                df_add(uh, ul, th, tl);
-                                df_mul(sxh, sxl, uh, ul, qh, ql);
-                                df_add(rh, rl, qh, ql);
-                            }
-                            float xh2, xl2;
-                            df_mul(ch, cl, rh, rl, xh2, xl2);
-                            df_add(nh, nl, xh2, xl2);
-                        }
-                        continue;
-                    }
-                    // num_t += dBeta_p isd_p isd_t (A + mean_p Bm - mean_t (Zsum_p
-                    // - mean_p N) - mean_p Zsum_t)
-                    ch = __shfl_sync(0xffffffffu, ch, p);
-                    cl = __shfl_sync(0xffffffffu, cl, p);
-                    const float mph = __shfl_sync(0xffffffffu, mh, p), mpl = __shfl_sync(0xffffffffu, ml, p);
-                    const float Zp = __shfl_sync(0xffffffffu, Zf, p);
-                    if (!done) {
-                        const unsigned long long v = s_pt[p * 32 + t];
-                        const float A = (float)(unsigned)v, Bm = (float)(unsigned)(v >> 32);
-                        float t1h, t1l, t2h, t2l, t3h, t3l, t4h, t4l;
-                        df_mul(mph, mpl, Bm, 0.f, t1h, t1l);
-                        df_add(t1h, t1l, A, 0.f);
-                        df_mul(mph, mpl, Nf, 0.f, t2h, t2l);
-                        t2h = -t2h;
-                        t2l = -t2l;
-                        df_add(t2h, t2l, Zp, 0.f);
-                        df_mul(mh, ml, t2h, t2l, t3h, t3l);
-                        df_mul(mph, mpl, Zf, 0.f, t4h, t4l);
-                        df_add(t1h, t1l, -t3h, -t3l);
-                        df_add(t1h, t1l, -t4h, -t4l);
-                        float kh, kl, xh, xl;
-                        df_mul(ch, cl, ih, il, kh, kl);
-                        df_mul(kh, kl, t1h, t1l, xh, xl);
-                        df_add(nh, nl, xh, xl);
-                    }
-                }
-            }
-            __syncthreads();
-            // beta and acum of every marker at its final num, and the residual
-            // deltas (ones, twos, missing genotypes) of every change, as the
-            // pass per marker forms them
-            if (tid < nb) {
-                const SweepRec &rc = ring_rec[(start + tid) & Rm];
-                if (!s_fbd[tid]) {
-                    const int g = rc.group;
-                    const double *gcg = gconst + (size_t)g * kMaxK * 4;
-                    const int comp = s_comp[tid];
-                    const float nh = s_nf[tid][0], nl = s_nf[tid][1];
-                    double bnew = comp == 0 ? 0.0 : rc.beta_old;
-                    if (comp > 0)
-                        bnew = __dadd_rn(__dmul_rn(rc.z, gcg[4 * comp + 3]),
-                                         __dmul_rn((double)nh + (double)nl, gcg[4 * comp + 1]));
-                    int c2;
-                    float a0;
-                    pick_f32<KM>(nh, nl, __double2float_rn(rc.u), gcf + (size_t)g * kMaxK * 2, gk[g], c2, a0);
-                    s_beta[tid] = bnew;
-                    s_acum[tid] = (double)a0;
-                }
-            }
-            if (tid < nb && s_chg[tid]) {
-                const SweepRec &rc = ring_rec[(start + tid) & Rm];
-                const double dBeta = rc.beta_old - s_beta[tid];
-                if (KIND == kKindDense) {
-                    // delta per 2-bit code: dBeta (g - colmean) sigma, a missing genotype dBeta xm
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const double gv = c == 0 ? 2.0 : (c == 2 ? 1.0 : 0.0);
-                        const double d = c == 1 ? dBeta * rc.t[2] : dBeta * ((gv - rc.t[1]) * rc.t[0]);
-                        df_from_double(d, s_pdf[tid][2 * c], s_pdf[tid][2 * c + 1]);
-                    }
-                } else {
-                    const double oneAdj = dBeta * rc.t[2];
-                    const double dk[3] = {oneAdj, 2.0 * oneAdj, dBeta * rc.t[0] * rc.t[2]};
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        df_from_double(dk[k], s_pdf[tid][2 * k], s_pdf[tid][2 * k + 1]);
-                }
-            }
-            __syncthreads();
-        } else if (tid < nb) {
+        if (tid < nb) {
             // ---- redundant sampling of the round's markers in every CTA, one thread per marker
             const SweepRec &rc = ring_rec[(start + tid) & Rm];
             const unsigned long long *acc = solo ? s_acc + tid * 4 : a.acc + (rb * kMaxSpec + tid) * 4;
@@ -1283,7 +784,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
         __syncthreads();
         mark(3);
 
-        const int first = (a.async_batch > 0 || PR) ? nb : s_first;
+        const int first = a.async_batch > 0 ? nb : s_first;
         const int last = first < nb ? first : nb - 1;
         if (sidx == 0) {
             // outputs of the resolved markers, only from CTA 0
@@ -1300,9 +801,6 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
             // all CTAs have read the accumulators of round r-1: recycle them
             if (!CL && tid < 4 * kMaxSpec)
                 a.acc[((rb + 2) % 3) * kMaxSpec * 4 + tid] = 0ull;
-            if (PR)
-                for (int e = tid; e < 2048; e += kThreads)
-                    a.pairs[(size_t)((rb + 2) % 3) * 2048 + e] = 0ull;
         }
         if (solo)   // the sampling has read this round's sums (barrier above)
             for (int i = tid; i < kMaxSpec * 4; i += kThreads)
@@ -1383,71 +881,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
                 }
             }
         };
-        if (PR) {
-            // every changing marker's residual update, in sweep order, by the
-            // owner of each individual from the round's bit masks (the same
-            // operations as a pass per marker, with the deltas the resolve
-            // formed); the pending shift and the running sum in order by one
-            // thread, one without individuals when there is one
-            unsigned chm = 0u;
-            for (int u = 0; u < nb; ++u)
-                chm |= s_chg[u] ? 1u << u : 0u;
-            if (tid == (ns < kThreads ? kThreads - 1 : 0)) {
-                for (unsigned m = chm; m; m &= m - 1u) {
-                    const int u = __ffs(m) - 1;
-                    const SweepRec &rc = ring_rec[(start + u) & Rm];
-                    const double dBeta = rc.beta_old - s_beta[u];
-                    if (KIND == kKindDense) {
-                        // the residual total moves by dBeta times the column sum
-                        s_scal[2] = s_scal[2] + dBeta * rc.t[3];
-                    } else {
-                        const double mean = rc.t[0], isd = rc.t[2], Zsum = rc.t[3];
-                        s_scal[0] = s_scal[0] - dBeta * mean * isd;
-                        s_scal[1] = s_scal[1] + ((dBeta * Zsum) * isd - ((dBeta * mean) * (double)a.N) * isd);
-                    }
-                }
-            }
-            if (chm && KIND == kKindDense) {
-                // every individual of the slice moves with every change: the
-                // delta of its code, marker by marker in sweep order
-                for (int i = tid; i < ns; i += kThreads) {
-                    float h = eh[i], l = el[i];
-                    for (unsigned m = chm; m; m &= m - 1u) {
-                        const int u = __ffs(m) - 1;
-                        const unsigned c = (ring_codes[((start + u) & Rm) * a.slot_bytes + (i >> 2)] >> (2 * (i & 3))) & 3u;
-                        df_add(h, l, s_pdf[u][2 * c], s_pdf[u][2 * c + 1]);
-                    }
-                    eh[i] = h;
-                    el[i] = l;
-                }
-            } else if (chm) {
-                for (int i = tid; i < ns; i += kThreads) {
-                    const int w = i >> 5;
-                    const unsigned bit = 1u << (i & 31);
-                    float h = eh[i], l = el[i];
-                    bool any = false;
-                    for (unsigned m = chm; m; m &= m - 1u) {
-                        const int u = __ffs(m) - 1;
-                        const int k = (bmask[w * 32 + u] & bit) ? 0
-                                      : (bmask[(mw + w) * 32 + u] & bit) ? 1
-                                      : (bmask[(2 * mw + w) * 32 + u] & bit) ? 2 : -1;
-                        if (k >= 0) {
-                            df_add(h, l, s_pdf[u][2 * k], s_pdf[u][2 * k + 1]);
-                            any = true;
-                        }
-                    }
-                    if (any) {
-                        eh[i] = h;
-                        el[i] = l;
-                    }
-                }
-            }
-            __syncthreads();
-            // the next round's codes start from zero
-            if (KIND == kKindRagged)
-                for (int i = tid; i < ns * 2; i += kThreads)
-                    reinterpret_cast<uint4 *>(gmap)[i] = make_uint4(0u, 0u, 0u, 0u);
-        } else if (a.async_batch > 0) {
+        if (a.async_batch > 0) {
             for (int u = 0; u < nb; ++u) {
                 if (ring_rec[(start + u) & Rm].beta_old != 0.0 || s_beta[u] != 0.0) {
                     apply_one(u);
@@ -1467,8 +901,6 @@ __device__ __forceinline__ void sweep_body(const SweepArgs &a, const int sidx)
         for (int k = 0; k < 5; ++k)
             a.prof[k] = ph[k];
         a.prof[5] = r;
-        a.prof[6] = ph[6];   // pair-resolved rounds: the dot products (phase 1 is then the publication)
-        a.prof[7] = ph[7];   // pair-resolved rounds: the pair terms
     }
     cp_async_wait_all();
     __syncthreads();
@@ -1527,13 +959,6 @@ template <int FORM, int KIND, int KM, bool PROF>
 __global__ void __launch_bounds__(kThreads, 1) k_sweep(SweepArgs a)
 {
     sweep_body<FORM, KIND, KM, PROF>(a, (int)blockIdx.x);
-}
-
-// Pair-resolved rounds over FP32C dense or ragged markers.
-template <int KIND, int KM, bool PROF>
-__global__ void __launch_bounds__(kThreads, 1) k_sweep_pr(SweepArgs a)
-{
-    sweep_body<kFormFP32C, KIND, KM, PROF, false, true>(a, (int)blockIdx.x);
 }
 
 // The sweep as one thread-block cluster of G CTAs (the whole grid); the
@@ -1623,9 +1048,9 @@ cudaError_t launch_gather(int form, int kind, const uint32_t *order, int64_t M, 
 }
 
 cudaError_t launch_mu_prep(int form, int64_t N, double mu_old, double *eps, float *eps_hi, float *eps_lo,
-                           double *part, int nblocks, cudaStream_t st)
+                           double *part, double *emax, int nblocks, cudaStream_t st)
 {
-    k_mu_prep<<<nblocks, kThreads, 0, st>>>(form, N, mu_old, eps, eps_hi, eps_lo, part);
+    k_mu_prep<<<nblocks, kThreads, 0, st>>>(form, N, mu_old, eps, eps_hi, eps_lo, part, emax);
     return cudaGetLastError();
 }
 
@@ -1666,7 +1091,7 @@ cudaError_t launch_sweep_stats(int64_t M, const int32_t *group, const int32_t *c
 
 size_t sweep_smem_bytes(int form, int kind, const SweepArgs &a)
 {
-    return make_plan(form, kind, a.slice_max, a.slot_bytes, a.B, a.n_groups, a.cluster, a.pairs != nullptr).total;
+    return make_plan(form, kind, a.slice_max, a.slot_bytes, a.B, a.n_groups, a.cluster).total;
 }
 
 // Clusters above 8 CTAs are a non-portable size, allowed per kernel.
@@ -1714,8 +1139,6 @@ static cudaError_t launch_one(const SweepArgs &a, size_t smem, cudaStream_t st)
     if (a.cluster > 0)
         return launch_one_cl<FORM, KIND, KM>(a, smem, st);
     const void *f = a.prof ? (const void *)k_sweep<FORM, KIND, KM, true> : (const void *)k_sweep<FORM, KIND, KM, false>;
-    if (FORM == kFormFP32C && a.pairs)
-        f = a.prof ? (const void *)k_sweep_pr<KIND, KM, true> : (const void *)k_sweep_pr<KIND, KM, false>;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
@@ -1832,22 +1255,11 @@ cudaError_t launch_sweep_multi(int form, int kmax, const MultiSweepArgs &m, size
     return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
-int sweep_max_ctas_per_sm(int form, int kind, size_t smem, bool pair_rounds)
+int sweep_max_ctas_per_sm(int form, int kind, size_t smem)
 {
     int n = 1 << 30;
     const void *fs[4] = {sweep_fn<4, false>(form, kind), sweep_fn<kMaxK, false>(form, kind),
                          sweep_fn<4, true>(form, kind), sweep_fn<kMaxK, true>(form, kind)};
-    if (pair_rounds && kind == kKindDense) {
-        fs[0] = (const void *)k_sweep_pr<kKindDense, 4, false>;
-        fs[1] = (const void *)k_sweep_pr<kKindDense, kMaxK, false>;
-        fs[2] = (const void *)k_sweep_pr<kKindDense, 4, true>;
-        fs[3] = (const void *)k_sweep_pr<kKindDense, kMaxK, true>;
-    } else if (pair_rounds) {
-        fs[0] = (const void *)k_sweep_pr<kKindRagged, 4, false>;
-        fs[1] = (const void *)k_sweep_pr<kKindRagged, kMaxK, false>;
-        fs[2] = (const void *)k_sweep_pr<kKindRagged, 4, true>;
-        fs[3] = (const void *)k_sweep_pr<kKindRagged, kMaxK, true>;
-    }
     for (const void *f : fs) {
         int m = 0;
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

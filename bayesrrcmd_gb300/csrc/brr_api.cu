@@ -507,10 +507,10 @@ int brr::sweep_enqueue_inputs(brr_ctx *c, double eps_total, cudaStream_t st)
     const size_t ng = (size_t)cf.n_groups;
     BRR_CUDA(cudaMemcpyAsync(c->d_gconst, c->h_gc, sizeof(double) * ng * kMaxK * 4, cudaMemcpyHostToDevice, st));
     BRR_CUDA(cudaMemcpyAsync(c->d_gK, c->h_gK, sizeof(int32_t) * ng, cudaMemcpyHostToDevice, st));
+    int kmax = 0;
+    for (int g = 0; g < cf.n_groups; ++g)
+        kmax = std::max(kmax, cf.K[g]);
     if (c->use_round()) {
-        int kmax = 0;
-        for (int g = 0; g < cf.n_groups; ++g)
-            kmax = std::max(kmax, cf.K[g]);
         // num of a marker without effect has variance about (N - 1) sigmaE: 2.5
         // standard deviations
         const float likely = (float)(6.25 * (double)cf.N * c->sigmaE);
@@ -523,7 +523,7 @@ int brr::sweep_enqueue_inputs(brr_ctx *c, double eps_total, cudaStream_t st)
                                         c->d_counts, c->d_rnz, round_all_rows(c), c->d_psum, c->d_rgram, c->sms, st));
     } else if (c->blocked)
         BRR_CUDA(launch_gather_block(c->d_order, cf.M, cf.N, c->d_table, c->d_scale, c->d_beta, c->d_u, c->d_z,
-                                     c->d_group, eps_total, c->d_brec, st));
+                                     c->d_group, eps_total, kmax, c->d_gconst, c->d_gK, c->d_brec, st));
     else
         BRR_CUDA(launch_gather(cf.form, c->kind, c->d_order, cf.M, c->d_table, c->d_scale, c->d_beta, c->d_u,
                                c->d_z, c->d_group, c->d_colsum, c->d_rec, st));
@@ -595,10 +595,12 @@ void brr::sweep_args(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, 
     a.has_missing = c->has_missing ? 1 : 0;
     a.brec = c->d_brec;
     a.order = c->d_order;
-    a.beta_df = c->d_bdf;
-    a.acum_df = c->d_bdf ? c->d_bdf + cf.M : nullptr;
+    a.num_df = c->d_bdf;
+    a.code_pos = c->d_bdf ? reinterpret_cast<int *>(c->d_bdf + cf.M) : nullptr;
     a.form = cf.form;
     a.rkind = c->kind;
+    a.u = c->d_u;
+    a.z = c->d_z;
     if (c->use_round()) {
         a.B = c->RB;
         a.rmode = round_mode(c);
@@ -608,7 +610,6 @@ void brr::sweep_args(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, 
         a.rgram = c->d_rgram;
         a.rnz = c->d_rnz;
         a.rall = round_all_rows(c);
-        a.u = c->d_u;
         a.num_out = c->d_num;
         a.eps_out = c->d_eps2;
         a.eps_hi_out = c->d_eps_hi2;
@@ -754,7 +755,8 @@ int run_sweep(brr_ctx *c, double mu_new, double eps_total, brr_sweep_out *out, f
         BRR_CUDA(launch_sweep(cf.form, c->kind, a, smem, c->st));
     BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
     if (c->blocked)
-        BRR_CUDA(launch_block_finish(cf.M, c->d_chosen, a.beta_df, a.acum_df, c->d_beta, c->d_acum, c->st));
+        BRR_CUDA(launch_block_finish(cf.M, a.kmax, c->d_brec, a.num_df, a.code_pos, c->d_u, c->d_z, c->d_gconst,
+                                     c->d_gK, c->d_beta, c->d_acum, c->d_comp, c->d_chosen, c->st));
 
     rc = sweep_finish(c, out);
     if (rc)
@@ -850,14 +852,22 @@ int prepare_blocked(brr_ctx *c)
     }
     if (cf.spec_width == 0)
         c->B = 64;
-    SweepArgs a{};
-    a.B = c->B;
-    a.n_groups = cf.n_groups;
-    a.slice_max = c->slice_max;
-    a.slot_bytes = c->slot_bytes;
-    const size_t smem = sweep_block_smem_bytes(a);
+    // narrower blocks where the asked width's buffers do not fit beside the slices
     std::string occ_why;
-    const int per_sm = sweep_block_max_ctas_per_sm(smem, &occ_why);
+    int per_sm = 0;
+    for (const int widest = c->B;; c->B /= 2) {
+        SweepArgs a{};
+        a.B = c->B;
+        a.n_groups = cf.n_groups;
+        a.slice_max = c->slice_max;
+        a.slot_bytes = c->slot_bytes;
+        per_sm = sweep_block_max_ctas_per_sm(sweep_block_smem_bytes(a), &occ_why);
+        if ((per_sm >= 1 && (int64_t)per_sm * c->sms >= c->G) || c->B <= 8) {
+            if (per_sm < 1 || (int64_t)per_sm * c->sms < c->G)
+                c->B = widest;
+            break;
+        }
+    }
     if (per_sm < 1 || (int64_t)per_sm * c->sms < c->G) {
         if (cf.gram > 0)
             return fail(BRR_ERR_ARG, "the blocked sweep does not fit its CTAs: " +

@@ -8,10 +8,13 @@
 //
 // The sweep order is cut into blocks of B consecutive markers.  One CTA per SM
 // owns a slice of individuals and keeps its residual slice in shared memory in
-// fixed point, E = eps * 2^50 as a signed 64-bit integer stored as four
-// balanced 16-bit limbs.  Block q's dot products sum_i g_i E_i (g in {0,1,2}
-// the genotype) are exact integer sums: dp2a (two int16 x int8 products per
-// instruction) over the limbs, one warp per 8 markers; they are summed across
+// fixed point, E = eps * 2^50 as a signed 64-bit integer, and as seven balanced
+// 10-bit limbs in FP16 planes.  Block q's dot products sum_i g_i E_i (g in {0,1,2}
+// the genotype) are exact integer sums on the tensor cores: 16 markers x 8 limb
+// columns x 16 individuals per mma.sync, the genotypes decoded in registers from the
+// 2-bit codes (brr_mma.cuh; two words per 16 genotypes and marker against 26 dp2a
+// instructions before: 4.6k to 0.9k issue clocks per block of 64 at 660
+// individuals); they are summed across
 // CTAs by exact 128-bit fixed-point integer atomics, and a grid-wide counter
 // barrier publishes the sums.  The residual update adds dBeta * x rounded to
 // the 2^-50 grid.  Every CTA then
@@ -25,7 +28,7 @@
 // is being resolved.  When block t is resolved, the updates of blocks t-2 and
 // t-1 enter through the cross Gram entries G[p, t'] (p in block t-2: "far",
 // p in block t-1: "near", t' in block t).  Per CTA and iteration r:
-//   8 dot warps:            rank-U update of block r-1; cp.async of block
+//   12 dot warps:           rank-U update of block r-1; cp.async of block
 //                           r+3's code slices into the slot block r-1 held;
 //                           dots of block r+2, publish, arrive at barrier r+2;
 //   the resolve warp:       near corrections of block r-1 (Gram entries in
@@ -36,21 +39,20 @@
 //                           block r+3; zeroed accumulators of block r+4 (first
 //                           CTA); a non-blocking arrival on the dot warps'
 //                           named barrier; the Gram loads of block r+4;
-//                           outputs of block r-1;
 //   the input warp:         the far corrections of block r-1 for block r+1
 //                           (entries read from the staging slot in L2), then
 //                           wait for barrier r+1 (arrived one iteration
 //                           earlier) and assemble block r+1's inputs from its
 //                           published sums.
 // So neither the grid barrier's latency nor the input assembly is on the path
-// of the dot warps or of the resolve warp.  The ten warps other than the
+// of the dot warps or of the resolve warp.  The warps other than the
 // resolve warp iterate in step (named barrier 3 at the top of each iteration);
 // the resolve warp runs on its own, tied to them by two signals in shared
 // memory (mbarriers, two per signal by block parity):
-//   GO(q)        320 arrivals in the others' iteration q-1: the dot threads
-//                after block q-2's update, the input warp after block q's
-//                inputs, the chore warp after block q-2's outputs; so block q
-//                can be resolved while the others finish iteration q-1;
+//   GO(q)        one arrival per other thread in their iteration q-1: the dot
+//                threads after block q-2's update, the input warp after block
+//                q's inputs, the chore warp after its Gram loads; so block q can
+//                be resolved while the others finish iteration q-1;
 //   RESOLVED(q)  the resolve warp's 32 lanes after block q's decisions; the
 //                others wait for it at the top of iteration q+1.
 // Block q's decisions (parity q % 2) are read by the others in iteration q+1
@@ -92,6 +94,7 @@
 
 #include "brr_device.cuh"
 #include "brr_internal.h"
+#include "brr_mma.cuh"
 #include "brr_pick.cuh"
 
 
@@ -100,22 +103,19 @@ namespace brr {
 
 namespace {
 
-// Roles by warp.  Warp w issues from sub-partition w % 4: the eight dot warps
-// 0-7 put two on every sub-partition (their dot products and updates are the
-// longest role), and the resolve, input and chore warps 8-10 take the third
-// slot of sub-partitions 0-2.  Measured against the resolve warp alone with
-// the input warp on sub-partition 3 (three dot warps on sub-partitions 0 and
-// 1): 3 % more marker-updates/s at N = M = 100,000 although the resolve warp
-// now shares its sub-partition with two dot warps.
-constexpr int kDotWarps = 8;
-constexpr int kResolveWarp = 8;    // samples the blocks
-constexpr int kInputWarp = 9;      // grid barrier, inputs of the next block
-constexpr int kChoreWarp = 10;     // Gram copies and gathers, outputs
+// Roles by warp.  Warp w issues from sub-partition w % 4: the twelve dot warps
+// 0-11 put three on every sub-partition (their dot products and updates are the
+// longest role), and the resolve, input and chore warps 12-14 take the fourth
+// slot of sub-partitions 0-2.
+constexpr int kDotWarps = 12;
+constexpr int kResolveWarp = kDotWarps;        // samples the blocks
+constexpr int kInputWarp = kDotWarps + 1;      // grid barrier, inputs of the next block
+constexpr int kChoreWarp = kDotWarps + 2;      // Gram copies and gathers
 constexpr int kBlockThreads = (kDotWarps + 3) * 32;
-// index 0..7 of a dot warp, -1 for the other roles
+// index of a dot warp, -1 for the other roles
 __host__ __device__ constexpr int dot_index(int w) { return w < kDotWarps ? w : -1; }
 static_assert(kResolveWarp >= kDotWarps && kInputWarp >= kDotWarps && kChoreWarp >= kDotWarps,
-              "the dot warps are warps 0..7");
+              "the dot warps come first");
 constexpr int kAccBufs = 8;
 constexpr int kAccCopies = 8;   // CTA s adds into copy s % 8: 19 atomics per address and block, not 152
 constexpr int kAccBufWords = kAccCopies * kMaxSpec * 4;
@@ -137,12 +137,12 @@ __host__ __device__ inline size_t block_gram_entries(int B) { return (size_t)B *
 __host__ __device__ inline size_t block_stage_entries(int B) { return block_gram_entries(B) + (size_t)B * B; }
 
 struct PipePlan {
-    size_t planes;          // residual limb planes: 8 words per 4 individuals
-    size_t fix;             // residual in fixed point: one int64 per individual
+    size_t planes;          // residual limb planes (FP16)
+    size_t fix;             // residual in fixed point: one int64 per individual, in the planes' order
     size_t codes;           // R x slot_bytes genotype codes
     size_t recs;            // R x BlockRec
     size_t gram;            // 2 x block_gram_entries double-float Gram entries
-    size_t pairs;           // B(B-1)/2 x 2 bytes: pair positions (a < b)
+    size_t part;            // the dot warps' sums: 2 x kDotWarps tiles of 16 markers x 8 limb columns
     size_t gcf;             // n_groups x kMaxK x {dc, h}
     size_t gbf;             // n_groups x kMaxK x {sdk hi, lo, invden hi, lo}
     size_t mbar;            // 2 mbarriers of the Gram copies
@@ -155,7 +155,7 @@ __host__ __device__ inline PipePlan make_pipe_plan(int slice_max, int slot_bytes
     const size_t R = 4 * (size_t)B;
     size_t o = 0;
     p.planes = o;
-    o += al16((size_t)slice_max / 4 * 32);
+    o += al16((size_t)kLimbPlanes * limb_plane_stride(slice_max));
     p.fix = o;
     o += al16((size_t)slice_max * 8);
     p.codes = o;
@@ -164,8 +164,8 @@ __host__ __device__ inline PipePlan make_pipe_plan(int slice_max, int slot_bytes
     o += R * sizeof(BlockRec);
     p.gram = o;
     o += al16(2 * block_gram_entries(B) * sizeof(float2));
-    p.pairs = o;
-    o += al16((size_t)B * (B - 1) / 2 * 2);
+    p.part = o;
+    o += 2 * kDotWarps * 16 * 8 * sizeof(float);
     p.gcf = o;
     o += al16((size_t)n_groups * kMaxK * 2 * sizeof(float));
     p.gbf = o;
@@ -241,24 +241,24 @@ __device__ __forceinline__ long long clk()
     return t;
 }
 
-__device__ __forceinline__ void dot_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void dot_warps_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kDotWarps * 32) : "memory"); }
 
 // Before the arrival at a grid barrier the dot warps wait on named barrier 2
 // for their own work and for the chore warp's staging stores; the chore warp
 // only signals it and goes on.
-__device__ __forceinline__ void arrive_sync() { asm volatile("bar.sync 2, 288;" ::: "memory"); }
-__device__ __forceinline__ void chore_signal() { asm volatile("bar.arrive 2, 288;" ::: "memory"); }
+__device__ __forceinline__ void arrive_sync() { asm volatile("bar.sync 2, %0;" ::"n"(kDotWarps * 32 + 32) : "memory"); }
+__device__ __forceinline__ void chore_signal() { asm volatile("bar.arrive 2, %0;" ::"n"(kDotWarps * 32 + 32) : "memory"); }
 
-// The ten warps other than the resolve warp: iteration barrier (named barrier
-// 3) with the OR of a flag over its 320 threads.
-constexpr int kOtherThreads = 320;
+// The warps other than the resolve warp: iteration barrier (named barrier 3)
+// with the OR of a flag over its threads.
+constexpr int kOtherThreads = kDotWarps * 32 + 64;
 __device__ __forceinline__ bool others_any(bool v)
 {
     unsigned r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 3, 320, q;\n\t"
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 3, %2, q;\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(r)
-                 : "r"((unsigned)v)
+                 : "r"((unsigned)v), "n"(kOtherThreads)
                  : "memory");
     return r != 0;
 }
@@ -272,51 +272,9 @@ __device__ __forceinline__ float2 ld_relaxed_f2(const float2 *p)
     return v;
 }
 
-// ---- fixed-point residual: E = eps * 2^kFrac, |E| < 2^62, as four balanced
-// 16-bit limbs E = l0 + l1 2^16 + l2 2^32 + l3 2^48 (l_k in [-2^15, 2^15)).
-// The limb planes of 4 individuals i0..i3 (byte position b of the codes) are 8
-// words: limb k's pair (i0, i1) at word 2(k ^ (b & 3)) and (i2, i3) at the next
-// word, each pair as two int16 (low half first).  The XOR with b & 3 makes the
-// lane that reads position b see the limbs in the order its reduction wants.
+// ---- fixed-point residual: E = eps * 2^kFrac, |E| < 2^62.
 constexpr int kFrac = 50;
 constexpr long long kFixMax = 1ll << 62;
-
-// A code byte (4 individuals, 2 bits each) as the byte selector of __byte_perm:
-// code k of the byte in bits 4k..4k+1 of the result.  Selecting from
-// kGenoBytes gives the 4 genotype bytes (code 0: 2, 2: 1, 1 and 3: 0), from
-// kMissBytes the 4 missing-indicator bytes (code 1), with no table lookup.
-constexpr unsigned kGenoBytes = 0x00010002u;
-constexpr unsigned kMissBytes = 0x00000100u;
-__device__ __forceinline__ unsigned code_nibbles(unsigned v)
-{
-    const unsigned x = (v | (v << 4)) & 0x0F0Fu;
-    return (x | (x << 2)) & 0x3333u;
-}
-
-__device__ __forceinline__ void split_limbs(long long E, int (&l)[4])
-{
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        l[k] = (int)((E << 48) >> 48);
-        E = (E - l[k]) >> 16;
-    }
-    l[3] = (int)E;
-}
-
-__device__ __forceinline__ void store_fix4(uint32_t *planes, int b, const long long (&E)[4])
-{
-    uint2 *w = reinterpret_cast<uint2 *>(planes + 8 * b);
-    const int p = b & 3;
-    int l0[4], l1[4], l2[4], l3[4];
-    split_limbs(E[0], l0);
-    split_limbs(E[1], l1);
-    split_limbs(E[2], l2);
-    split_limbs(E[3], l3);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        w[k ^ p] = make_uint2(__byte_perm((unsigned)l0[k], (unsigned)l1[k], 0x5410),
-                              __byte_perm((unsigned)l2[k], (unsigned)l3[k], 0x5410));
-}
 
 // Double-float value to the fixed-point grid (truncation below 2^-60, then
 // rounding to the nearest multiple of 2^-kFrac); false when out of range.
@@ -372,10 +330,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *m, unsigned parity, uint64_t
 
 // Records of the Gram-blocked FP32C dense sweep (all markers in parallel, the
 // FP64 work of the sweep's per-marker constants done once here).
+template <int KM>
 __global__ void k_gather_block(const uint32_t *__restrict__ order, int64_t M, int64_t N,
                                const double *__restrict__ table, const double *__restrict__ scale,
                                const double *__restrict__ beta, const double *__restrict__ u,
                                const double *__restrict__ z, const int32_t *__restrict__ group, double S,
+                               const double *__restrict__ gconst, const int32_t *__restrict__ gK,
                                BlockRec *__restrict__ rec)
 {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -396,29 +356,69 @@ __global__ void k_gather_block(const uint32_t *__restrict__ order, int64_t M, in
     df_from_double(z[j], r.zf[0], r.zf[1]);
     r.uf = __double2float_rn(u[j]);
     r.bnz = bo != 0.0 ? 1u : 0u;
-    r.beta_old = bo;
-    r.u = u[j];
-    r.z = z[j];
     r.j = j;
     r.group = group[j];
-    r.pad[0] = r.pad[1] = r.pad[2] = r.pad[3] = 0u;
+    r.s0 = certain_zero<KM>(r.uf, gconst + (size_t)r.group * kMaxK * 4, gK[r.group]);
+    r.pad = 0u;
     rec[q] = r;
 }
 
-// After a blocked sweep: FP64 beta (markers that chose a component) and acum.
-__global__ void k_block_finish(int64_t M, const uint8_t *__restrict__ chosen, const float2 *__restrict__ beta_df,
-                               const float2 *__restrict__ acum_df, double *__restrict__ beta,
-                               double *__restrict__ acum)
+// After a blocked sweep, one thread per sweep position: beta (markers that chose a
+// component: z * sdk + num * invden in double-float, 0 for component 0), acum
+// (P(component 0) of the FP32 sampler at the final num, or of the FP64 evaluation
+// that decided), chosen flag and component, by marker id.  code: component & 0xFF |
+// FP64 decision << 8.
+template <int KM>
+__global__ void k_block_finish(int64_t M, const BlockRec *__restrict__ rec, const float2 *__restrict__ num,
+                               const int *__restrict__ code, const double *__restrict__ u,
+                               const double *__restrict__ z, const double *__restrict__ gconst,
+                               const int32_t *__restrict__ gK, double *__restrict__ beta, double *__restrict__ acum,
+                               int32_t *__restrict__ comp, uint8_t *__restrict__ chosen)
 {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= M)
+    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= M)
         return;
-    const float2 a = acum_df[j];
-    acum[j] = __dadd_rn((double)a.x, (double)a.y);
-    if (chosen[j]) {
-        const float2 b = beta_df[j];
-        beta[j] = __dadd_rn((double)b.x, (double)b.y);
+    const BlockRec &r = rec[q];
+    const int oc = code[q], K = gK[r.group];
+    const int c = (oc & 0x80) ? -1 : (oc & 0xFF);
+    const float2 x = num[q];
+    const double *gc = gconst + (size_t)r.group * kMaxK * 4;
+    if (oc & 0x100) {
+        const Pick p = pick_marker<false, KM>((double)x.x + (double)x.y, u[r.j], z[r.j], beta[r.j], gc, K);
+        float h, l;
+        df_from_double(p.acum0, h, l);
+        acum[r.j] = __dadd_rn((double)h, (double)l);
+        if (c >= 0) {
+            df_from_double(c > 0 ? p.beta : 0.0, h, l);
+            beta[r.j] = __dadd_rn((double)h, (double)l);
+        }
+    } else {
+        float gcf[2 * KM];
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+            gcf[2 * k] = k == 0 ? 0.f : (float)(gc[4 * k] - gc[0]);
+            gcf[2 * k + 1] = k == 0 ? 0.f : (float)gc[4 * k + 2];
+        }
+        int c2;
+        float a0;
+        pick_f32<KM>(x.x, x.y, r.uf, gcf, K, c2, a0);
+        acum[r.j] = (double)a0;
+        if (c >= 0) {
+            float bh = 0.f, bl = 0.f;
+            if (c > 0) {
+                float sh, sl, ih, il, ph, pl;
+                df_from_double(gc[4 * c + 3], sh, sl);
+                df_from_double(gc[4 * c + 1], ih, il);
+                df_mul(r.zf[0], r.zf[1], sh, sl, bh, bl);
+                df_mul(x.x, x.y, ih, il, ph, pl);
+                df_add(bh, bl, ph, pl);
+            }
+            beta[r.j] = __dadd_rn((double)bh, (double)bl);
+        }
     }
+    chosen[r.j] = c >= 0 ? 1 : 0;
+    if (c >= 0)
+        comp[r.j] = c;
 }
 
 // One halving exchange of a warp's reduce-scatter over double-float sums:
@@ -447,75 +447,12 @@ __device__ __forceinline__ void df_xor_add(float &h, float &l, int off)
     df_add(h, l, rh, rl);
 }
 
-// Outputs of one resolved block, written by one warp of the CTA whose turn it
-// is (block q by CTA q mod G, one iteration later, off the critical path): new
-// beta as double-float (z * sdk + num * invden for a component k > 0, 0 for
-// component 0), acum (P(component 0) of the FP32 sampler at the final num, or
-// of the FP64 evaluation), chosen flag and component, by marker id.
-struct BlockOut {
-    float2 x[kMaxSpec];   // final num (double-float)
-    float2 fb[kMaxSpec];  // beta of an FP64 decision
-    float2 fa[kMaxSpec];  // acum of an FP64 decision
-    float2 zf[kMaxSpec];  // z
-    float uf[kMaxSpec];
-    uint32_t j[kMaxSpec];
-    int group[kMaxSpec];
-    int code[kMaxSpec];   // comp & 0xFF | FP64 decision << 8; -2: no marker
-};
-
-template <int KM>
-__device__ __forceinline__ void write_block_outputs(const SweepArgs &a, const BlockOut &o, const float *gcf,
-                                                    const int32_t *gk, const float *gbf, int lane)
-{
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int m = lane + 32 * h;
-        const int oc = o.code[m];
-        if (oc == -2)
-            continue;
-        const int c = (oc & 0x80) ? -1 : (oc & 0xFF);
-        const bool fp64 = (oc & 0x100) != 0;
-        const int g = o.group[m];
-        const float2 x = o.x[m];
-        float bh = 0.f, bl = 0.f;
-        float2 acum;
-        if (fp64) {
-            if (c > 0) {
-                bh = o.fb[m].x;
-                bl = o.fb[m].y;
-            }
-            acum = o.fa[m];
-        } else {
-            if (c > 0) {
-                const float4 gc = reinterpret_cast<const float4 *>(gbf + (size_t)g * kMaxK * 4)[c];
-                float ph, pl;
-                df_mul(o.zf[m].x, o.zf[m].y, gc.x, gc.y, bh, bl);
-                df_mul(x.x, x.y, gc.z, gc.w, ph, pl);
-                df_add(bh, bl, ph, pl);
-            }
-            int c2;
-            float a0;
-            pick_f32<KM>(x.x, x.y, o.uf[m], gcf + (size_t)g * kMaxK * 2, gk[g], c2, a0);
-            acum = make_float2(a0, 0.f);
-        }
-        const uint32_t j = o.j[m];
-        a.beta_df[j] = make_float2(bh, bl);
-        a.acum_df[j] = acum;
-        a.chosen[j] = c >= 0 ? 1 : 0;
-        if (c >= 0)
-            a.comp[j] = c;
-    }
-}
-
-// One CTA of 11 warps per SM (8 dot warps, the resolve, chore and input
-// warps).  The register file is split between the SM's four sub-partitions
-// (16K registers each) and warps are placed round-robin, so the sub-partitions
-// holding three warps bound every thread to 168 registers: the launch bound is
-// stated for 12 warps to give the compiler that limit.  PROF: the variant that
-// counts phase cycles on the first CTA (the clock reads constrain the code's
-// scheduling, so the plain variant has none).
+// One CTA of 15 warps per SM (12 dot warps, the resolve, input and chore warps) at
+// 128 registers a thread.  PROF: the variant that counts phase cycles on the first
+// CTA (the clock reads constrain the code's scheduling, so the plain variant has
+// none).
 template <int KM, bool MISS, bool PROF>
-__global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
+__global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     // per block parity: residual-changing markers of the block (positions,
@@ -526,10 +463,8 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
     __shared__ int s_nupd[2];
     __shared__ float2 s_inum[2][kMaxSpec];   // num from the block's dot products (double-float)
     __shared__ float s_iuf[2][kMaxSpec];
-    __shared__ unsigned s_imeta[2][kMaxSpec]; // group | K << 8 | (beta_old != 0) << 16
-    __shared__ float s_H[kMaxGroups];
+    __shared__ float s_is0[2][kMaxSpec];      // num^2 above which the marker may change
     __shared__ int32_t s_gk[kMaxGroups];
-    __shared__ BlockOut s_out[2];
     __shared__ long long s_D[kMaxSpec][4];   // residual change per update and code, fixed point
     __shared__ unsigned s_uoff[kMaxSpec];    // offset of each update's codes in the ring
     // marker ids of blocks q (slot q % kIdSlots), copied from the sweep order
@@ -538,7 +473,7 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
     __shared__ __align__(16) uint32_t s_ids[kIdSlots][kMaxSpec];
     __shared__ int s_abort;
     __shared__ int s_cp_issued;
-    // resolve warp <-> other warps: GO(q) on s_mb[q & 1] (320 arrivals: the dot
+    // resolve warp <-> other warps: GO(q) on s_mb[q & 1] (one arrival per thread: the dot
     // threads after block q-2's update, the input warp after block q's inputs,
     // the chore warp after block q-2's outputs), RESOLVED(q) on s_mb[2 + (q & 1)]
     // (the resolve warp's 32 lanes after block q's decisions)
@@ -546,14 +481,15 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
 
     const int B = a.B;
     const unsigned Bu = (unsigned)B;
+    const int lB = 31 - __clz(B);                         // B is a power of two
     const unsigned R = 4u * Bu;
     const unsigned Rm = R - 1u;
     const int sidx = blockIdx.x;
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int dw = dot_index(warp);                       // dot warps: 0..7
-    const int dtid = dw >= 0 ? dw * 32 + lane : kBlockThreads;   // dot warps: 0..255
-    const int otid = tid - (warp > kResolveWarp ? 32 : 0);       // the other warps: 0..319
+    const int dw = dot_index(warp);
+    const int dtid = dw >= 0 ? dw * 32 + lane : kBlockThreads;   // dot warps: 0 ..
+    const int otid = tid - (warp > kResolveWarp ? 32 : 0);       // the warps but the resolve warp: 0 ..
     const int lo = a.slice_lo[sidx];
     const int ns = a.slice_lo[sidx + 1] - lo;
     const int nbytes = ((ns + kChunk - 1) / kChunk) * 16;
@@ -566,12 +502,13 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
     const int nblk = (int)((M32 + Bu - 1) / Bu);
     auto nb_of = [&](int q) { return (int)min(Bu, M32 - (unsigned)q * Bu); };
 
-    uint32_t *planes = reinterpret_cast<uint32_t *>(smem + plan.planes);
+    unsigned char *planes = smem + plan.planes;
+    const int pstride = limb_plane_stride(a.slice_max);
+    float *part = reinterpret_cast<float *>(smem + plan.part);
     long long *fix = reinterpret_cast<long long *>(smem + plan.fix);
     uint8_t *ring_codes = smem + plan.codes;
     BlockRec *ring_rec = reinterpret_cast<BlockRec *>(smem + plan.recs);
     float2 *gbuf = reinterpret_cast<float2 *>(smem + plan.gram);
-    uint8_t *pair_ab = smem + plan.pairs;
     float *gcf = reinterpret_cast<float *>(smem + plan.gcf);
     float *gbf = reinterpret_cast<float *>(smem + plan.gbf);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + plan.mbar);
@@ -581,12 +518,14 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
     {
         float muh, mul;
         df_from_double(-a.mu_new, muh, mul);
-        for (int b = tid; b < a.slice_max / 4; b += kBlockThreads) {
-            long long E[4];
+        for (int i = tid; i < pstride / 4; i += kBlockThreads)
+            reinterpret_cast<unsigned *>(planes + (size_t)3 * pstride)[i] = 0u;
+        for (int pr = tid; pr < a.slice_max / 2; pr += kBlockThreads) {
+            long long E[2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 2; ++i) {
                 E[i] = 0;
-                const int ii = 4 * b + i;
+                const int ii = limb_individual(2 * pr + i);
                 if (ii < ns) {
                     float h = a.eps_hi[lo + ii], l = a.eps_lo[lo + ii];
                     df_add(h, l, muh, mul);
@@ -596,20 +535,12 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
                     }
                 }
             }
-            store_fix4(planes, b, E);
-            reinterpret_cast<longlong2 *>(fix)[2 * b] = make_longlong2(E[0], E[1]);
-            reinterpret_cast<longlong2 *>(fix)[2 * b + 1] = make_longlong2(E[2], E[3]);
+            put_limbs(planes, pstride, pr, E[0], E[1]);
+            reinterpret_cast<longlong2 *>(fix)[pr] = make_longlong2(E[0], E[1]);
         }
     }
     for (int i = tid; i < a.n_groups; i += kBlockThreads) {
         s_gk[i] = a.gK[i];
-        const double *row = a.gconst + (size_t)i * kMaxK * 4;
-        double hmax = 0.0, hmin = 0.0;
-        for (int k = 1; k < a.gK[i]; ++k) {
-            hmax = fmax(hmax, row[4 * k + 2]);
-            hmin = fmin(hmin, row[4 * k + 2]);
-        }
-        s_H[i] = (float)((hmax - hmin) * (1.0 + 1e-6));
     }
     for (int i = tid; i < a.n_groups * kMaxK; i += kBlockThreads) {
         const int g = i / kMaxK, k = i - g * kMaxK;
@@ -619,12 +550,6 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
         df_from_double(row[4 * k + 3], gbf[4 * i], gbf[4 * i + 1]);
         df_from_double(row[4 * k + 1], gbf[4 * i + 2], gbf[4 * i + 3]);
     }
-    for (int pb = 1 + tid; pb < B; pb += kBlockThreads)
-        for (int pa = 0; pa < pb; ++pa) {
-            const int p = pb * (pb - 1) / 2 + pa;
-            pair_ab[2 * p] = (uint8_t)pa;
-            pair_ab[2 * p + 1] = (uint8_t)pb;
-        }
     if (tid == 0) {
         s_abort = 0;
         s_nupd[0] = 0;
@@ -703,25 +628,27 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
         const int nbq = nb_of(q);
         unsigned pa, pb, qa;
         if (e < (unsigned)npairs) {
-            pa = pair_ab[2 * e];
-            pb = pair_ab[2 * e + 1];
+            // e = pb (pb - 1) / 2 + pa with pa < pb
+            pb = (unsigned)((1.f + __fsqrt_rn(8.f * (float)e + 1.f)) * 0.5f);
+            if (pb * (pb - 1u) / 2u > e)
+                --pb;
+            pa = e - pb * (pb - 1u) / 2u;
             if ((int)pb >= nbq)
                 return false;
             qa = q0 + pa;
         } else {
             // near (block q-1) or far (block q-2) entries; those blocks are full
             const unsigned c = e - (unsigned)npairs;
-            const unsigned back = c < Bu * Bu ? 1u : 2u;
+            const unsigned back = 1u + (c >> (2 * lB));
             if ((unsigned)q < back)
                 return false;
-            const unsigned cc = c - (back - 1u) * Bu * Bu;
-            pa = cc / Bu;
-            pb = cc - pa * Bu;
+            pa = (c >> lB) & (Bu - 1u);
+            pb = c & (Bu - 1u);
             if ((int)pb >= nbq)
                 return false;
             qa = q0 - back * Bu + pa;
         }
-        const int64_t ja = s_ids[(qa / Bu) % kIdSlots][qa % Bu], jb = s_ids[q % kIdSlots][pb];
+        const int64_t ja = s_ids[(qa >> lB) % kIdSlots][qa & (Bu - 1u)], jb = s_ids[q % kIdSlots][pb];
         const int64_t hi = ja > jb ? ja : jb, lw = ja > jb ? jb : ja;
         *out = __ldg(&a.gram[hi * (hi - 1) / 2 + lw]);
         return true;
@@ -749,98 +676,46 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
         }
     };
 
-    auto publish = [&](unsigned long long *acc, __int128 x) {
-        const Fx f = fx_split(x);
-        red_add_u64(acc, (unsigned long long)f.hi);
-        red_add_u64(acc + 1, f.lo);
-    };
-
     // ---- partial dot products of block q against the current residual (dot
-    // warps), exact in integers.  Warp w owns markers w, w+8, ..., w+56 of the
-    // block; its lanes stride over the slice's code bytes (lane l reads byte
-    // positions b = l mod 32).  Accumulator slot s = 4 m' + k' of lane l holds
-    // marker w + 8 (m' ^ (l >> 2)) and limb k' ^ (l & 3) (the plane order of its
-    // byte positions), so value s of lane l is value s ^ l of the warp and the
-    // reduction is a butterfly without selects: after it lane l holds limb
-    // l & 3 of marker w + 8 (l >> 2), and four lanes combine a marker's limbs.
+    // warps), exact in integers: tiles of 16 markers, the warps of a tile sharing the
+    // slice's 64-individual chunks; the tiles' sums meet in shared memory and
+    // thread (m, word) publishes a marker's low or high word (sum = high 2^30 + low).
+    // Rows past the end of a short block read a stale slot; their sums are never
+    // published.
+    const int nmt = B <= 16 ? 1 : B / 16, nkg = kDotWarps / nmt;
+    const int nchunk = nbytes / 16;
     auto dot_block = [&](int q) {
         const unsigned q0 = (unsigned)q * Bu;
         const int nbq = nb_of(q);
-        constexpr int MPW = kMaxSpec / 8;
-        int A[MPW * 4], Mx[MPW * 4];
-        unsigned cofs[MPW];
-#pragma unroll
-        for (int k = 0; k < MPW; ++k) {
-            // markers past the end of a short block read a stale slot; their
-            // sums are never published
-            const unsigned m = (unsigned)dw + 8u * ((unsigned)k ^ (unsigned)(lane >> 2));
-            cofs[k] = ((q0 + m) & Rm) * (unsigned)a.slot_bytes;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                A[4 * k + t] = 0;
-                Mx[4 * k + t] = 0;
-            }
+        const int fg = lane >> 2, fq = lane & 3;
+        const int mt = dw % nmt, kg = dw / nmt;
+        const uint8_t *ra = ring_codes + (size_t)((q0 + 16 * mt + fg) & Rm) * a.slot_bytes + 4 * fq;
+        const uint8_t *rb = ring_codes + (size_t)((q0 + 16 * mt + fg + 8) & Rm) * a.slot_bytes + 4 * fq;
+        const unsigned char *pb = planes + (size_t)fg * pstride + 32 * fq;
+        float c[4] = {0.f, 0.f, 0.f, 0.f}, cm[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int ch = kg; ch < nchunk; ch += nkg) {
+            const unsigned w0 = *reinterpret_cast<const unsigned *>(ra + 16 * ch);
+            const unsigned w1 = *reinterpret_cast<const unsigned *>(rb + 16 * ch);
+            const uint4 x = *reinterpret_cast<const uint4 *>(pb + 128 * ch);
+            const uint4 y = *reinterpret_cast<const uint4 *>(pb + 128 * ch + 16);
+            mma_chunk(c, w0, w1, kGenoTable, x, y);
+            if (MISS)
+                mma_chunk(cm, w0, w1, kMissTable, x, y);
         }
-        // all 8 slots are summed; with B < 64 the slots past the block read ring
-        // slots of other blocks and are never published
-        for (int b = lane; b < nbytes; b += 32) {
-            const uint4 w0 = reinterpret_cast<const uint4 *>(planes)[2 * b];
-            const uint4 w1 = reinterpret_cast<const uint4 *>(planes)[2 * b + 1];
-            const int wv[8] = {(int)w0.x, (int)w0.y, (int)w0.z, (int)w0.w,
-                               (int)w1.x, (int)w1.y, (int)w1.z, (int)w1.w};
-#pragma unroll
-            for (int k = 0; k < MPW; ++k) {
-                const unsigned v = ring_codes[cofs[k] + b];
-                const unsigned sel = code_nibbles(v);
-                const int g = (int)__byte_perm(kGenoBytes, 0u, sel);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    A[4 * k + t] = __dp2a_lo(wv[2 * t], g, A[4 * k + t]);
-                    A[4 * k + t] = __dp2a_hi(wv[2 * t + 1], g, A[4 * k + t]);
-                }
-                if (MISS) {
-                    const int mm = (int)__byte_perm(kMissBytes, 0u, sel);
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        Mx[4 * k + t] = __dp2a_lo(wv[2 * t], mm, Mx[4 * k + t]);
-                        Mx[4 * k + t] = __dp2a_hi(wv[2 * t + 1], mm, Mx[4 * k + t]);
-                    }
-                }
-            }
+        float2 *dst = reinterpret_cast<float2 *>(part + ((size_t)dw * 16 + fg) * 8) + fq;
+        dst[0] = make_float2(c[0], c[1]);
+        dst[32] = make_float2(c[2], c[3]);
+        if (MISS) {
+            dst[kDotWarps * 64] = make_float2(cm[0], cm[1]);
+            dst[kDotWarps * 64 + 32] = make_float2(cm[2], cm[3]);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int i = 0; i < o; ++i) {
-                A[i] += __shfl_xor_sync(0xffffffffu, A[i + o], o);
-                if (MISS)
-                    Mx[i] += __shfl_xor_sync(0xffffffffu, Mx[i + o], o);
-            }
-        }
-        // limb l & 3 of marker w + 8 (l >> 2): combine the four limbs (int128)
-        const int limb = lane & 3;
-        auto combine = [&](int v) {
-            __int128 x = (__int128)(long long)v << (16 * limb);
-            unsigned long long xl = (unsigned long long)x, xh = (unsigned long long)(x >> 64);
-#pragma unroll
-            for (int o = 1; o <= 2; o <<= 1) {
-                const unsigned long long yl = __shfl_xor_sync(0xffffffffu, xl, o);
-                const unsigned long long yh = __shfl_xor_sync(0xffffffffu, xh, o);
-                const unsigned long long sl = xl + yl;
-                xh = xh + yh + (sl < xl ? 1ull : 0ull);
-                xl = sl;
-            }
-            return (__int128)(((unsigned __int128)xh << 64) | xl);
-        };
-        const __int128 T = combine(A[0]);
-        const __int128 Tm = MISS ? combine(Mx[0]) : (__int128)0;
-        const int m = dw + 8 * (lane >> 2);
-        if (limb == 0 && m < nbq) {
-            unsigned long long *acc =
-                a.acc + (size_t)(q % kAccBufs) * kAccBufWords + ((size_t)(sidx % kAccCopies) * kMaxSpec + m) * 4;
-            publish(acc, T << (60 - kFrac));
-            if (MISS && Tm != 0)
-                publish(acc + 2, Tm << (60 - kFrac));
+        dot_warps_sync();
+        const int m = dtid & 63, word = (dtid >> 6) & 1, half = dtid >> 7;
+        if (m < nbq && half < (MISS ? 2 : 1)) {
+            const long long v = limb_sum(part + (size_t)half * kDotWarps * 16 * 8, m, word, nkg, nmt * 32);
+            red_add_u64(a.acc + (size_t)(q % kAccBufs) * kAccBufWords +
+                            ((size_t)(sidx % kAccCopies) * kMaxSpec + m) * 4 + 2 * half + word,
+                        (unsigned long long)v);
         }
     };
     auto arrive = [&](int q) {
@@ -904,43 +779,42 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
         // The sum of the residual is left as it was at the sweep start: the
         // standardised columns sum to zero, so a dense update moves it only
         // by rounding (dBeta times a column sum of order 1e-11).
-        for (int b = dtid; b < nbytes; b += kDotWarps * 32) {
-            const longlong2 e01 = reinterpret_cast<const longlong2 *>(fix)[2 * b];
-            const longlong2 e23 = reinterpret_cast<const longlong2 *>(fix)[2 * b + 1];
-            long long E[4] = {e01.x, e01.y, e23.x, e23.y};
-            // four updates' code bytes loaded at a time
+        long long top = 0;
+        for (int pr = dtid; pr < 32 * nchunk; pr += kDotWarps * 32) {
+            longlong2 e = reinterpret_cast<const longlong2 *>(fix)[pr];
+            const int sh = limb_pair_shift(pr);
+            const unsigned at = 4u * (unsigned)(pr >> 3);
+            // four updates' code words loaded at a time
             int u = 0;
             for (; u + 4 <= U; u += 4) {
-                unsigned v[4];
+                unsigned w[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    v[k] = ring_codes[s_uoff[u + k] + b];
+                    w[k] = *reinterpret_cast<const unsigned *>(ring_codes + s_uoff[u + k] + at) >> sh;
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        E[i] += s_D[u + k][(v[k] >> (2 * i)) & 3u];
-            }
-            for (; u < U; ++u) {
-                const unsigned v = ring_codes[s_uoff[u] + b];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    E[i] += s_D[u][(v >> (2 * i)) & 3u];
-            }
-            // padding individuals past the slice end keep a zero residual
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (4 * b + i >= ns)
-                    E[i] = 0;
-                if (E[i] >= kFixMax || E[i] <= -kFixMax) {
-                    atomicCAS(a.err, kDevOk, kDevRange);
-                    E[i] = 0;
+                for (int k = 0; k < 4; ++k) {
+                    e.x += s_D[u + k][w[k] & 3u];
+                    e.y += s_D[u + k][(w[k] >> 8) & 3u];
+                    top |= (e.x ^ (e.x << 1)) | (e.y ^ (e.y << 1));
                 }
             }
-            reinterpret_cast<longlong2 *>(fix)[2 * b] = make_longlong2(E[0], E[1]);
-            reinterpret_cast<longlong2 *>(fix)[2 * b + 1] = make_longlong2(E[2], E[3]);
-            store_fix4(planes, b, E);
+            for (; u < U; ++u) {
+                const unsigned w = *reinterpret_cast<const unsigned *>(ring_codes + s_uoff[u] + at) >> sh;
+                e.x += s_D[u][w & 3u];
+                e.y += s_D[u][(w >> 8) & 3u];
+                top |= (e.x ^ (e.x << 1)) | (e.y ^ (e.y << 1));
+            }
+            // padding individuals past the slice end keep a zero residual
+            const int ind = limb_individual(2 * pr);
+            if (ind >= ns)
+                e.x = 0;
+            if (ind + 4 >= ns)
+                e.y = 0;
+            reinterpret_cast<longlong2 *>(fix)[pr] = e;
+            put_limbs(planes, pstride, pr, e.x, e.y);
         }
+        if (top < 0)   // some |E| reached 2^62
+            atomicCAS(a.err, kDevOk, kDevRange);
         if (tid == 0)
             stamp(q + 1, 14);
         dot_warps_sync();
@@ -1026,48 +900,45 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
         if (!ok)
             return;
         // the published sums of the lane's two markers, every load issued
-        // before the first use; the copies' 56-bit low words sum to less than
-        // 2^64 (152 parts at most)
+        // before the first use
         const unsigned long long *accb = a.acc + (size_t)(q % kAccBufs) * kAccBufWords;
-        long long th64[2] = {0, 0}, sh64[2] = {0, 0};
-        unsigned long long tl64[2] = {0ull, 0ull}, sl64[2] = {0ull, 0ull};
+        long long th64[2] = {0, 0}, sh64[2] = {0, 0}, tl64[2] = {0, 0}, sl64[2] = {0, 0};   // high and low words
 #pragma unroll
         for (int c = 0; c < kAccCopies; ++c) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const unsigned long long *ac = accb + ((size_t)c * kMaxSpec + lane + 32 * h) * 4;
-                th64[h] += (long long)ld_relaxed_u64(ac);
-                tl64[h] += ld_relaxed_u64(ac + 1);
+                tl64[h] += (long long)ld_relaxed_u64(ac);
+                th64[h] += (long long)ld_relaxed_u64(ac + 1);
                 if (MISS) {
-                    sh64[h] += (long long)ld_relaxed_u64(ac + 2);
-                    sl64[h] += ld_relaxed_u64(ac + 3);
+                    sl64[h] += (long long)ld_relaxed_u64(ac + 2);
+                    sh64[h] += (long long)ld_relaxed_u64(ac + 3);
                 }
             }
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int m = lane + 32 * h;
-            float nh = 0.f, nl = 0.f, uf = 2.f;
-            unsigned meta = 2u << 8;
+            float nh = 0.f, nl = 0.f, uf = 2.f, s0 = INFINITY;
             if (m < nbq) {
                 const BlockRec &rc = ring_rec[(qb + m) & Rm];
                 float th, tl;
-                fx_to_df(th64[h], tl64[h], th, tl);
+                fixed_to_df(th64[h], tl64[h], -kFrac, th, tl);
                 df_mul(rc.sig[0], rc.sig[1], th, tl, nh, nl);
                 df_add(nh, nl, rc.cst[0], rc.cst[1]);
                 if (MISS) {
                     float sh, sl, qh, ql;
-                    fx_to_df(sh64[h], sl64[h], sh, sl);
+                    fixed_to_df(sh64[h], sl64[h], -kFrac, sh, sl);
                     df_mul(rc.dm[0], rc.dm[1], sh, sl, qh, ql);
                     df_add(nh, nl, qh, ql);
                 }
                 df_add(nh, nl, fh[h], fl[h]);
                 uf = rc.uf;
-                meta = (unsigned)rc.group | ((unsigned)s_gk[rc.group] << 8) | (rc.bnz ? 1u << 16 : 0u);
+                s0 = rc.bnz ? -1.f : rc.s0;   // a marker with an old effect always may
             }
             s_inum[par][m] = make_float2(nh, nl);
             s_iuf[par][m] = uf;
-            s_imeta[par][m] = meta;
+            s_is0[par][m] = s0;
         }
         if (prof) {
             const long long t2 = clk();
@@ -1092,6 +963,7 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
     __syncthreads();
     if (dw >= 0) {
         dot_block(0);
+        dot_warps_sync();
         if (nblk > 1)
             dot_block(1);
         arrive_sync();
@@ -1151,6 +1023,7 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
         // ---- resolve warp: block r once GO(r) (inputs of block r, the
         // residual-changing markers of block r-2 applied and read, its outputs
         // read), then RESOLVED(r)
+        int turn = 0;   // r mod G
         for (; r < nblk; ++r) {
             const bool ok = role_wait(&s_mb[r & 1], (unsigned)((r >> 1) & 1));
             if (__any_sync(0xffffffffu, !ok || *(volatile int *)&s_abort != 0))
@@ -1165,9 +1038,8 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
             mark(prof_r, 8);
             {
                 const int par = r & 1;
-                float nh[2], nl[2], ufr[2];
-                int grp[2], kk[2];
-                bool own[2], bnz[2];
+                float nh[2], nl[2], s0[2];
+                bool own[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int m = lane + 32 * h;
@@ -1175,11 +1047,7 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
                     const float2 n = s_inum[par][m];
                     nh[h] = n.x;
                     nl[h] = n.y;
-                    ufr[h] = s_iuf[par][m];
-                    const unsigned meta = s_imeta[par][m];
-                    grp[h] = (int)(meta & 0xFFu);
-                    kk[h] = (int)((meta >> 8) & 0xFFu);
-                    bnz[h] = (meta >> 16) != 0u;
+                    s0[h] = s_is0[par][m];
                 }
                 // Gram entries of block r (copied one iteration ahead)
                 bool gok = mbar_wait(&mbar[r & 1], (unsigned)((r >> 1) & 1), a.timeout_ns);
@@ -1214,177 +1082,121 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
                     mark(prof_r, 7);
 
 
-                    // ---- resolve block r: lane l owns markers l and l+32; a
-                    // decision is kept while its certified margin covers the move of
-                    // num^2; ballots find the first residual-changing marker p, the
-                    // later markers move by dBeta_p * G[p, t]
-                    float ch[2] = {0.f, 0.f}, cl[2] = {0.f, 0.f};
-                    float fbh[2] = {0.f, 0.f}, fbl[2] = {0.f, 0.f}, fah[2] = {0.f, 0.f}, fal[2] = {0.f, 0.f};
-                    float sref[2] = {0.f, 0.f}, wmar[2] = {-1.f, -1.f}, hg[2];
-                    int comp[2] = {-1, -1};
+                    // ---- resolve block r: lane l owns markers l and l+32.  A marker may
+                    // change when it has an old effect or num^2 has left the range
+                    // where component 0 is certain; only such a marker's component is
+                    // worked out, when the chain reaches it, by the whole warp; when it
+                    // changes the residual the later markers move by dBeta_p * G[p, t].
+                    // (Deciding every marker again after every change took 150
+                    // instructions a marker pair on this one warp.)
+                    int comp[2] = {0, 0};
                     bool fb[2] = {false, false};
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        hg[h] = s_H[grp[h]];
+                    float sx[2] = {num_sq(nh[0], nl[0]), num_sq(nh[1], nl[1])};
                     int next = 0, nupd = 0;
-                    while (true) {
+                    while (next < kMaxSpec) {
                         const long long tl0 = prof_r ? clk() : 0;
-                        bool need[2], upd[2];
-                        float sx[2];
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float xh = nh[h], xl = nl[h];
-                            df_add(xh, xl, ch[h], cl[h]);
-                            sx[h] = __fmaf_rn(xh, xh, 2.f * xh * xl);
-                            const float delta = fabsf(sx[h] - sref[h]) * 1.000001f + 4e-7f * (sx[h] + sref[h]);
-                            need[h] = own[h] && lane + 32 * h >= next && !(hg[h] * delta <= wmar[h]);
-                        }
-                        const unsigned need_halves = (__ballot_sync(0xffffffffu, need[0]) ? 1u : 0u) |
-                                                     (__ballot_sync(0xffffffffu, need[1]) ? 2u : 0u);
-                        if (need_halves) {
-                            bool slow[2];
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                slow[h] = false;
-                                // a half none of whose markers needs a new decision is skipped
-                                if (!(need_halves & (1u << h)))
-                                    continue;
-                                int c;
-                                float w;
-                                const bool okm =
-                                    pick_margin<KM>(sx[h], ufr[h], gcf + (size_t)grp[h] * kMaxK * 2, kk[h], c, w);
-                                if (need[h]) {
-                                    comp[h] = c;
-                                    fb[h] = false;
-                                    sref[h] = sx[h];
-                                    wmar[h] = okm ? w : -1.f;
-                                }
-                                slow[h] = need[h] && !okm;
-                            }
-                            if (__any_sync(0xffffffffu, slow[0] || slow[1])) {
-#pragma unroll
-                                for (int h = 0; h < 2; ++h) {
-                                    if (!slow[h])
-                                        continue;
-                                    // 700 guards possibly active, or u near a boundary:
-                                    // the guarded FP32 sampler, then FP64
-                                    float xh = nh[h], xl = nl[h];
-                                    df_add(xh, xl, ch[h], cl[h]);
-                                    int c;
-                                    float a0;
-                                    if (pick_f32<KM>(xh, xl, ufr[h], gcf + (size_t)grp[h] * kMaxK * 2, kk[h], c,
-                                                     a0)) {
-                                        comp[h] = c;
-                                    } else {
-                                        const BlockRec &rc = ring_rec[(q0 + lane + 32 * h) & Rm];
-                                        const Pick r64 = pick_marker<false, KM>(
-                                            (double)xh + (double)xl, rc.u, rc.z, rc.beta_old,
-                                            a.gconst + (size_t)grp[h] * kMaxK * 4, kk[h]);
-                                        comp[h] = r64.comp;
-                                        df_from_double(r64.acum0, fah[h], fal[h]);
-                                        df_from_double(r64.beta, fbh[h], fbl[h]);
-                                        fb[h] = true;
-                                        if (sidx == 0 && fb_counter)
-                                            atomicAdd(fb_counter, 1ull);
-                                    }
+                        const unsigned b0 = __ballot_sync(0xffffffffu, lane >= next && sx[0] > s0[0]);
+                        const unsigned b1 = __ballot_sync(0xffffffffu, lane + 32 >= next && sx[1] > s0[1]);
+                        if (!(b0 | b1))
+                            break;
+                        const int p = b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);
+                        const int owner = p & 31;
+                        const bool half = p >= 32;
+                        const BlockRec &rc = ring_rec[(q0 + p) & Rm];
+                        const float *gf = gcf + (size_t)rc.group * kMaxK * 2;
+                        float2 g2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                        if (own[0] && lane > p)
+                            g2[0] = gtri[lane * (lane - 1) / 2 + p];
+                        if (own[1] && lane + 32 > p)
+                            g2[1] = gtri[(lane + 32) * (lane + 31) / 2 + p];
+                        const float xh = half ? nh[1] : nh[0], xl = half ? nl[1] : nl[0];
+                        int c = pick_lanes<KM>(lane, __shfl_sync(0xffffffffu, half ? sx[1] : sx[0], owner), rc.uf, gf,
+                                               s_gk[rc.group]);
+                        bool f64 = false;
+                        float bh = 0.f, bl = 0.f;
+                        if (c == -2) {
+                            // 700 guards possibly active, or u near a boundary: the guarded
+                            // FP32 sampler, then FP64
+                            if (lane == owner) {
+                                float a0;
+                                if (!pick_f32<KM>(xh, xl, rc.uf, gf, s_gk[rc.group], c, a0)) {
+                                    const Pick r64 = pick_marker<false, KM>(
+                                        (double)xh + (double)xl, a.u[rc.j], a.z[rc.j], a.beta[rc.j],
+                                        a.gconst + (size_t)rc.group * kMaxK * 4, s_gk[rc.group]);
+                                    c = r64.comp;
+                                    f64 = true;
+                                    df_from_double(r64.beta, bh, bl);
+                                    if (half)
+                                        fb[1] = true;
+                                    else
+                                        fb[0] = true;
+                                    if (sidx == 0 && fb_counter)
+                                        atomicAdd(fb_counter, 1ull);
                                 }
                             }
+                            c = __shfl_sync(0xffffffffu, c, owner);
                         }
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            upd[h] = own[h] && lane + 32 * h >= next && (bnz[h] || comp[h] > 0);
+                        if (lane == owner) {
+                            if (half)
+                                comp[1] = c;
+                            else
+                                comp[0] = c;
+                        }
+                        next = p + 1;
+                        ++steps;
                         const long long tl1 = prof_r ? clk() : 0;
                         if (prof_r)
                             ph[9] += tl1 - tl0;
-                        ++steps;
-                        const unsigned b0 = __ballot_sync(0xffffffffu, upd[0]);
-                        const unsigned b1 = __ballot_sync(0xffffffffu, upd[1]);
-                        const int p = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : kMaxSpec);
-                        if (p >= nb)
-                            break;
+                        if (c <= 0 && !rc.bnz)
+                            continue;
                         // dBeta_p = beta_old - beta_new as double-float, by the owner
-                        const int owner = p & 31;
-                        const bool half = p >= 32;
                         float dh = 0.f, dl = 0.f;
-                        if (lane == owner) {
-                            const BlockRec &rc = ring_rec[(q0 + p) & Rm];
-                            const int c = half ? comp[1] : comp[0];
-                            if (c >= 0) {
-                                float bh = 0.f, bl = 0.f;
-                                if (c > 0) {
-                                    if (half ? fb[1] : fb[0]) {
-                                        bh = half ? fbh[1] : fbh[0];
-                                        bl = half ? fbl[1] : fbl[0];
-                                    } else {
-                                        float xh = half ? nh[1] : nh[0], xl = half ? nl[1] : nl[0];
-                                        df_add(xh, xl, half ? ch[1] : ch[0], half ? cl[1] : cl[0]);
-                                        const float4 gc =
-                                            reinterpret_cast<const float4 *>(gbf + (size_t)rc.group * kMaxK * 4)[c];
-                                        float ph2, pl2;
-                                        df_mul(rc.zf[0], rc.zf[1], gc.x, gc.y, bh, bl);
-                                        df_mul(xh, xl, gc.z, gc.w, ph2, pl2);
-                                        df_add(bh, bl, ph2, pl2);
-                                    }
-                                }
-                                dh = rc.bo[0];
-                                dl = rc.bo[1];
-                                df_add(dh, dl, -bh, -bl);
+                        if (c >= 0) {
+                            if (c > 0 && !f64) {
+                                const float4 gc = reinterpret_cast<const float4 *>(gbf + (size_t)rc.group * kMaxK * 4)[c];
+                                float ph2, pl2;
+                                df_mul(rc.zf[0], rc.zf[1], gc.x, gc.y, bh, bl);
+                                df_mul(xh, xl, gc.z, gc.w, ph2, pl2);
+                                df_add(bh, bl, ph2, pl2);
                             }
+                            dh = rc.bo[0];
+                            dl = rc.bo[1];
+                            df_add(dh, dl, -bh, -bl);
                         }
                         dh = __shfl_sync(0xffffffffu, dh, owner);
                         dl = __shfl_sync(0xffffffffu, dl, owner);
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
-                            const int m = lane + 32 * h;
-                            if (own[h] && m > p) {
-                                const float2 g2 = gtri[m * (m - 1) / 2 + p];
-                                float ph2, pl2;
-                                df_mul(dh, dl, g2.x, g2.y, ph2, pl2);
-                                df_add(ch[h], cl[h], ph2, pl2);
-                            }
+                            float ph2, pl2;
+                            df_mul(dh, dl, g2[h].x, g2[h].y, ph2, pl2);
+                            df_add(nh[h], nl[h], ph2, pl2);
+                            sx[h] = num_sq(nh[h], nl[h]);
                         }
                         if (lane == 0) {
                             s_upd[par][nupd] = p;
                             s_dB[par][nupd] = make_float2(dh, dl);
                         }
                         if (lane == owner) {
-                            const float4 *xs = reinterpret_cast<const float4 *>(ring_rec[(q0 + p) & Rm].x);
+                            const float4 *xs = reinterpret_cast<const float4 *>(rc.x);
                             s_x[par][nupd][0] = xs[0];
                             s_x[par][nupd][1] = xs[1];
                         }
                         ++nupd;
-                        next = p + 1;
                         if (prof_r)
                             ph[10] += clk() - tl1;
                     }
                     if (lane == 0)
                         s_nupd[par] = nupd;
-                    // the decisions of the markers whose outputs this CTA writes
-                    // (sweep position p by CTA p mod G)
-                    {
-                        BlockOut &o = s_out[r & 1];
+                    // the block's outputs by sweep position, by one CTA in turn
+                    if (turn == sidx) {
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int m = lane + 32 * h;
-                            if ((q0 + (unsigned)m) % (unsigned)a.G != (unsigned)sidx) {
-                                o.code[m] = -2;
-                                continue;
-                            }
-                            float xh = nh[h], xl = nl[h];
-                            df_add(xh, xl, ch[h], cl[h]);
-                            o.x[m] = make_float2(xh, xl);
-                            o.fb[m] = make_float2(fbh[h], fbl[h]);
-                            o.fa[m] = make_float2(fah[h], fal[h]);
-                            o.uf[m] = ufr[h];
-                            o.group[m] = grp[h];
-                            o.code[m] = own[h] ? ((comp[h] & 0xFF) | (fb[h] ? 0x100 : 0)) : -2;
+                        for (int h = 0; h < 2; ++h)
                             if (own[h]) {
-                                const BlockRec &rc = ring_rec[(q0 + m) & Rm];
-                                o.zf[m] = make_float2(rc.zf[0], rc.zf[1]);
-                                o.j[m] = rc.j;
+                                a.num_df[q0 + lane + 32 * h] = make_float2(nh[h], nl[h]);
+                                a.code_pos[q0 + lane + 32 * h] = (comp[h] & 0xFF) | (fb[h] ? 0x100 : 0);
                             }
-                        }
                     }
+                    turn = turn + 1 == a.G ? 0 : turn + 1;
                     mark(prof_r, 3);
                 }
             }
@@ -1454,11 +1266,9 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
                     gather_load(r + 4);
                 if (lane == 0)
                     stamp(r, 11);
-                if (r >= 1)
-                    write_block_outputs<KM>(a, s_out[(r - 1) & 1], gcf, s_gk, gbf, lane);
                 if (lane == 0)
                     stamp(r, 5);
-                mbar_arrive(&s_mb[(r + 1) & 1]);   // GO(r+1): block r-1's outputs read
+                mbar_arrive(&s_mb[(r + 1) & 1]);   // GO(r+1)
             } else if (warp == kInputWarp) {
                 // ---- input warp: block r+1's inputs
                 if (r + 1 < nblk)
@@ -1500,8 +1310,6 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
     if (!s_abort && r == nblk) {
         if (dw >= 0)
             apply_update(nblk - 1);
-        else if (warp == kChoreWarp)
-            write_block_outputs<KM>(a, s_out[(nblk - 1) & 1], gcf, s_gk, gbf, lane);
     }
     if (prof_d) {
         a.prof[0] = ph[0];
@@ -1538,21 +1346,16 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
 
     // ---- epilogue: residual back to HBM, per-slice sums
     double s1 = 0.0, s2 = 0.0;
-    for (int b = tid; b < nbytes; b += kBlockThreads) {
-        const longlong2 e01 = reinterpret_cast<const longlong2 *>(fix)[2 * b];
-        const longlong2 e23 = reinterpret_cast<const longlong2 *>(fix)[2 * b + 1];
-        const long long E[4] = {e01.x, e01.y, e23.x, e23.y};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (4 * b + i < ns) {
-                float h, l;
-                fix_to_df(E[i], h, l);
-                a.eps_hi[lo + 4 * b + i] = h;
-                a.eps_lo[lo + 4 * b + i] = l;
-                const double e = (double)h + (double)l;
-                s1 += e;
-                s2 = fma(e, e, s2);
-            }
+    for (int i = tid; i < a.slice_max; i += kBlockThreads) {
+        const int ii = limb_individual(i);
+        if (ii < ns) {
+            float h, l;
+            fix_to_df(fix[i], h, l);
+            a.eps_hi[lo + ii] = h;
+            a.eps_lo[lo + ii] = l;
+            const double e = (double)h + (double)l;
+            s1 += e;
+            s2 = fma(e, e, s2);
         }
     }
     __shared__ double s_red[kBlockThreads / 32][2];
@@ -1586,17 +1389,27 @@ __global__ void __launch_bounds__(12 * 32, 1) k_sweep_block(SweepArgs a)
 
 cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, const double *table,
                                 const double *scale, const double *beta, const double *u, const double *z,
-                                const int32_t *group, double eps_total, BlockRec *rec, cudaStream_t st)
+                                const int32_t *group, double eps_total, int kmax, const double *gconst,
+                                const int32_t *gK, BlockRec *rec, cudaStream_t st)
 {
-    k_gather_block<<<(unsigned)((M + 255) / 256), 256, 0, st>>>(order, M, N, table, scale, beta, u, z, group,
-                                                                eps_total, rec);
+    const unsigned nb = (unsigned)((M + 255) / 256);
+    if (kmax <= 4)
+        k_gather_block<4><<<nb, 256, 0, st>>>(order, M, N, table, scale, beta, u, z, group, eps_total, gconst, gK, rec);
+    else
+        k_gather_block<kMaxK><<<nb, 256, 0, st>>>(order, M, N, table, scale, beta, u, z, group, eps_total, gconst, gK,
+                                                  rec);
     return cudaGetLastError();
 }
 
-cudaError_t launch_block_finish(int64_t M, const uint8_t *chosen, const float2 *beta_df, const float2 *acum_df,
-                                double *beta, double *acum, cudaStream_t st)
+cudaError_t launch_block_finish(int64_t M, int kmax, const BlockRec *rec, const float2 *num, const int *code,
+                                const double *u, const double *z, const double *gconst, const int32_t *gK, double *beta,
+                                double *acum, int32_t *comp, uint8_t *chosen, cudaStream_t st)
 {
-    k_block_finish<<<(unsigned)((M + 255) / 256), 256, 0, st>>>(M, chosen, beta_df, acum_df, beta, acum);
+    const unsigned nb = (unsigned)((M + 127) / 128);
+    if (kmax <= 4)
+        k_block_finish<4><<<nb, 128, 0, st>>>(M, rec, num, code, u, z, gconst, gK, beta, acum, comp, chosen);
+    else
+        k_block_finish<kMaxK><<<nb, 128, 0, st>>>(M, rec, num, code, u, z, gconst, gK, beta, acum, comp, chosen);
     return cudaGetLastError();
 }
 

@@ -58,7 +58,7 @@ struct brr_ctx {
     double *d_eps_dl = nullptr;         // FP32C: the residual as doubles for its read-back (allocated on use)
     double *d_gstage = nullptr;         // blocked FP32C: staged Gram entries (8 blocks)
     brr::BlockRec *d_brec = nullptr;         // blocked FP32C: records in sweep order
-    float2 *d_bdf = nullptr;            // blocked FP32C: [2][M] new beta, acum (double-float)
+    float2 *d_bdf = nullptr;            // blocked FP32C, by sweep position: M nums (double-float), M decision codes
     bool blocked = false;
     // whole-round sweep (brr_round.cu): taken by every chain it fits but the Gram-blocked ones
     bool round_ok = false;

@@ -234,4 +234,50 @@ __device__ __forceinline__ void fx_to_df(long long hi, unsigned long long lo, fl
     }
 }
 
+// (H 2^30 + L) 2^e as a double, rounded once, with integer operations (FP64
+// conversions issue at the FP64 rate).
+__device__ __forceinline__ double fixed_to_double(long long H, long long L, int e)
+{
+    const __int128 X = ((__int128)H << 30) + L;
+    const bool neg = X < 0;
+    const unsigned __int128 A = neg ? (unsigned __int128)(-X) : (unsigned __int128)X;
+    const unsigned long long hi = (unsigned long long)(A >> 64), lo = (unsigned long long)A;
+    if ((hi | lo) == 0ull)
+        return 0.0;
+    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+    const unsigned __int128 N = A << lz;
+    const unsigned long long th = (unsigned long long)(N >> 64);
+    // 53 bits, to the nearest (the sticky bits below the 64 kept are ignored: a tie moves by less than 2^-63)
+    const unsigned long long m = (th >> 11) + ((th >> 10) & 1ull);
+    const int ex = 127 - lz + e + 1023;   // exponent of the leading bit
+    if (ex < 1 || ex > 2045)
+        return ldexp(neg ? -(double)m : (double)m, 127 - lz + e - 52);
+    const unsigned long long bits = ((unsigned long long)ex << 52) + (m - (1ull << 52));
+    return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
+}
+
+// (H 2^30 + L) 2^e as a float pair (48 bits, truncated), with integer operations.
+__device__ __forceinline__ void fixed_to_df(long long H, long long L, int e, float &h, float &l)
+{
+    const __int128 X = ((__int128)H << 30) + L;
+    unsigned long long hi = (unsigned long long)(X >> 64), lo = (unsigned long long)X;
+    const unsigned sign = (unsigned)(hi >> 32) & 0x80000000u;
+    if (sign) {
+        lo = 0ull - lo;
+        hi = ~hi + (lo == 0ull ? 1ull : 0ull);
+    }
+    h = l = 0.f;
+    if ((hi | lo) == 0ull)
+        return;
+    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+    unsigned long long th = lz >= 64 ? lo << (lz - 64) : lz == 0 ? hi : (hi << lz) | (lo >> (64 - lz));
+    const int ex = 127 - lz + e + 127;   // FP32 exponent field of the leading bit
+    if (ex < 60 || ex > 250) {
+        df_from_double(fixed_to_double(H, L, e), h, l);
+        return;
+    }
+    h = __uint_as_float(sign | ((unsigned)ex << 23) | ((unsigned)(th >> 40) & 0x7FFFFFu));
+    l = __uint2float_rn((unsigned)(th >> 16) & 0xFFFFFFu) * __uint_as_float(sign | ((unsigned)(ex - 47) << 23));
+}
+
 }  // namespace brr

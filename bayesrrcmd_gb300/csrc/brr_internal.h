@@ -41,14 +41,12 @@ struct alignas(16) BlockRec {
     float zf[2];         // z
     float uf;            // u rounded to FP32 (certified sampler)
     uint32_t bnz;        // beta_old != 0
-    double beta_old;     // FP64 draws for the sampler's FP64 fallback
-    double u;
-    double z;
     uint32_t j;
     int32_t group;
-    uint32_t pad[4];
+    float s0;            // num^2 up to which component 0 is certain (negative: never)
+    uint32_t pad;
 };
-static_assert(sizeof(BlockRec) == 128, "BlockRec must be 128 bytes");
+static_assert(sizeof(BlockRec) == 96, "BlockRec must be 96 bytes");
 
 // Record of the whole-round sweep (brr_round.cu, k_round_gather), in sweep order:
 // num = c + s S + am Sm + at T with S the sum of genotype x residual, Sm the residual
@@ -112,8 +110,8 @@ struct SweepArgs {
     int has_missing;             // any missing genotype in the packed markers
     const BlockRec *brec;        // blocked FP32C sweep: M records in sweep order
     const uint32_t *order;       // blocked FP32C sweep: the M marker ids in sweep order
-    float2 *beta_df;             // blocked FP32C sweep: new beta per marker (hi, lo)
-    float2 *acum_df;             // blocked FP32C sweep: acum per marker (hi, lo)
+    float2 *num_df;              // blocked FP32C sweep: final num (hi, lo) by sweep position
+    int *code_pos;               // blocked FP32C sweep: component & 0xFF | FP64 decision << 8, by position
     int eigen;                   // ragged sweep: Eigen sparse markers (missing genotypes enter
                                  // the dot product at the marker's mean)
     unsigned long long *t_out;   // optional [2]: global timer (ns) at the start and end of the sweep (CTA 0)
@@ -131,7 +129,7 @@ struct SweepArgs {
     const double *emax;          // [n_emax] partial maxima of |eps| before mu_new is subtracted
     const RoundRec *rrec;        // M records in sweep order
     const double *rgram;         // [blocks of B][B (B-1) / 2] pair products in sweep order (pairs only)
-    const double *u;             // M: the markers' uniforms, by marker id
+    const double *u, *z;         // M: the markers' draws, by marker id (also the blocked sweep's)
     const uint32_t *rnz;         // one bit per sweep position: the marker is sure or likely to change
     int rall;                    // the products of every row are formed, not only those of rnz
     double *num_out;             // M: the num each marker was decided on
@@ -308,9 +306,11 @@ cudaError_t launch_round_finish(int64_t M, int form, int kmax, const double *num
 size_t sweep_block_smem_bytes(const SweepArgs &a);
 cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, const double *table,
                                 const double *scale, const double *beta, const double *u, const double *z,
-                                const int32_t *group, double eps_total, BlockRec *rec, cudaStream_t st);
-cudaError_t launch_block_finish(int64_t M, const uint8_t *chosen, const float2 *beta_df, const float2 *acum_df,
-                                double *beta, double *acum, cudaStream_t st);
+                                const int32_t *group, double eps_total, int kmax, const double *gconst,
+                                const int32_t *gK, BlockRec *rec, cudaStream_t st);
+cudaError_t launch_block_finish(int64_t M, int kmax, const BlockRec *rec, const float2 *num, const int *code,
+                                const double *u, const double *z, const double *gconst, const int32_t *gK, double *beta,
+                                double *acum, int32_t *comp, uint8_t *chosen, cudaStream_t st);
 cudaError_t launch_sweep_block(const SweepArgs &a, size_t smem, cudaStream_t st);
 size_t sweep_block_stage_bytes(int B);   // global Gram staging of the blocked sweep
 int sweep_block_threads();

@@ -259,4 +259,96 @@ __device__ __forceinline__ bool pick_margin(float s, float uf, const float *__re
     return far && !close && chosen < K && w > 0.f;
 }
 
+// The largest num^2 up to which component 0 is certain for a marker with
+// uniform u: P(component 0) = 1 / f(s), f(s) = 1 + sum exp(dc_k + h_k s), falls as s =
+// num^2 grows (h_k > 0), so the marker stays in component 0 exactly while f(s) <=
+// 1/u.  Newton's iteration on the convex log f, started right of the root where
+// one term alone reaches 1/u, then the certificate of pick_margin at a point a little
+// to the left.  Negative when no point can be certified (the 700 guards of the
+// reference could matter, or u is above P(component 0) at s = 0).
+template <int KM>
+__device__ __forceinline__ float certain_zero(float uf, const double *gc, int K)
+{
+    float dc[KM], hh[KM];
+    float lo = 0.f;
+    bool usable = uf > 1e-30f && uf < 1.f;
+    const float L = -__logf(uf);
+    float s = INFINITY;
+#pragma unroll
+    for (int k = 1; k < KM; ++k) {
+        dc[k] = k < K ? __double2float_rn(gc[4 * k] - gc[0]) : -INFINITY;
+        hh[k] = k < K ? __double2float_rn(gc[4 * k + 2]) : 0.f;
+        if (k < K) {
+            lo = fminf(lo, dc[k]);
+            usable = usable && hh[k] > 0.f;
+            s = fminf(s, __fdividef(L - dc[k], hh[k]));
+        }
+    }
+    if (!usable || !(lo > -600.f) || !(s > 0.f))
+        return -1.f;
+    auto eval = [&](float x, float &f, float &df, float &err) {
+        f = 1.f;
+        df = 0.f;
+        err = 0.f;
+        float top = 0.f;
+#pragma unroll
+        for (int k = 1; k < KM; ++k)
+            if (k < K) {
+                const float D = __fmaf_rn(hh[k], x, dc[k]);
+                top = fmaxf(top, D);
+                const float e = __expf(fminf(D, 80.f));
+                f += e;
+                df = __fmaf_rn(hh[k], e, df);
+                err = fmaxf(err, 3.0e-7f * (fabsf(dc[k]) + fabsf(hh[k] * x)));
+            }
+        return top;
+    };
+    float f, df, err;
+    for (int it = 0; it < 10; ++it) {
+        eval(s, f, df, err);
+        s = fmaxf(s - (__logf(f) - L) * __fdividef(f, df), 0.f);
+    }
+    float back = 2e-4f;
+#pragma unroll
+    for (int tries = 0; tries < 3; ++tries, back *= 20.f) {
+        const float x = s * (1.f - back);
+        const float top = eval(x, f, df, err);
+        if (top < 80.f && uf * f < 1.f - (4e-5f + 4.f * err) * f)
+            return x * (1.f - 2e-6f);   // num^2 is evaluated to 4e-7
+    }
+    return -1.f;
+}
+
+// Component of one marker at num^2 = x by a whole warp, one mixture component per
+// lane: the certified decision of pick_margin without its margin; -2 where it cannot
+// certify.  gcf: the group's FP32 constants {dc_k, h_k}.  About 40 instructions against
+// 150, which matters where the decision lies on a sweep's chain.
+template <int KM>
+__device__ __forceinline__ int pick_lanes(int lane, float x, float uf, const float *gcf, int K)
+{
+    const float2 f = reinterpret_cast<const float2 *>(gcf)[lane & (kMaxK - 1)];
+    const bool in = lane < K;
+    const float hx = f.y * x;
+    const float D = in ? f.x + hx : 0.f;   // lane 0: 0
+    // non-negative floats order as integers; |dc| + |h x| bounds |D|, and 4e-7 of it the
+    // error of D (six roundings)
+    const float dmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(D, 0.f))));
+    const float mag =
+        __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(in ? fabsf(f.x) + fabsf(hx) : 0.f)));
+    float c = in ? __expf(D - dmax) : 0.f;
+#pragma unroll
+    for (int o = 1; o < KM; o <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, c, o);
+        c += lane >= o ? v : 0.f;
+    }
+    const float es = __shfl_sync(0xffffffffu, c, K - 1), target = uf * es;
+    const float tol = (4e-5f + 1.6e-6f * mag) * es;
+    const int comp = __popc(__ballot_sync(0xffffffffu, in && c < target));
+    const bool close = __any_sync(0xffffffffu, in && fabsf(c - target) < tol);
+    return (close || comp >= K || !(mag < 300.f)) ? -2 : comp;
+}
+
+// num^2 of num = nh + nl, to 4e-7.
+__device__ __forceinline__ float num_sq(float nh, float nl) { return __fmaf_rn(nh, nh, 2.f * nh * nl); }
+
 }  // namespace brr

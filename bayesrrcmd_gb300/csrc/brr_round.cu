@@ -42,11 +42,10 @@
 // their stability margins (FP64 where they cannot certify); num, beta and the
 // corrections are FP64.  P(component 0) is left to k_round_finish, one thread
 // per marker over the whole GPU, from the stored num.
-#include <cuda_fp16.h>
-
 #include "brr_cluster.cuh"
 #include "brr_device.cuh"
 #include "brr_internal.h"
+#include "brr_mma.cuh"
 #include "brr_pick.cuh"
 
 namespace brr {
@@ -55,7 +54,6 @@ namespace {
 
 constexpr int kRT = 512;                 // threads per CTA
 constexpr int kRW = kRT / 32;
-constexpr int kLimbs = 7;                // 10-bit limbs of the residual
 // Accumulators in L2: two alternating buffers of up to kAccCopies copies, each
 // four rows (low and high word of the markers' sums and of their sums over the
 // missing genotypes) of 65 words (64 markers and the slice totals) in 72.  A row is
@@ -98,14 +96,14 @@ __host__ __device__ inline RoundPlan round_plan(int slice_max, int B, int n_grou
 {
     RoundPlan p;
     const int chunks = slice_max / kChunk;
-    p.plane_stride = 2 * slice_max + 16;
+    p.plane_stride = limb_plane_stride(slice_max);
     p.code_stride = 16 * (chunks | 1);
     const int B16 = B < 16 ? 16 : B;
     size_t o = 0;
     p.E = o;
     o += (size_t)8 * slice_max;
     p.planes = o;
-    o += al16((size_t)8 * p.plane_stride);   // limbs 0-2, a zero plane, limbs 3-6: the tensor tile's 8 columns
+    o += al16((size_t)kLimbPlanes * p.plane_stride);
     p.codes = o;
     o += (size_t)2 * B16 * p.code_stride;
     p.rec = o;
@@ -132,49 +130,6 @@ __host__ __device__ inline RoundPlan round_plan(int slice_max, int B, int n_grou
         o += (size_t)2 * kAccCopyWords * kAccCopies * sizeof(unsigned long long);
     p.total = al16(o);
     return p;
-}
-
-// 16 genotypes of a code word as FP16 pairs: pair k holds individuals
-// (k & 3) + 8 (k >> 2) and that + 4, the order the limb planes are stored in.
-// `table` holds the high byte of the FP16 value of each 2-bit code.
-constexpr unsigned kGenoTable = 0x003C0040u;   // codes 0: 2.0, 1 (missing): 0, 2: 1.0, 3: 0
-constexpr unsigned kMissTable = 0x00003C00u;   // code 1: 1.0
-template <int K>
-__device__ __forceinline__ unsigned geno_pair(unsigned w, unsigned table)
-{
-    const unsigned s = K == 0 ? w << 4 : K == 1 ? w << 2 : K == 2 ? w : w >> (K == 3 ? 2 : 4 + 2 * K);
-    return __byte_perm(table, 0u, (s & 0x3030u) | 0x0404u);
-}
-
-__device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
-                                        unsigned b1)
-{
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                 "{%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// (H 2^30 + L) 2^e as a double, rounded once, with integer operations (FP64
-// conversions issue at the FP64 rate).
-__device__ __forceinline__ double fixed_to_double(long long H, long long L, int e)
-{
-    const __int128 X = ((__int128)H << 30) + L;
-    const bool neg = X < 0;
-    const unsigned __int128 A = neg ? (unsigned __int128)(-X) : (unsigned __int128)X;
-    const unsigned long long hi = (unsigned long long)(A >> 64), lo = (unsigned long long)A;
-    if ((hi | lo) == 0ull)
-        return 0.0;
-    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
-    const unsigned __int128 N = A << lz;
-    const unsigned long long th = (unsigned long long)(N >> 64);
-    // 53 bits, to the nearest (the sticky bits below the 64 kept are ignored: a tie moves by less than 2^-63)
-    const unsigned long long m = (th >> 11) + ((th >> 10) & 1ull);
-    const int ex = 127 - lz + e + 1023;   // exponent of the leading bit
-    if (ex < 1 || ex > 2045)
-        return ldexp(neg ? -(double)m : (double)m, 127 - lz + e - 52);
-    const unsigned long long bits = ((unsigned long long)ex << 52) + (m - (1ull << 52));
-    return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
 }
 
 __device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
@@ -205,32 +160,6 @@ __device__ __noinline__ int decide_slow(float nh, float nl, double u, const doub
     if (!pick_f32<KM>(nh, nl, __double2float_rn(u), gcf, K, comp, a0))
         comp = pick_marker<true, KM>((double)nh + (double)nl, u, 0.0, 0.0, gc, K).comp;
     return comp;
-}
-
-__device__ __forceinline__ float num_sq(float nh, float nl) { return __fmaf_rn(nh, nh, 2.f * nh * nl); }
-
-// (H 2^30 + L) 2^e as a float pair (48 bits, truncated), with integer operations.
-__device__ __forceinline__ void fixed_to_df(long long H, long long L, int e, float &h, float &l)
-{
-    const __int128 X = ((__int128)H << 30) + L;
-    unsigned long long hi = (unsigned long long)(X >> 64), lo = (unsigned long long)X;
-    const unsigned sign = (unsigned)(hi >> 32) & 0x80000000u;
-    if (sign) {
-        lo = 0ull - lo;
-        hi = ~hi + (lo == 0ull ? 1ull : 0ull);
-    }
-    h = l = 0.f;
-    if ((hi | lo) == 0ull)
-        return;
-    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
-    unsigned long long th = lz >= 64 ? lo << (lz - 64) : lz == 0 ? hi : (hi << lz) | (lo >> (64 - lz));
-    const int ex = 127 - lz + e + 127;   // FP32 exponent field of the leading bit
-    if (ex < 60 || ex > 250) {
-        df_from_double(fixed_to_double(H, L, e), h, l);
-        return;
-    }
-    h = __uint_as_float(sign | ((unsigned)ex << 23) | ((unsigned)(th >> 40) & 0x7FFFFFu));
-    l = __uint2float_rn((unsigned)(th >> 16) & 0xFFFFFFu) * __uint_as_float(sign | ((unsigned)(ex - 47) << 23));
 }
 
 // --------------------------------------------------------------------------
@@ -424,10 +353,8 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     const int sc = min(59 - e2 - a.headroom, 100);
     const double up = pow2d(sc), down = pow2d(-sc);
     bool range = false;
-    // position i of the slice: pair (i & 15) >> 1 of its 16-individual group
-    auto individual = [](int i) { return (i & ~15) + (((i >> 1) & 3) | (((i >> 3) & 1) << 3) | ((i & 1) << 2)); };
     for (int i = tid; i < a.slice_max; i += kRT) {
-        const int ind = individual(i);
+        const int ind = limb_individual(i);
         long long v = 0;
         if (ind < ns) {
             if (a.form == BRR_FORM_FP64) {
@@ -442,38 +369,13 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
         E[i] = v;
     }
     __syncthreads();
-    // limbs of a pair of neighbouring positions into the planes
-    auto put_limbs = [&](int pr, long long e0, long long e1) {
-        constexpr unsigned long long bias =
-            512ull * (1ull + (1ull << 10) + (1ull << 20) + (1ull << 30) + (1ull << 40) + (1ull << 50));
-        const unsigned long long b0 = (unsigned long long)e0 + bias, b1 = (unsigned long long)e1 + bias;
-        unsigned char *dst = planes + 4 * pr;
-#pragma unroll
-        for (int k = 0; k < kLimbs; ++k) {
-            const int col = k < 3 ? k : k + 1;   // column 3 of the tensor tile is zero
-            unsigned v0, v1;
-            half2 off;
-            if (k < kLimbs - 1) {
-                v0 = (unsigned)(b0 >> (10 * k)) & 1023u;
-                v1 = (unsigned)(b1 >> (10 * k)) & 1023u;
-                off = __half2half2(__ushort_as_half(0x6600));   // 1024 + 512
-            } else {
-                v0 = (unsigned)((long long)b0 >> 60) + 8u;
-                v1 = (unsigned)((long long)b1 >> 60) + 8u;
-                off = __half2half2(__ushort_as_half(0x6408));   // 1024 + 8
-            }
-            const unsigned w = 0x64006400u | v0 | (v1 << 16);
-            half2 h = __hsub2(*reinterpret_cast<const half2 *>(&w), off);
-            *reinterpret_cast<half2 *>(dst + (size_t)col * plan.plane_stride) = h;
-        }
-    };
     {
         long long tl = 0, th = 0;
         for (int i = tid; i < plan.plane_stride / 4; i += kRT)
             reinterpret_cast<unsigned *>(planes + (size_t)3 * plan.plane_stride)[i] = 0u;
         for (int pr = tid; pr < a.slice_max / 2; pr += kRT) {
             const longlong2 e = reinterpret_cast<const longlong2 *>(E)[pr];
-            put_limbs(pr, e.x, e.y);
+            put_limbs(planes, plan.plane_stride, pr, e.x, e.y);
             tl += (e.x & kLow30) + (e.y & kLow30);
             th += (e.x >> 30) + (e.y >> 30);
         }
@@ -552,24 +454,9 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 const unsigned w1 = *reinterpret_cast<const unsigned *>(rbp + 16 * ch);
                 const uint4 x = *reinterpret_cast<const uint4 *>(pb + 128 * ch);
                 const uint4 y = *reinterpret_cast<const uint4 *>(pb + 128 * ch + 16);
-                mma_f16(c, geno_pair<0>(w0, kGenoTable), geno_pair<0>(w1, kGenoTable), geno_pair<1>(w0, kGenoTable),
-                        geno_pair<1>(w1, kGenoTable), x.x, x.y);
-                mma_f16(c, geno_pair<2>(w0, kGenoTable), geno_pair<2>(w1, kGenoTable), geno_pair<3>(w0, kGenoTable),
-                        geno_pair<3>(w1, kGenoTable), x.z, x.w);
-                mma_f16(c, geno_pair<4>(w0, kGenoTable), geno_pair<4>(w1, kGenoTable), geno_pair<5>(w0, kGenoTable),
-                        geno_pair<5>(w1, kGenoTable), y.x, y.y);
-                mma_f16(c, geno_pair<6>(w0, kGenoTable), geno_pair<6>(w1, kGenoTable), geno_pair<7>(w0, kGenoTable),
-                        geno_pair<7>(w1, kGenoTable), y.z, y.w);
-                if (msum) {
-                    mma_f16(cm, geno_pair<0>(w0, kMissTable), geno_pair<0>(w1, kMissTable),
-                            geno_pair<1>(w0, kMissTable), geno_pair<1>(w1, kMissTable), x.x, x.y);
-                    mma_f16(cm, geno_pair<2>(w0, kMissTable), geno_pair<2>(w1, kMissTable),
-                            geno_pair<3>(w0, kMissTable), geno_pair<3>(w1, kMissTable), x.z, x.w);
-                    mma_f16(cm, geno_pair<4>(w0, kMissTable), geno_pair<4>(w1, kMissTable),
-                            geno_pair<5>(w0, kMissTable), geno_pair<5>(w1, kMissTable), y.x, y.y);
-                    mma_f16(cm, geno_pair<6>(w0, kMissTable), geno_pair<6>(w1, kMissTable),
-                            geno_pair<7>(w0, kMissTable), geno_pair<7>(w1, kMissTable), y.z, y.w);
-                }
+                mma_chunk(c, w0, w1, kGenoTable, x, y);
+                if (msum)
+                    mma_chunk(cm, w0, w1, kMissTable, x, y);
             }
             float2 *dst = reinterpret_cast<float2 *>(part + ((size_t)(kg * nmt + mt) * 16 + fg) * 8) + fq;
             dst[0] = make_float2(c[0], c[1]);
@@ -594,16 +481,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 if (total) {
                     v = m == 0 ? s_T[0] & kLow30 : s_T[1] + (s_T[0] >> 30);
                 } else {
-                    const float4 *src =
-                        reinterpret_cast<const float4 *>(part + (size_t)half * kRW * 16 * 8 + (size_t)m * 8) + word;
-                    // integers below 2^24 in any order of addition
-                    float4 f = src[0];
-                    for (int k = 1; k < nkg; ++k) {
-                        const float4 g = src[(size_t)k * nmt * 32];
-                        f.x += g.x; f.y += g.y; f.z += g.z; f.w += g.w;
-                    }
-                    v = (long long)(int)f.x + ((long long)(int)f.y << 10) + ((long long)(int)f.z << 20) +
-                        ((long long)(int)f.w << 30);
+                    v = limb_sum(part + (size_t)half * kRW * 16 * 8, m, word, nkg, nmt * 32);
                 }
                 if (CL) {
                     reinterpret_cast<long long *>(
@@ -861,31 +739,6 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 return decide_slow<KM>(h ? nh[1] : nh[0], h ? nl[1] : nl[0], a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
                                        gcf + (size_t)g * kMaxK * 2, gk[g]);
             };
-            // Component of marker p at num^2 = x, one mixture component per lane: the
-            // certified decision of pick_margin; -2 where it cannot certify.
-            auto component = [&](const RoundRec &rc, float x) {
-                const int gp = (int)(rc.gm & 255u), K = gk[gp];
-                const float2 f = reinterpret_cast<const float2 *>(gcf)[gp * kMaxK + (lane & (kMaxK - 1))];
-                const bool in = lane < K;
-                const float hx = f.y * x;
-                const float D = in ? f.x + hx : 0.f;   // lane 0: 0
-                // non-negative floats order as integers
-                const float dmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(D, 0.f))));
-                // |dc| + |h x| bounds |D| from below too
-                const float mag = __uint_as_float(
-                    __reduce_max_sync(0xffffffffu, __float_as_uint(in ? fabsf(f.x) + fabsf(hx) : 0.f)));
-                float c = in ? __expf(D - dmax) : 0.f;
-#pragma unroll
-                for (int o = 1; o < KM; o <<= 1) {
-                    const float v = __shfl_up_sync(0xffffffffu, c, o);
-                    c += lane >= o ? v : 0.f;
-                }
-                const float es = __shfl_sync(0xffffffffu, c, K - 1), target = rc.uf * es;
-                const float tol = (4e-5f + 1.6e-6f * mag) * es;
-                const int comp = __popc(__ballot_sync(0xffffffffu, in && c < target));
-                const bool close = __any_sync(0xffffffffu, in && fabsf(c - target) < tol);
-                return (close || comp >= K || !(mag < 300.f)) ? -2 : comp;
-            };
             // A marker may change when its old effect is not zero or num^2 is not in
             // the range where component 0 is certain (s0; P(component 0) falls as
             // num^2 grows).  Only such a marker's component is worked out, when the
@@ -934,7 +787,8 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 }
                 const RoundRec &rc = rec[(start + p) & Rm];
                 const float ph = hi ? nh[1] : nh[0], pl = hi ? nl[1] : nl[0];
-                int comp = component(rc, __shfl_sync(0xffffffffu, hi ? sx[1] : sx[0], p & 31));
+                int comp = pick_lanes<KM>(lane, __shfl_sync(0xffffffffu, hi ? sx[1] : sx[0], p & 31), rc.uf,
+                                          gcf + (size_t)(rc.gm & 255u) * kMaxK * 2, gk[rc.gm & 255u]);
                 if (comp == -2) {
                     if (own)
                         comp = slow(hi, p);
@@ -1106,8 +960,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             long long top = 0;
             for (int pr = tid; pr < 32 * nchunk; pr += kRT) {
                 longlong2 e = reinterpret_cast<const longlong2 *>(E)[pr];
-                const int k = pr & 7;
-                const int sh = 2 * ((k & 3) | ((k >> 2) << 3));
+                const int sh = limb_pair_shift(pr);
                 for (int u = 0; u < nchg; ++u) {
                     const unsigned w = *reinterpret_cast<const unsigned *>(
                                            codes + (size_t)((start + s_ci[u]) & Rm) * plan.code_stride + 4 * (pr >> 3)) >> sh;
@@ -1122,7 +975,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 if (ind + 4 >= ns)
                     e.y = 0;
                 reinterpret_cast<longlong2 *>(E)[pr] = e;
-                put_limbs(pr, e.x, e.y);
+                put_limbs(planes, plan.plane_stride, pr, e.x, e.y);
             }
             if (top < 0)
                 range = true;
@@ -1145,7 +998,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     // ---- epilogue: the residual to its output buffer, per-slice sums
     double s1 = 0.0, s2 = 0.0;
     for (int i = tid; i < a.slice_max; i += kRT) {
-        const int ind = individual(i);
+        const int ind = limb_individual(i);
         if (ind >= ns)
             continue;
         double e = (double)E[i] * down;
@@ -1216,66 +1069,6 @@ __global__ void __launch_bounds__(kRT, 1) k_round_multi(const __grid_constant__ 
 }
 
 // --------------------------------------------------------------------------
-// The largest num^2 up to which component 0 is certain for a marker with
-// uniform u: P(component 0) = 1 / f(s), f(s) = 1 + sum exp(dc_k + h_k s), falls as s =
-// num^2 grows (h_k > 0), so the marker stays in component 0 exactly while f(s) <=
-// 1/u.  Newton's iteration on the convex log f, started right of the root where
-// one term alone reaches 1/u, then the certificate of pick_margin at a point a little
-// to the left.  Negative when no point can be certified (the 700 guards of the
-// reference could matter, or u is above P(component 0) at s = 0).
-template <int KM>
-__device__ __forceinline__ float certain_zero(float uf, const double *gc, int K)
-{
-    float dc[KM], hh[KM];
-    float lo = 0.f;
-    bool usable = uf > 1e-30f && uf < 1.f;
-    const float L = -__logf(uf);
-    float s = INFINITY;
-#pragma unroll
-    for (int k = 1; k < KM; ++k) {
-        dc[k] = k < K ? __double2float_rn(gc[4 * k] - gc[0]) : -INFINITY;
-        hh[k] = k < K ? __double2float_rn(gc[4 * k + 2]) : 0.f;
-        if (k < K) {
-            lo = fminf(lo, dc[k]);
-            usable = usable && hh[k] > 0.f;
-            s = fminf(s, __fdividef(L - dc[k], hh[k]));
-        }
-    }
-    if (!usable || !(lo > -600.f) || !(s > 0.f))
-        return -1.f;
-    auto eval = [&](float x, float &f, float &df, float &err) {
-        f = 1.f;
-        df = 0.f;
-        err = 0.f;
-        float top = 0.f;
-#pragma unroll
-        for (int k = 1; k < KM; ++k)
-            if (k < K) {
-                const float D = __fmaf_rn(hh[k], x, dc[k]);
-                top = fmaxf(top, D);
-                const float e = __expf(fminf(D, 80.f));
-                f += e;
-                df = __fmaf_rn(hh[k], e, df);
-                err = fmaxf(err, 3.0e-7f * (fabsf(dc[k]) + fabsf(hh[k] * x)));
-            }
-        return top;
-    };
-    float f, df, err;
-    for (int it = 0; it < 10; ++it) {
-        eval(s, f, df, err);
-        s = fmaxf(s - (__logf(f) - L) * __fdividef(f, df), 0.f);
-    }
-    float back = 2e-4f;
-#pragma unroll
-    for (int tries = 0; tries < 3; ++tries, back *= 20.f) {
-        const float x = s * (1.f - back);
-        const float top = eval(x, f, df, err);
-        if (top < 80.f && uf * f < 1.f - (4e-5f + 4.f * err) * f)
-            return x * (1.f - 2e-6f);   // num^2 is evaluated to 4e-7
-    }
-    return -1.f;
-}
-
 // Records in sweep order, and the bits of the markers that are sure to change (an
 // old effect) or likely to (component 0 not certain at num^2 = `likely`).
 template <int KM>

@@ -350,6 +350,14 @@ int build_ragged_lists(brr_ctx &c)
 
 }  // namespace
 
+// FP32C chains of at least this many markers take pair-resolved rounds of 64 (see
+// use_pair_rounds).  Measured, ragged, ms per iteration with 64 markers and pair
+// products / 32 and pair products / 32 and rounds that end at a change: N 2,000 x
+// M 4,000 0.49 / 0.65 / 0.85 past the burn-in and 1.58 / 1.75 / 6.6 in it, N 20,000 x
+// M 50,000 4.6 / 6.8 / 8.2, N 100,000 x M 8,000 1.08 / 1.37 / 1.44.  Below it the
+// three differ by about a tenth of a millisecond and keep the rounds of 32.
+constexpr int64_t kWidePairM = 4096;
+
 // Whether the whole-round sweep fits this chain's slices at its round width
 // (the widest that does when none was asked for), and whether FP32C chains can
 // take pair-resolved rounds.
@@ -362,7 +370,9 @@ void brr::choose_round(brr_ctx &c)
     a.cluster = cf.cluster > 0 && c.G > 1 ? c.G : 0;
     a.rmode = kRoundPairs;
     a.has_missing = 1;
-    const int asked = cf.spec_width || cf.async_batch ? c.B : (cf.form == BRR_FORM_FP64 ? 64 : 32);
+    // FP32C rounds are 64 markers wide from kWidePairM markers on, 32 below
+    const int wide = cf.form == BRR_FORM_FP64 || cf.M >= kWidePairM ? 64 : 32;
+    const int asked = cf.spec_width || cf.async_batch ? c.B : wide;
     c.round_ok = false;
     for (int B = asked; B >= 8 && !c.round_ok && !c.no_round; B /= 2) {
         a.B = B;
@@ -373,8 +383,8 @@ void brr::choose_round(brr_ctx &c)
         if (cf.spec_width || cf.async_batch)
             break;
     }
-    c.pair_rounds = cf.form == BRR_FORM_FP32C && !c.eigen && c.round_ok && c.RB <= 32 && cf.pair_rounds >= 0 &&
-                    a.cluster == 0 && cf.async_batch == 0 && cf.N < (1 << 24);
+    c.pair_rounds = cf.form == BRR_FORM_FP32C && !c.eigen && c.round_ok && (cf.spec_width == 0 || c.RB <= 32) &&
+                    cf.pair_rounds >= 0 && a.cluster == 0 && cf.async_batch == 0 && cf.N < (1 << 24);
 }
 
 namespace {
@@ -467,16 +477,16 @@ void brr::sweep_stage(brr_ctx *c)
     std::memcpy(c->h_gK, gK.data(), sizeof(int32_t) * gK.size());
 }
 
-// FP32C sweeps choose between pair-resolved rounds and rounds that end at their
-// first change by the chain's state after the last sweep (a deterministic
-// function of the chain, which keeps it reproducible): a pair-resolved sweep
-// also forms the pair products of its rounds, a restart sweep pays one round
-// per residual-changing marker.
+// FP32C sweeps of pair_rounds = 0: pair-resolved rounds from kWidePairM markers
+// on (the Gram-blocked sweep aside).  Below, ragged markers choose by the chain's
+// state after the last sweep (a deterministic function of the chain, which keeps
+// it reproducible): a sweep that leaves few effects is followed by one whose
+// rounds end at their first change and need no pair products.
 static bool use_pair_rounds(const brr_ctx *c)
 {
     if (!c->pair_rounds || c->blocked)
         return false;
-    if (c->cfg.pair_rounds > 0)
+    if (c->cfg.pair_rounds > 0 || c->cfg.M >= kWidePairM)
         return true;
     return c->kind != BRR_KIND_DENSE && (c->last_nnz < 0 || c->last_nnz * 40 > c->cfg.M);
 }

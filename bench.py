@@ -516,8 +516,7 @@ def run_ragged(lib, gpu, torch, device, steps, warmup, cpu=True):
     torch.cuda.empty_cache()
     out = {
         "workload": R_WORKLOAD, "value": f32["rate"], "unit": "marker-updates/s",
-        "form": "fp32c (refresh 50); pair-resolved rounds of 32 markers while more than M/40 effects are non-zero, "
-                "restart rounds otherwise",
+        "form": "fp32c (refresh 50); pair-resolved rounds of 64 markers",
         "timed_iterations": f"{warmup + 1}..{warmup + steps} (burn-in)",
         "steps": steps, "ms_per_step": f32["ms_per_step"], "sweep_ms": f32["sweep_ms"], "rounds_per_step": f32["rounds"],
         "stationary": f32["late"],

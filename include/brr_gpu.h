@@ -123,12 +123,14 @@ typedef struct brr_config {
                                   one thread-block cluster of C CTAs, each holding its slice of the
                                   residual in shared memory and storing its partial sums into every
                                   CTA's shared memory (no Gram-blocked form; gram must not be 1) */
-    int32_t pair_rounds;       /* FP32C restart sweep (ragged markers other than Eigen, and dense markers
-                                  without the Gram-blocked sweep): rounds of up to 32 markers resolved
-                                  whole with exact integer pair terms of the round's markers.  0: ragged
-                                  markers in the first sweep and after any sweep that leaves more than
-                                  M/40 non-zero effects, dense markers never; 1: in every sweep;
-                                  -1: never */
+    int32_t pair_rounds;       /* FP32C whole-round sweep (ragged markers other than Eigen, and dense markers
+                                  without the Gram-blocked sweep): rounds resolved whole with exact
+                                  integer pair products of the round's markers.  0: chains of 4,096
+                                  markers or more in every sweep, with rounds of 64 (spec_width 0);
+                                  shorter ones, with rounds of 32, ragged markers in the first sweep and
+                                  after any sweep that leaves more than M/40 non-zero effects, dense
+                                  markers never; 1: in every sweep; -1: never (rounds end at their
+                                  first change).  A spec_width above 32 takes none. */
 } brr_config;
 
 /* Chain state; arrays are caller-owned, sized M (beta, comp, acum) and N (eps).

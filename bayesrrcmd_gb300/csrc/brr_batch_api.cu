@@ -63,10 +63,13 @@ struct brr_batch {
     float4 *d_gdf = nullptr;
     double *d_beta = nullptr, *d_acum = nullptr, *d_gconst = nullptr;
     int32_t *d_comp = nullptr;
-    uint8_t *d_chosen = nullptr;
+    float4 *d_pos = nullptr;
+    signed char *d_pcomp = nullptr;
+    uint8_t *d_wt = nullptr;
+    int32_t *d_moved = nullptr;
+    int *d_pairs[2] = {};
     long long *d_E = nullptr, *d_dmu = nullptr, *d_sumE = nullptr, *d_wx = nullptr, *d_prof = nullptr;
     unsigned long long *d_acc = nullptr, *d_counter = nullptr, *d_stats = nullptr;
-    unsigned *d_pacc = nullptr;
     double *d_part = nullptr;
     int *d_err = nullptr;
 
@@ -96,8 +99,8 @@ void free_batch(brr_batch *b)
         b->perm_future.wait();
     void *dev[] = {b->d_codes, b->d_counts, b->d_lut,  b->d_scale, b->d_colsum, b->d_slice_lo, b->d_group,
                    b->d_gK,    b->d_order,  b->d_rec,  b->d_crec,  b->d_gcf,    b->d_gdf,      b->d_beta,     b->d_acum,
-                   b->d_gconst, b->d_comp,  b->d_chosen, b->d_E,    b->d_dmu,   b->d_sumE,   b->d_wx,       b->d_prof,
-                   b->d_acc,   b->d_counter, b->d_stats, b->d_pacc, b->d_part,  b->d_err};
+                   b->d_gconst, b->d_comp,  b->d_pos,   b->d_pcomp, b->d_wt, b->d_moved, b->d_pairs[0], b->d_pairs[1], b->d_E,    b->d_dmu,   b->d_sumE,   b->d_wx,       b->d_prof,
+                   b->d_acc,   b->d_counter, b->d_stats, b->d_part,  b->d_err};
     for (void *p : dev)
         cudaFree(p);
     cudaFreeHost(b->h_order);
@@ -136,7 +139,12 @@ void release_pack_buffers(brr_batch *b)
     drop_dev(b->d_beta);
     drop_dev(b->d_acum);
     drop_dev(b->d_comp);
-    drop_dev(b->d_chosen);
+    drop_dev(b->d_pos);
+    drop_dev(b->d_pcomp);
+    drop_dev(b->d_wt);
+    drop_dev(b->d_moved);
+    drop_dev(b->d_pairs[0]);
+    drop_dev(b->d_pairs[1]);
     drop_dev(b->d_gconst);
     drop_dev(b->d_E);
     drop_dev(b->d_dmu);
@@ -146,15 +154,13 @@ void release_pack_buffers(brr_batch *b)
     drop_dev(b->d_acc);
     drop_dev(b->d_counter);
     drop_dev(b->d_stats);
-    drop_dev(b->d_pacc);
     drop_dev(b->d_part);
     drop_dev(b->d_err);
     cudaFreeHost(b->h_order);
     b->h_order = nullptr;
 }
 
-size_t acc_words(int C) { return (size_t)kBatchCopies * C * kBatchBlock; }
-size_t pacc_words() { return (size_t)2 * kBatchPCopies * kBatchBlock * kBatchBlock; }
+size_t acc_words(int C) { return (size_t)2 * kBatchCopies * C * kBatchBlock; }
 size_t stats_words(int C, int ng) { return (size_t)C * (ng * kMaxK + 2 * ng); }
 
 // Sampler constants of chain c (src/BayesRBase.cpp:309-333), as in the
@@ -294,12 +300,12 @@ int brr_batch_create(const brr_config *cfg, int32_t chains, brr_batch **out)
     }
     b->kext = (int)(maxch * 16);
     b->col_stride = 16 * ((c.N + 63) / 64);
-    const size_t smem = batch_smem_bytes(chains, b->kext, G);
+    const size_t smem = batch_smem_bytes(chains, b->kext);
     const int per_sm = smem <= (size_t)prop.sharedMemPerBlockOptin ? batch_max_ctas_per_sm(chains, b->kext, smem) : 0;
     if (per_sm < 1 || (int64_t)per_sm * b->sms < G) {
-        // shared memory per individual of a slice: genotypes 64 B, residual limbs 8 B per chain, codes 8 B
-        const int64_t fixed = 256 * (int64_t)chains + 2048;
-        const int64_t per_ind = 72 + 8 * (int64_t)chains;
+        // shared memory per individual of a slice: genotypes 64 B, residual limbs 8 B per chain
+        const int64_t fixed = batch_tile_bytes(chains) + 9216;
+        const int64_t per_ind = 64 + 8 * (int64_t)chains;
         const int64_t cap = (int64_t)b->sms * (((int64_t)prop.sharedMemPerBlockOptin - fixed) / per_ind / 16 * 16);
         free_batch(b);
         delete b;
@@ -346,12 +352,14 @@ int brr_batch_pack_bed_device(brr_batch *b, const uint8_t *d_bed, int64_t nbytes
             balloc(&b->d_gdf, (size_t)C * cf.n_groups * kMaxK) ||
             balloc(&b->d_beta, (size_t)(C * M)) ||
             balloc(&b->d_acum, (size_t)(C * M)) || balloc(&b->d_comp, (size_t)(C * M)) ||
-            balloc(&b->d_chosen, (size_t)(C * M)) ||
+            balloc(&b->d_pos, (size_t)(C * M)) || balloc(&b->d_pcomp, (size_t)(C * M)) ||
+            balloc(&b->d_wt, (size_t)2 * batch_tile_bytes(b->C)) || balloc(&b->d_moved, (size_t)2 * kBatchMaxChains) ||
+            balloc(&b->d_pairs[0], batch_pair_words(M)) || balloc(&b->d_pairs[1], batch_pair_words(M)) ||
             balloc(&b->d_gconst, (size_t)C * cf.n_groups * kMaxK * 4) || balloc(&b->d_E, (size_t)(C * cf.N)) ||
             balloc(&b->d_dmu, (size_t)C) || balloc(&b->d_sumE, (size_t)C) ||
             balloc(&b->d_wx, (size_t)C * (kBatchBlock + 1)) || balloc(&b->d_prof, 8) ||
             balloc(&b->d_acc, acc_words(b->C)) || balloc(&b->d_counter, 64) ||
-            balloc(&b->d_stats, stats_words(b->C, cf.n_groups)) || balloc(&b->d_pacc, pacc_words()) ||
+            balloc(&b->d_stats, stats_words(b->C, cf.n_groups)) ||
             balloc(&b->d_part, (size_t)b->G * C * 2) || balloc(&b->d_err, 1) ||
             cudaMallocHost((void **)&b->h_order, sizeof(uint32_t) * M) != cudaSuccess) {
             cudaGetLastError();
@@ -540,7 +548,6 @@ int brr_batch_iterate(brr_batch *b, int32_t n_iter)
         b->perm_future.wait();
         std::memcpy(b->h_order, b->perm_next.data(), sizeof(uint32_t) * M);
         BATCH_CUDA(cudaMemcpyAsync(b->d_order, b->h_order, sizeof(uint32_t) * M, cudaMemcpyHostToDevice, b->st));
-        BATCH_CUDA(launch_batch_draws(cf.seed, cf.chain, it, M, C, b->d_order, b->d_beta, b->d_crec, b->st));
         for (int c = 0; c < C; ++c)
             chain_constants(b, c, gc.data() + (size_t)c * ng * kMaxK * 4, gcf.data() + (size_t)c * ng * kMaxK * 2,
                             gdf.data() + (size_t)c * ng * kMaxK, gK.data());
@@ -552,7 +559,6 @@ int brr_batch_iterate(brr_batch *b, int32_t n_iter)
         BATCH_CUDA(cudaMemcpyAsync(b->d_sumE, b->sumE.data(), sizeof(long long) * C, cudaMemcpyHostToDevice, b->st));
         BATCH_CUDA(launch_batch_gather(b->d_order, M, b->d_scale, b->d_counts, b->d_group, b->d_rec, b->st));
         BATCH_CUDA(cudaMemsetAsync(b->d_acc, 0, sizeof(unsigned long long) * acc_words(C), b->st));
-        BATCH_CUDA(cudaMemsetAsync(b->d_pacc, 0, sizeof(unsigned) * pacc_words(), b->st));
         BATCH_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long) * 64, b->st));
         BATCH_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(int), b->st));
         BATCH_CUDA(cudaMemsetAsync(b->d_prof, 0, sizeof(long long) * 8, b->st));
@@ -568,7 +574,10 @@ int brr_batch_iterate(brr_batch *b, int32_t n_iter)
         a.slice_lo = b->d_slice_lo;
         a.codes = b->d_codes;
         a.col_stride = b->col_stride;
+        a.order = b->d_order;
         a.rec = b->d_rec;
+        a.pairs[0] = b->d_pairs[0];
+        a.pairs[1] = b->d_pairs[1];
         a.gconst = b->d_gconst;
         a.gcf = b->d_gcf;
         a.gdf = b->d_gdf;
@@ -577,12 +586,14 @@ int brr_batch_iterate(brr_batch *b, int32_t n_iter)
         a.beta = b->d_beta;
         a.acum = b->d_acum;
         a.comp = b->d_comp;
-        a.chosen = b->d_chosen;
+        a.pos = b->d_pos;
+        a.pcomp = b->d_pcomp;
+        a.wt = b->d_wt;
+        a.moved = b->d_moved;
         a.E = b->d_E;
         a.dmu = b->d_dmu;
         a.sumE = b->d_sumE;
         a.acc = b->d_acc;
-        a.pacc = b->d_pacc;
         a.wx = b->d_wx;
         a.counter = b->d_counter;
         a.part = b->d_part;
@@ -590,11 +601,13 @@ int brr_batch_iterate(brr_batch *b, int32_t n_iter)
         a.timeout_ns = b->wait_limit_ns;
         a.phantom = b->phantom;
         a.prof = b->profile ? b->d_prof : nullptr;
+        BATCH_CUDA(launch_batch_draws(cf.seed, cf.chain, it, a, kmax, b->d_group, b->d_crec, b->st));
         BATCH_CUDA(cudaEventRecord(b->ev[0], b->st));
+        BATCH_CUDA(launch_batch_pairs(b->d_order, M, b->d_codes, b->col_stride, b->d_pairs[0], b->d_pairs[1], b->sms, b->st));
         BATCH_CUDA(launch_sweep_batch(a, kmax, b->st));
         BATCH_CUDA(cudaEventRecord(b->ev[1], b->st));
         BATCH_CUDA(cudaMemsetAsync(b->d_stats, 0, sizeof(unsigned long long) * stats.size(), b->st));
-        BATCH_CUDA(launch_batch_stats(M, C, b->d_group, b->d_comp, b->d_chosen, b->d_beta, ng, b->d_stats, b->st));
+        BATCH_CUDA(launch_batch_finish(a, kmax, b->d_stats, b->st));
         BATCH_CUDA(cudaMemcpyAsync(stats.data(), b->d_stats, sizeof(unsigned long long) * stats.size(),
                                    cudaMemcpyDeviceToHost, b->st));
         BATCH_CUDA(cudaMemcpyAsync(part.data(), b->d_part, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, b->st));
@@ -737,7 +750,7 @@ int brr_batch_get_geometry(brr_batch *b, int32_t *ctas, int32_t *slice, int64_t 
     if (slice)
         *slice = b->kext;
     if (smem_bytes)
-        *smem_bytes = (int64_t)batch_smem_bytes(b->C, b->kext, b->G);
+        *smem_bytes = (int64_t)batch_smem_bytes(b->C, b->kext);
     return BRR_OK;
 }
 

@@ -161,26 +161,32 @@ constexpr int kBatchFrac = 40;
 constexpr int kBatchLimbs = 4;
 constexpr int kBatchBlock = 32;          // markers per block
 constexpr int kBatchMaxChains = 64;
-constexpr int kBatchCopies = 8;          // copies of the dot accumulators (CTA s adds into s % 8)
-constexpr int kBatchPCopies = 4;         // copies of the block Gram accumulators (CTA s adds into s % 4)
+constexpr int kBatchCopies = 4;          // copies of the dot accumulators (CTA s adds into s % 4)
+
+// Bytes of a block's update coefficients: FP16 limbs of W as the tensor-core
+// operand, then those of the chains' constants in FP32.
+__host__ __device__ constexpr int batch_tile_bytes(int C) { return 4 * C * kBatchBlock * 2 + C * kBatchLimbs * 4; }
 
 struct alignas(16) BatchRec {
-    double sigma;        // 1 / sd of the marker column
-    double colmean;      // column mean
-    double S;            // sum of the genotypes over all individuals (exact integer)
-    uint32_t j;          // marker id
+    double sA, sB;         // sigma 2^-kBatchFrac and -sigma colmean 2^-kBatchFrac (sigma: 1 / sd of the marker column)
+    float sh, sl, mh, ml;  // sigma and the column mean as double-float pairs
+    int32_t S;             // sum of the genotypes over all individuals
     int32_t group;
+    uint32_t j;            // marker id
+    uint32_t pad;
 };
-static_assert(sizeof(BatchRec) == 32, "BatchRec must be 32 bytes");
+static_assert(sizeof(BatchRec) == 48, "BatchRec must be 48 bytes");
 
-// Per chain and sweep position: beta_old of the marker and its draws.
-struct alignas(32) ChainRec {
-    double beta_old;
-    double u;
-    double z;
-    double pad;
+// Per chain and sweep position: the marker's old effect and its draws.
+constexpr float kHasEffect = -2.f;
+struct alignas(16) ChainRec {
+    double bN1;            // beta_old (N - 1)
+    double u, z;
+    float boh, bol, zh, zl;   // beta_old and z as double-float pairs
+    float uf;
+    float s0;              // num^2 up to which component 0 is certain; kHasEffect: beta_old is not zero
 };
-static_assert(sizeof(ChainRec) == 32, "ChainRec must be 32 bytes");
+static_assert(sizeof(ChainRec) == 48, "ChainRec must be 48 bytes");
 
 struct BatchArgs {
     int64_t N, M;
@@ -191,7 +197,11 @@ struct BatchArgs {
     const int32_t *slice_lo;         // G+1 slice boundaries
     const uint8_t *codes;            // M x col_stride 2-bit codes
     int64_t col_stride;
+    const uint32_t *order;           // marker ids in sweep order
     const BatchRec *rec;             // M records in sweep order
+    // pair sums (genotype x genotype) of 64 consecutive markers of the sweep order,
+    // [64][64] each: [0] of blocks (0, 1), (2, 3), ..., [1] of blocks (1, 2), (3, 4), ...
+    const int *pairs[2];
     const double *gconst;            // [C][n_groups][kMaxK][4] sampler constants per chain
     const float *gcf;                // [C][n_groups][kMaxK][2] FP32 {logL_k - logL_0 constant, h_k}
     const float4 *gdf;               // [C][n_groups][kMaxK] double-float {sdk hi, lo, invden hi, lo}
@@ -199,14 +209,16 @@ struct BatchArgs {
     const ChainRec *crec;            // [C][M] in sweep order
     double *beta, *acum;             // [C][M] by marker id
     int32_t *comp;                   // [C][M]
-    uint8_t *chosen;                 // [C][M] the sampler chose a component in this sweep
+    float4 *pos;                     // [C][M] by sweep position: num and the new effect, double-float pairs
+    signed char *pcomp;              // [C][M] by sweep position: the component, -1 where none was chosen
     long long *E;                    // [C][N] fixed-point residual (in at sweep start, out at the end)
     const long long *dmu;            // [C] fixed-point shift added to E at the start (updateMu)
     long long *sumE;                 // [C] exact residual total, carried through the sweep
-    unsigned long long *acc;         // [kBatchCopies][C][32] dot-product accumulators (zero at launch)
-    unsigned *pacc;                  // [2][kBatchPCopies][32][32] integer block Gram accumulators (zero at launch)
-    long long *wx;                   // [C][33] per block: W per marker, then the constant
-    unsigned long long *counter;     // 2 barrier counters, 32 words apart (zero at launch)
+    unsigned long long *acc;         // [2][kBatchCopies][8][C][4] dot-product accumulators (zero at launch)
+    uint8_t *wt;                     // [2][batch_tile_bytes(C)] update coefficients of a block
+    int32_t *moved;                  // [2][kBatchMaxChains] whether a chain changed in a block
+    long long *wx;                   // [C][33] W per marker, then the constant (CTAs that resolve several chains per warp)
+    unsigned long long *counter;     // 4 arrival counters, 16 words apart (zero at launch)
     double *part;                    // [G][C][2] per slice: sum(E) (bits of an int64) and sum(eps^2)
     int *err;
     uint64_t timeout_ns;
@@ -221,11 +233,14 @@ cudaError_t launch_batch_gather(const uint32_t *order, int64_t M, const double *
                                 const int32_t *group, BatchRec *rec, cudaStream_t st);
 // Per chain c and sweep position q: beta_old of marker order[q] and its draws
 // (u, z) from chain (chain0 + c)'s stream for iteration it.
-cudaError_t launch_batch_draws(uint32_t seed, uint32_t chain0, uint32_t it, int64_t M, int C, const uint32_t *order,
-                               const double *beta, ChainRec *crec, cudaStream_t st);
-cudaError_t launch_batch_stats(int64_t M, int C, const int32_t *group, const int32_t *comp, const uint8_t *chosen,
-                               const double *beta, int n_groups, unsigned long long *out, cudaStream_t st);
-size_t batch_smem_bytes(int C, int kext, int G);
+cudaError_t launch_batch_draws(uint32_t seed, uint32_t chain0, uint32_t it, const BatchArgs &a, int kmax,
+                               const int32_t *group, ChainRec *crec, cudaStream_t st);
+cudaError_t launch_batch_finish(const BatchArgs &a, int kmax, unsigned long long *out, cudaStream_t st);
+// Integer pair sums of a batch's consecutive blocks (BatchArgs::pairs; every genotype present).
+size_t batch_pair_words(int64_t M);   // per half
+cudaError_t launch_batch_pairs(const uint32_t *order, int64_t M, const uint8_t *codes, int64_t col_stride, int *sums0,
+                               int *sums1, int sms, cudaStream_t st);
+size_t batch_smem_bytes(int C, int kext);
 int batch_max_ctas_per_sm(int C, int kext, size_t smem);
 cudaError_t launch_sweep_batch(const BatchArgs &a, int kmax, cudaStream_t st);
 

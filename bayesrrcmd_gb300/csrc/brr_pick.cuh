@@ -321,12 +321,11 @@ __device__ __forceinline__ float certain_zero(float uf, const double *gc, int K)
 
 // Component of one marker at num^2 = x by a whole warp, one mixture component per
 // lane: the certified decision of pick_margin without its margin; -2 where it cannot
-// certify.  gcf: the group's FP32 constants {dc_k, h_k}.  About 40 instructions against
+// certify.  f: the FP32 constants {dc_k, h_k} of the group's component k = lane.  About 40 instructions against
 // 150, which matters where the decision lies on a sweep's chain.
 template <int KM>
-__device__ __forceinline__ int pick_lanes(int lane, float x, float uf, const float *gcf, int K)
+__device__ __forceinline__ int pick_lanes(int lane, float x, float uf, float2 f, int K)
 {
-    const float2 f = reinterpret_cast<const float2 *>(gcf)[lane & (kMaxK - 1)];
     const bool in = lane < K;
     const float hx = f.y * x;
     const float D = in ? f.x + hx : 0.f;   // lane 0: 0
@@ -346,6 +345,12 @@ __device__ __forceinline__ int pick_lanes(int lane, float x, float uf, const flo
     const int comp = __popc(__ballot_sync(0xffffffffu, in && c < target));
     const bool close = __any_sync(0xffffffffu, in && fabsf(c - target) < tol);
     return (close || comp >= K || !(mag < 300.f)) ? -2 : comp;
+}
+
+template <int KM>
+__device__ __forceinline__ int pick_lanes(int lane, float x, float uf, const float *gcf, int K)
+{
+    return pick_lanes<KM>(lane, x, uf, reinterpret_cast<const float2 *>(gcf)[lane & (kMaxK - 1)], K);
 }
 
 // num^2 of num = nh + nl, to 4e-7.

@@ -1574,6 +1574,30 @@ cudaError_t launch_round_pairs(const uint32_t *order, int64_t M, int64_t N, int 
     return cudaGetLastError();
 }
 
+size_t batch_pair_words(int64_t M) { return (size_t)((M + 63) / 64) * 64 * 64; }
+
+cudaError_t launch_batch_pairs(const uint32_t *order, int64_t M, const uint8_t *codes, int64_t col_stride, int *sums0,
+                               int *sums1, int sms, cudaStream_t st)
+{
+    for (int half = 0; half < 2; ++half) {
+        const int64_t m = M - 32 * half;
+        if (m < 1)
+            break;
+        const int64_t nb = (m + 63) / 64;
+        int *sums = half ? sums1 : sums0;
+        const int64_t split = imax64(1, imin64((2 * sms + nb - 1) / nb, (col_stride + kPairSeg - 1) / kPairSeg));
+        cudaError_t e = cudaSuccess;
+        if (split > 1)
+            e = cudaMemsetAsync(sums, 0, sizeof(int) * (size_t)nb * 4096, st);
+        if (e == cudaSuccess)
+            e = pair_sums<64, 0>(order + 32 * half, m, 64, codes, col_stride, nullptr, 1, sums, nb * 4096,
+                                 dim3((unsigned)nb, (unsigned)split, 64 / kPairCols), st);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t launch_round_finish(int64_t M, int form, int kmax, const double *num, const double *u, const int32_t *group,
                                 const double *gconst, const int32_t *gK, double *acum, cudaStream_t st)
 {

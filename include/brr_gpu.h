@@ -291,9 +291,10 @@ int brr_batch_iterate(brr_batch *b, int32_t n_iter);
 int brr_batch_get_chain_state(brr_batch *b, int32_t chain, brr_state *st);
 /* Device time of the sweeps and of the whole last brr_batch_iterate call (ms);
  * cycles (optional, 8 values), summed over the sweeps of that call, measured on
- * CTA 0 (indicative): the dot, publish, resolve and update phases; then, of
- * the resolve phase, the wait for all CTAs' dot products, chain 0's own
- * resolve, chain 0's sampling steps, and the wait for the slowest chain. */
+ * CTA 0 (indicative), whose workers and resolvers run side by side: [0] dot
+ * products, [1] their publication, [3] residual updates, [7] the workers' wait for the
+ * resolved chains; [2] all of chain 0's resolve, of it [4] the wait for all CTAs' dot
+ * products and [5] the rest, [6] chain 0's sampling steps. */
 int brr_batch_get_timing(brr_batch *b, double *sweep_ms, double *total_ms, int64_t *cycles);
 /* Phase counters on (1) or off (0, the default; the cycles then read zero):
  * the counting runs a variant of the sweep kernel with clock reads. */

@@ -128,6 +128,7 @@ void release_pack_buffers(brr_ctx &c)
     drop_dev(c.d_eps_hi);
     drop_dev(c.d_eps_lo);
     drop_dev(c.d_emax);
+    drop_dev(c.d_pstat);
     drop_host(c.h_order);
     drop_host(c.h_stats);
     drop_host(c.h_part);
@@ -186,6 +187,7 @@ void free_all(brr_ctx *c)
     cudaFree(c->d_rgram);
     cudaFree(c->d_num);
     cudaFree(c->d_emax);
+    cudaFree(c->d_pstat);
     cudaFree(c->d_eps2);
     cudaFree(c->d_eps_hi2);
     cudaFree(c->d_eps_lo2);
@@ -308,41 +310,24 @@ int build_ragged_lists(brr_ctx &c)
     const int64_t MG1 = M * (int64_t)c.G + 1;
     if (3 * MG1 > (int64_t)INT_MAX)
         return fail(BRR_ERR_ARG, "ragged offset table too large for int32");
+    for (int k = 0; k < 3; ++k)
+        if (c.rtot[k] > (int64_t)INT_MAX)
+            return fail(BRR_ERR_ARG, "ragged index list longer than 2^31 entries");
+    // offsets, then the scans' words
+    const size_t words = (size_t)(3 * MG1 + 3 * scan_tiles(MG1));
     cudaFree(c.d_roff);
     c.d_roff = nullptr;
-    if (dalloc(&c.d_roff, (size_t)(3 * MG1)))
+    if (dalloc(&c.d_roff, words))
         return fail(BRR_ERR_OOM, "device allocation failed");
-    BRR_CUDA(cudaMemsetAsync(c.d_roff, 0, sizeof(int32_t) * 3 * MG1, c.st));
-    BRR_CUDA(launch_ragged_slice_counts(c.d_codes, c.col_stride, M, c.G, c.d_slice_lo, c.d_roff, c.st));
-    int32_t *tmp = nullptr;
-    if (dalloc(&tmp, (size_t)((MG1 + 1023) / 1024 + 1)))
-        return fail(BRR_ERR_OOM, "device allocation failed");
-    // totals must fit int32: the counts bound them by the genotype counts
-    std::vector<int64_t> cnt(M * 4);
-    BRR_CUDA(cudaMemcpyAsync(cnt.data(), c.d_counts, sizeof(int64_t) * M * 4, cudaMemcpyDeviceToHost, c.st));
-    BRR_CUDA(cudaStreamSynchronize(c.st));
-    int64_t tot[3] = {0, 0, 0};
-    for (int64_t j = 0; j < M; ++j) {
-        tot[0] += cnt[4 * j + 1];
-        tot[1] += cnt[4 * j + 2];
-        tot[2] += cnt[4 * j + 3];
-    }
     for (int k = 0; k < 3; ++k) {
-        if (tot[k] > (int64_t)INT_MAX) {
-            cudaFree(tmp);
-            return fail(BRR_ERR_ARG, "ragged index list longer than 2^31 entries");
-        }
-        BRR_CUDA(launch_exclusive_scan_i32(c.d_roff + k * MG1, MG1, tmp, c.st));
         cudaFree(c.d_ridx[k]);
         c.d_ridx[k] = nullptr;
-        if (dalloc(&c.d_ridx[k], (size_t)tot[k] + 1)) {
-            cudaFree(tmp);
+        if (dalloc(&c.d_ridx[k], (size_t)c.rtot[k] + 1))
             return fail(BRR_ERR_OOM, "device allocation failed");
-        }
-        c.rtot[k] = tot[k];
+        BRR_CUDA(cudaMemsetAsync(c.d_roff + (k + 1) * MG1 - 1, 0, sizeof(int32_t), c.st));
     }
-    BRR_CUDA(cudaStreamSynchronize(c.st));
-    cudaFree(tmp);
+    BRR_CUDA(launch_ragged_slice_counts(c.d_codes, c.col_stride, M, c.G, c.d_slice_lo, c.d_roff, c.st));
+    BRR_CUDA(launch_exclusive_scans_i32(c.d_roff, MG1, 3, c.d_roff + 3 * MG1, c.st));
     BRR_CUDA(launch_ragged_fill(c.d_codes, c.col_stride, M, c.G, c.d_slice_lo, c.d_roff, c.d_roff + MG1,
                                 c.d_roff + 2 * MG1, c.d_ridx[0], c.d_ridx[1], c.d_ridx[2], c.st));
     return BRR_OK;
@@ -1149,7 +1134,8 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
             dalloc(&c.d_stats, (size_t)cf.n_groups * kMaxK + cf.n_groups + 1) ||
             dalloc(&c.d_part, (size_t)std::max(2 * c.G, kPartBlocks)) || dalloc(&c.d_err, 1) ||
             dalloc(&c.d_rounds, 1) || dalloc(&c.d_prof, 16) || dalloc(&c.d_gstage, sweep_block_stage_bytes(kMaxSpec) / sizeof(double)) || dalloc(&c.d_group, (size_t)M) || dalloc(&c.d_ystd, (size_t)cf.N) ||
-            dalloc(&c.d_nzj, (size_t)M) || dalloc(&c.d_nzb, (size_t)M) || dalloc(&c.d_emax, (size_t)kPartBlocks)) {
+            dalloc(&c.d_nzj, (size_t)M) || dalloc(&c.d_nzb, (size_t)M) || dalloc(&c.d_emax, (size_t)kPartBlocks) ||
+            dalloc(&c.d_pstat, 4)) {
             release_pack_buffers(c);
             return fail(BRR_ERR_OOM, "device allocation failed");
         }
@@ -1181,35 +1167,25 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
     }
     BRR_CUDA(cudaMemcpy(c.d_slice_lo, c.slice_lo.data(), sizeof(int32_t) * (c.G + 1), cudaMemcpyHostToDevice));
     BRR_CUDA(launch_pack_counts(d_bed, cf.N, M, c.d_codes, c.col_stride, c.d_counts, c.st));
-    int *d_bad = nullptr;
-    if (dalloc(&d_bad, 1))
-        return fail(BRR_ERR_OOM, "device allocation failed");
-    const int big = INT_MAX;
-    int bad = INT_MAX;
-    cudaError_t le = cudaMemcpy(d_bad, &big, sizeof(int), cudaMemcpyHostToDevice);
-    if (le == cudaSuccess)
-        le = cf.kind == BRR_KIND_DENSE
+    // totals of the counts, and the first marker that does not vary (0x7F7F7F7F: none)
+    unsigned long long stat[4] = {0, 0, 0, 0};
+    int *d_bad = reinterpret_cast<int *>(c.d_pstat + 3);
+    BRR_CUDA(cudaMemsetAsync(d_bad, 0x7F, sizeof(int), c.st));
+    BRR_CUDA(cf.kind == BRR_KIND_DENSE
                  ? launch_dense_tables(c.d_counts, cf.N, M, c.d_table, c.d_scale, c.d_colsum, d_bad, c.st)
-                 : launch_ragged_stats(c.d_counts, cf.N, M, c.eigen ? 1 : 0, c.d_table, d_bad, c.st);
-    if (le == cudaSuccess)
-        le = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c.st);
-    if (le == cudaSuccess)
-        le = cudaStreamSynchronize(c.st);
-    cudaFree(d_bad);
-    if (le != cudaSuccess)
-        return fail(BRR_ERR_CUDA, std::string("marker statistics: ") + cudaGetErrorString(le));
-    BRR_CUDA(cudaGetLastError());
-    if (bad != INT_MAX)
+                 : launch_ragged_stats(c.d_counts, cf.N, M, c.eigen ? 1 : 0, c.d_table, d_bad, c.st));
+    BRR_CUDA(launch_count_totals(c.d_counts, M, c.d_pstat, c.st));
+    BRR_CUDA(cudaMemcpyAsync(stat, c.d_pstat, sizeof(stat), cudaMemcpyDeviceToHost, c.st));
+    BRR_CUDA(cudaStreamSynchronize(c.st));
+    int bad;
+    std::memcpy(&bad, &stat[3], sizeof bad);
+    if (bad != 0x7F7F7F7F)
         return fail(BRR_ERR_MARKER, "marker " + std::to_string(bad) +
                                         " does not vary or is all missing; SNPs that do not vary should be "
                                         "removed prior to analysis");
-    {
-        std::vector<int64_t> cnt(M * 4);
-        BRR_CUDA(cudaMemcpy(cnt.data(), c.d_counts, sizeof(int64_t) * M * 4, cudaMemcpyDeviceToHost));
-        c.has_missing = false;
-        for (int64_t j = 0; j < M && !c.has_missing; ++j)
-            c.has_missing = cnt[4 * j + 3] != 0;
-    }
+    for (int k = 0; k < 3; ++k)
+        c.rtot[k] = (int64_t)stat[k];
+    c.has_missing = stat[2] != 0;
     if (c.kind == BRR_KIND_RAGGED) {
         const int rc = build_ragged_lists(c);
         if (rc)

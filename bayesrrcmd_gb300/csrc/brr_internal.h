@@ -267,7 +267,10 @@ cudaError_t launch_ragged_stats(const int64_t *counts, int64_t N, int64_t M, int
                                 int *bad, cudaStream_t st);
 cudaError_t launch_ragged_slice_counts(const uint8_t *codes, int64_t col_stride, int64_t M, int G,
                                        const int32_t *slice_lo, int32_t *cnt3, cudaStream_t st);
-cudaError_t launch_exclusive_scan_i32(int32_t *data, int64_t n, int32_t *tmp, cudaStream_t st);
+cudaError_t launch_count_totals(const int64_t *counts, int64_t M, unsigned long long *tot, cudaStream_t st);
+// Exclusive scans of `arrays` arrays of n elements; tmp: arrays * scan_tiles(n) words.
+int64_t scan_tiles(int64_t n);
+cudaError_t launch_exclusive_scans_i32(int32_t *data, int64_t n, int arrays, int32_t *tmp, cudaStream_t st);
 cudaError_t launch_ragged_fill(const uint8_t *codes, int64_t col_stride, int64_t M, int G,
                                const int32_t *slice_lo, const int32_t *off0, const int32_t *off1,
                                const int32_t *off2, uint16_t *idx0, uint16_t *idx1, uint16_t *idx2,

@@ -16,61 +16,94 @@ namespace brr {
 // allele2 = !bit1; (0,1) is missing (src/densemarkerbuilder.cpp:30).
 //   code 0 -> g = 2, code 1 -> missing, code 2 -> g = 1, code 3 -> g = 0.
 
+// Genotype counts of the 16 codes in a word whose low 2 * n bits are valid, by
+// population counts: g = 1, g = 2, missing.
+struct CodeCounts {
+    int c1, c2, cm;
+};
+__device__ __forceinline__ void count_codes(unsigned w, unsigned valid, CodeCounts &c)
+{
+    const unsigned m = valid & 0x55555555u, l = w & m, h = (w >> 1) & m;
+    c.c1 += __popc(h & ~l);
+    c.cm += __popc(l & ~h);
+    c.c2 += __popc(m & ~(l | h));
+}
+// Mask of the first n codes of a word.
+__device__ __forceinline__ unsigned code_mask(int64_t n)
+{
+    return n <= 0 ? 0u : n >= 16 ? 0xFFFFFFFFu : (1u << (2 * n)) - 1u;
+}
+
+// One warp per marker, a lane per 16 bytes of its column: the payload's bytes start
+// at any address, so a lane reads the five aligned words around its 16 bytes and
+// shifts them into place; the few lanes whose words would leave the payload read
+// bytes.  Bits past the last individual become missing codes.  Bound by HBM: a byte
+// at a time took 374 us for N = 20,011 x M = 20,000 (100 MB in and out), this 50 us.
 __global__ void __launch_bounds__(kThreads) k_pack_counts(const uint8_t *__restrict__ bed, int64_t N,
                                                           int64_t M, uint8_t *__restrict__ codes,
                                                           int64_t col_stride, int64_t *__restrict__ counts)
 {
-    const int64_t cb = (N + 3) >> 2;
-    __shared__ int red[4][kThreads / 32];
-    for (int64_t j = blockIdx.x; j < M; j += gridDim.x) {
+    const int64_t cb = (N + 3) >> 2, chunks = col_stride / 16;
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    const uint8_t *const end = bed + M * cb;
+    for (int64_t j = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); j < M; j += warps) {
         const uint8_t *src = bed + j * cb;
-        uint8_t *dst = codes + j * col_stride;
-        int c0 = 0, c1 = 0, c2 = 0, c3 = 0;
-        for (int64_t b = threadIdx.x; b < col_stride; b += blockDim.x) {
-            if (b < cb) {
-                unsigned v = src[b];
-                const int64_t i0 = b * 4;
-                const int nvalid = (int)imin64(4, N - i0);
-                if (nvalid < 4)   // the payload's own padding bits: missing codes, as past the last byte
-                    v = (v & ((1u << (2 * nvalid)) - 1u)) | (0x55u & ~((1u << (2 * nvalid)) - 1u));
-                dst[b] = (uint8_t)v;
+        uint4 *dst = reinterpret_cast<uint4 *>(codes + j * col_stride);
+        CodeCounts c{0, 0, 0};
+#pragma unroll 2
+        for (int64_t k = lane; k < chunks; k += 32) {
+            const uint8_t *at = src + 16 * k;
+            const uint32_t *al = reinterpret_cast<const uint32_t *>((uintptr_t)at & ~(uintptr_t)3);
+            unsigned w[4];
+            if (reinterpret_cast<const uint8_t *>(al) >= bed && reinterpret_cast<const uint8_t *>(al + 5) <= end) {
+                unsigned x[5];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (k < nvalid) {
-                        const unsigned c = (v >> (2 * k)) & 3u;
-                        c0 += c == 3u;   // g = 0
-                        c1 += c == 2u;   // g = 1
-                        c2 += c == 0u;   // g = 2
-                        c3 += c == 1u;   // missing
-                    }
-                }
+                for (int q = 0; q < 5; ++q)
+                    x[q] = __ldg(al + q);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    w[q] = __funnelshift_r(x[q], x[q + 1], 8u * (unsigned)((uintptr_t)at & 3));
             } else {
-                dst[b] = 0x55;  // padding: missing codes
-            }
-        }
-        // block reduction of the four counters
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            c0 += __shfl_xor_sync(0xffffffffu, c0, o);
-            c1 += __shfl_xor_sync(0xffffffffu, c1, o);
-            c2 += __shfl_xor_sync(0xffffffffu, c2, o);
-            c3 += __shfl_xor_sync(0xffffffffu, c3, o);
+                for (int q = 0; q < 4; ++q) {
+                    w[q] = 0u;
+                    for (int e = 0; e < 4; ++e)
+                        if (16 * k + 4 * q + e < cb)
+                            w[q] |= (unsigned)at[4 * q + e] << (8 * e);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned v = code_mask(N - 64 * k - 16 * q);
+                count_codes(w[q], v, c);
+                w[q] = (w[q] & v) | (0x55555555u & ~v);
+            }
+            dst[k] = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-        if (l == 0) {
-            red[0][w] = c0;
-            red[1][w] = c1;
-            red[2][w] = c2;
-            red[3][w] = c3;
-        }
-        __syncthreads();
-        if (threadIdx.x < 4) {
-            long long s = 0;
-            for (int q = 0; q < (int)(blockDim.x >> 5); ++q)
-                s += red[threadIdx.x][q];
-            counts[4 * j + threadIdx.x] = s;
-        }
-        __syncthreads();
+        const int c1 = __reduce_add_sync(0xffffffffu, c.c1), c2 = __reduce_add_sync(0xffffffffu, c.c2),
+                  cm = __reduce_add_sync(0xffffffffu, c.cm);
+        if (lane < 4)
+            counts[4 * j + lane] = lane == 0 ? N - c1 - c2 - cm : lane == 1 ? c1 : lane == 2 ? c2 : cm;
+    }
+}
+
+// Totals over the markers of the counts of g = 1, g = 2 and missing.
+__global__ void __launch_bounds__(kThreads) k_count_totals(const int64_t *__restrict__ counts, int64_t M,
+                                                           unsigned long long *__restrict__ tot)
+{
+    long long t[3] = {0, 0, 0};
+    for (int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x; j < M; j += (int64_t)gridDim.x * kThreads)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            t[k] += counts[4 * j + 1 + k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+        if ((threadIdx.x & 31) == 0 && t[k])
+            atomicAdd(&tot[k], (unsigned long long)t[k]);
     }
 }
 
@@ -149,35 +182,44 @@ __global__ void k_ragged_stats(const int64_t *__restrict__ counts, int64_t N, in
         atomicMin(bad, (int)j);
 }
 
-// Per (marker, slice) counts of ones / twos / missing for the slice-major
-// ragged layout.  One CTA per marker, threads over slices.
+// Per (marker, slice) counts of ones / twos / missing for the slice-major ragged
+// layout: a thread per slice, 64 individuals (16 bytes: slices begin on chunks) at a
+// time.  N = 20,011 x M = 20,000, 152 slices: 382 us an individual at a time, 34 us so.
 __global__ void __launch_bounds__(kThreads) k_ragged_slice_counts(const uint8_t *__restrict__ codes,
                                                                   int64_t col_stride, int64_t M, int G,
                                                                   const int32_t *__restrict__ slice_lo,
                                                                   int32_t *__restrict__ cnt3)
 {
     const int64_t MG = M * (int64_t)G;
-    for (int64_t j = blockIdx.x; j < M; j += gridDim.x) {
-        const uint8_t *col = codes + j * col_stride;
-        for (int s = threadIdx.x; s < G; s += blockDim.x) {
-            const int lo = slice_lo[s], hi = slice_lo[s + 1];
-            int a = 0, b = 0, m = 0;
-            for (int i = lo; i < hi; ++i) {
-                const unsigned c = (col[i >> 2] >> (2 * (i & 3))) & 3u;
-                a += c == 2u;
-                b += c == 0u;
-                m += c == 1u;
-            }
-            const int64_t e = j * G + s;
-            cnt3[e] = a;
-            cnt3[MG + 1 + e] = b;
-            cnt3[2 * (MG + 1) + e] = m;
+    // M G fits 31 bits
+    for (unsigned e = blockIdx.x * kThreads + threadIdx.x; e < (unsigned)MG; e += gridDim.x * kThreads) {
+        const unsigned j = e / (unsigned)G, s = e - j * (unsigned)G;
+        const int lo = slice_lo[s], hi = slice_lo[s + 1];
+        const uint4 *col = reinterpret_cast<const uint4 *>(codes + (int64_t)j * col_stride + (lo >> 2));
+        CodeCounts c{0, 0, 0};
+        for (int i = lo; i < hi; i += 64) {
+            const uint4 w = __ldg(col++);
+            count_codes(w.x, code_mask(hi - i), c);
+            count_codes(w.y, code_mask(hi - i - 16), c);
+            count_codes(w.z, code_mask(hi - i - 32), c);
+            count_codes(w.w, code_mask(hi - i - 48), c);
         }
+        cnt3[e] = c.c1;
+        cnt3[MG + 1 + e] = c.c2;
+        cnt3[2 * (MG + 1) + e] = c.cm;
     }
 }
 
 // Fill slice-local indices in ascending order (src/raggedsparsemarkerbuilder.cpp:25-41
-// appends in decode order, i.e. ascending individual index).
+// appends in decode order, i.e. ascending individual index), from the set bits of the
+// genotypes that are not 0.  A warp takes 32 consecutive (marker, slice) pairs, whose
+// lists lie one behind the other: they are put together in shared memory and leave as
+// contiguous stores, because a store per entry costs a sector of the L2 each.  Pairs
+// with more entries than the buffer holds are stored one by one.  N = 20,011 x
+// M = 20,000 (80 M entries): 780 us an individual at a time, 544 us from the set
+// bits with a store per entry, 314 us this way.
+constexpr int kFillEntries = 4608;      // per warp
+
 __global__ void __launch_bounds__(kThreads) k_ragged_fill(const uint8_t *__restrict__ codes, int64_t col_stride,
                                                           int64_t M, int G, const int32_t *__restrict__ slice_lo,
                                                           const int32_t *__restrict__ off0,
@@ -186,32 +228,78 @@ __global__ void __launch_bounds__(kThreads) k_ragged_fill(const uint8_t *__restr
                                                           uint16_t *__restrict__ idx0, uint16_t *__restrict__ idx1,
                                                           uint16_t *__restrict__ idx2)
 {
-    for (int64_t j = blockIdx.x; j < M; j += gridDim.x) {
-        const uint8_t *col = codes + j * col_stride;
-        for (int s = threadIdx.x; s < G; s += blockDim.x) {
-            const int lo = slice_lo[s], hi = slice_lo[s + 1];
-            const int64_t e = j * G + s;
-            int32_t a = off0[e], b = off1[e], m = off2[e];
-            for (int i = lo; i < hi; ++i) {
-                const unsigned c = (col[i >> 2] >> (2 * (i & 3))) & 3u;
-                const uint16_t li = (uint16_t)(i - lo);
-                if (c == 2u)
-                    idx0[a++] = li;
-                else if (c == 0u)
-                    idx1[b++] = li;
-                else if (c == 1u)
-                    idx2[m++] = li;
+    extern __shared__ uint16_t s_fill[];
+    const unsigned MG = (unsigned)(M * (int64_t)G);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint16_t *const buf = s_fill + warp * kFillEntries;
+    const int32_t *const off[3] = {off0, off1, off2};
+    uint16_t *const idx[3] = {idx0, idx1, idx2};
+    const unsigned step = gridDim.x * kThreads;
+    for (unsigned e0 = blockIdx.x * kThreads + 32 * warp; e0 < MG; e0 += step) {
+        const unsigned e = e0 + lane < MG ? e0 + lane : MG, e1 = e0 + 32 < MG ? e0 + 32 : MG;
+        int32_t first[3], count[3];
+        uint16_t *at[3];
+        int32_t total = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            first[k] = off[k][e0];
+            count[k] = off[k][e1] - first[k];
+            total += count[k];
+        }
+        const bool staged = total <= kFillEntries;
+        uint16_t *seg = buf;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int32_t o = off[k][e];
+            at[k] = staged ? seg + (o - first[k]) : idx[k] + o;
+            seg += count[k];
+        }
+        if (e < MG) {
+            const unsigned j = e / (unsigned)G, s = e - j * (unsigned)G;
+            const int lo = slice_lo[s], n = slice_lo[s + 1] - lo;
+            const uint4 *col = reinterpret_cast<const uint4 *>(codes + (int64_t)j * col_stride + (lo >> 2));
+            for (int i = 0; i < n; i += 64) {
+                const uint4 v = __ldg(col++);
+                const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const unsigned in = code_mask(n - i - 16 * q) & 0x55555555u, l = w[q] & in, h = (w[q] >> 1) & in;
+                    for (unsigned r = in & ~(l & h); r; r &= r - 1u) {
+                        const int p = __ffs(r) - 1;
+                        const uint16_t li = (uint16_t)(i + 16 * q + (p >> 1));
+                        if ((h >> p) & 1u)
+                            *at[0]++ = li;
+                        else if ((l >> p) & 1u)
+                            *at[2]++ = li;
+                        else
+                            *at[1]++ = li;
+                    }
+                }
             }
+        }
+        if (staged) {
+            __syncwarp();
+            const uint16_t *src = buf;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                for (int32_t x = lane; x < count[k]; x += 32)
+                    idx[k][first[k] + x] = src[x];
+                src += count[k];
+            }
+            __syncwarp();
         }
     }
 }
 
-// Exclusive scan of int32 in three passes (tile scan, scan of tile sums in one
-// CTA, add).  Tiles of 1024 elements.
+// Exclusive scans of several int32 arrays of n elements one behind the other, in
+// three passes (tile scan, scan of tile sums in one CTA per array, add).  Tiles of
+// 1024 elements; tile_sums: as many words per array as there are tiles.
 constexpr int kScanTile = 1024;
 
 __global__ void __launch_bounds__(kThreads) k_scan_tiles(int32_t *data, int64_t n, int32_t *tile_sums)
 {
+    data += n * blockIdx.y;
+    tile_sums += (int64_t)gridDim.x * blockIdx.y;
     __shared__ int32_t sh[kScanTile];
     __shared__ int32_t wsum[kThreads / 32];
     const int64_t base = (int64_t)blockIdx.x * kScanTile;
@@ -253,29 +341,47 @@ __global__ void __launch_bounds__(kThreads) k_scan_tiles(int32_t *data, int64_t 
     }
 }
 
-__global__ void k_scan_sums(int32_t *tile_sums, int64_t ntiles)
+__global__ void __launch_bounds__(1024) k_scan_sums(int32_t *tile_sums, int64_t ntiles)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0)
-        return;
+    __shared__ int32_t wsum[32];
+    tile_sums += ntiles * blockIdx.x;
+    const int t = threadIdx.x, l = t & 31, w = t >> 5;
     int32_t run = 0;
-    for (int64_t q = 0; q < ntiles; ++q) {
-        const int32_t v = tile_sums[q];
-        tile_sums[q] = run;
-        run += v;
+    for (int64_t q0 = 0; q0 < ntiles; q0 += 1024) {
+        const int32_t v = q0 + t < ntiles ? tile_sums[q0 + t] : 0;
+        int32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (l >= o)
+                x += y;
+        }
+        if (l == 31)
+            wsum[w] = x;
+        __syncthreads();
+        int32_t pre = 0, all = 0;
+        for (int k = 0; k < 32; ++k) {
+            pre += k < w ? wsum[k] : 0;
+            all += wsum[k];
+        }
+        if (q0 + t < ntiles)
+            tile_sums[q0 + t] = run + pre + x - v;
+        run += all;
+        __syncthreads();
     }
 }
 
-__global__ void k_scan_add(int32_t *data, int64_t n, const int32_t *tile_sums)
+__global__ void k_scan_add(int32_t *data, int64_t n, const int32_t *tile_sums, int64_t ntiles)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
-        data[i] += tile_sums[i / kScanTile];
+        data[n * blockIdx.y + i] += tile_sums[ntiles * blockIdx.y + i / kScanTile];
 }
 
 cudaError_t launch_pack_counts(const uint8_t *bed, int64_t N, int64_t M, uint8_t *codes, int64_t col_stride,
                                int64_t *counts, cudaStream_t st)
 {
-    const int blocks = (int)imin64(M, 152 * 16);
+    const int blocks = (int)imin64((M + 7) / 8, 152 * 8);
     k_pack_counts<<<blocks, kThreads, 0, st>>>(bed, N, M, codes, col_stride, counts);
     return cudaGetLastError();
 }
@@ -297,17 +403,29 @@ cudaError_t launch_ragged_stats(const int64_t *counts, int64_t N, int64_t M, int
 cudaError_t launch_ragged_slice_counts(const uint8_t *codes, int64_t col_stride, int64_t M, int G,
                                        const int32_t *slice_lo, int32_t *cnt3, cudaStream_t st)
 {
-    const int blocks = (int)imin64(M, 152 * 16);
+    const int blocks = (int)imin64((M * G + kThreads - 1) / kThreads, 152 * 32);
     k_ragged_slice_counts<<<blocks, kThreads, 0, st>>>(codes, col_stride, M, G, slice_lo, cnt3);
     return cudaGetLastError();
 }
 
-cudaError_t launch_exclusive_scan_i32(int32_t *data, int64_t n, int32_t *tmp, cudaStream_t st)
+cudaError_t launch_count_totals(const int64_t *counts, int64_t M, unsigned long long *tot, cudaStream_t st)
 {
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    k_scan_tiles<<<(unsigned)ntiles, kThreads, 0, st>>>(data, n, tmp);
-    k_scan_sums<<<1, 32, 0, st>>>(tmp, ntiles);
-    k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(data, n, tmp);
+    const cudaError_t e = cudaMemsetAsync(tot, 0, 3 * sizeof *tot, st);
+    if (e != cudaSuccess)
+        return e;
+    k_count_totals<<<(unsigned)imin64((M + kThreads - 1) / kThreads, 152), kThreads, 0, st>>>(counts, M, tot);
+    return cudaGetLastError();
+}
+
+int64_t scan_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
+
+cudaError_t launch_exclusive_scans_i32(int32_t *data, int64_t n, int arrays, int32_t *tmp, cudaStream_t st)
+{
+    const int64_t ntiles = scan_tiles(n);
+    const unsigned y = (unsigned)arrays;
+    k_scan_tiles<<<dim3((unsigned)ntiles, y), kThreads, 0, st>>>(data, n, tmp);
+    k_scan_sums<<<y, 1024, 0, st>>>(tmp, ntiles);
+    k_scan_add<<<dim3((unsigned)((n + 255) / 256), y), 256, 0, st>>>(data, n, tmp, ntiles);
     return cudaGetLastError();
 }
 
@@ -315,9 +433,12 @@ cudaError_t launch_ragged_fill(const uint8_t *codes, int64_t col_stride, int64_t
                                const int32_t *off0, const int32_t *off1, const int32_t *off2, uint16_t *idx0,
                                uint16_t *idx1, uint16_t *idx2, cudaStream_t st)
 {
-    const int blocks = (int)imin64(M, 152 * 16);
-    k_ragged_fill<<<blocks, kThreads, 0, st>>>(codes, col_stride, M, G, slice_lo, off0, off1, off2, idx0, idx1,
-                                               idx2);
+    const int blocks = (int)imin64((M * G + kThreads - 1) / kThreads, 152 * 32);
+    const int smem = kThreads / 32 * kFillEntries * (int)sizeof(uint16_t);
+    const cudaError_t e = cudaFuncSetAttribute((const void *)k_ragged_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess)
+        return e;
+    k_ragged_fill<<<blocks, kThreads, smem, st>>>(codes, col_stride, M, G, slice_lo, off0, off1, off2, idx0, idx1, idx2);
     return cudaGetLastError();
 }
 

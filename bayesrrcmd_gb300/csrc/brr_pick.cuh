@@ -321,10 +321,11 @@ __device__ __forceinline__ float certain_zero(float uf, const double *gc, int K)
 
 // Component of one marker at num^2 = x by a whole warp, one mixture component per
 // lane: the certified decision of pick_margin without its margin; -2 where it cannot
-// certify.  f: the FP32 constants {dc_k, h_k} of the group's component k = lane.  About 40 instructions against
+// certify.  f: the FP32 constants {dc_k, h_k} of the group's component k = lane; more: an
+// error of num^2 beyond its rounding, in units of 4e-7.  About 40 instructions against
 // 150, which matters where the decision lies on a sweep's chain.
 template <int KM>
-__device__ __forceinline__ int pick_lanes(int lane, float x, float uf, float2 f, int K)
+__device__ __forceinline__ int pick_lanes(int lane, float x, float uf, float2 f, int K, float more = 0.f)
 {
     const bool in = lane < K;
     const float hx = f.y * x;
@@ -333,7 +334,7 @@ __device__ __forceinline__ int pick_lanes(int lane, float x, float uf, float2 f,
     // error of D (six roundings)
     const float dmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(D, 0.f))));
     const float mag =
-        __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(in ? fabsf(f.x) + fabsf(hx) : 0.f)));
+        __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(in ? fabsf(f.x) + fabsf(f.y) * (x + more) : 0.f)));
     float c = in ? __expf(D - dmax) : 0.f;
 #pragma unroll
     for (int o = 1; o < KM; o <<= 1) {

@@ -150,6 +150,19 @@ __device__ __forceinline__ void split_double(double v, float &h, float &l)
     l = __uint2float_rn((unsigned)b & 0x1FFFFFFFu) * __uint_as_float(sign | ((unsigned)(e - 948) << 23));
 }
 
+// v as the FP32 value next to it towards zero, by integer operations (an FP64
+// instruction takes 64 clocks); below 2^-126 zero.
+__device__ __forceinline__ float double_hi(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned top = (unsigned)(b >> 32);
+    return (top & 0x7FF00000u) < (897u << 20)
+               ? 0.f
+               : __uint_as_float((top & 0x80000000u) | (((unsigned)(b >> 29) + 0x40000000u) & 0x7FFFFFFFu));
+}
+
+__device__ __forceinline__ bool nonzero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) != 0ull; }
+
 // A decision the margin sampler cannot certify: the guarded FP32 sampler, else
 // FP64.  Out of line: about one marker in a thousand.
 template <int KM>
@@ -176,6 +189,8 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     __shared__ volatile int s_ev2[kMaxSpec + 1];  // the FP64 warp's progress over them
     __shared__ double s_Td;               // dense: the residual total
     __shared__ float2 s_Tf;               // the residual total or the running sum as a float pair
+    __shared__ volatile int s_ask;        // the chain's question to the FP64 warp: events before it << 8, marker + 1
+    __shared__ volatile double s_told;    // and its answer: the marker's num
     __shared__ volatile int s_ev[kMaxSpec + 1];   // changes of the round in order, for the FP64 warp
     __shared__ double s_dB[kMaxSpec];
     __shared__ int s_ci[kMaxSpec];
@@ -305,6 +320,8 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     }
     for (int i = tid; i <= kMaxSpec; i += kRT)
         s_ev[i] = s_ev2[i] = 0;
+    if (tid == 0)
+        s_ask = 0;
     if (!CL)
         for (int i = tid; i < 2 * kRoundAccStride; i += kRT)
             reinterpret_cast<unsigned long long *>(smem + plan.prev)[i] = 0ull;
@@ -691,12 +708,13 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                         break;
                     const RoundRec &rp = rec[(start + ((ev - 1) & 63)) & Rm];
                     // (genotype - mean) scale; missing genotypes apart
-                    const double x = lane == 1 ? (dense ? rp.x : 0.0)
-                                               : __dmul_rn(__dsub_rn(lane == 0 ? 2.0 : lane == 2 ? 1.0 : 0.0, rp.m), rp.s);
+                    const double x = up * (lane == 1 ? (dense ? rp.x : 0.0)
+                                                     : __dmul_rn(__dsub_rn(lane == 0 ? 2.0 : lane == 2 ? 1.0 : 0.0, rp.m), rp.s));
                     wait_event(&s_ev2[u]);
                     if (lane < 4) {
-                        const double d = __dmul_rn(s_dB[u], x) * up;
-                        const bool ok = fabs(d) < 4.6e18;
+                        const double d = __dmul_rn(s_dB[u], x);   // up is a power of two
+                        // |d| < 2^62, by its exponent
+                        const bool ok = ((unsigned)__double2hiint(d) & 0x7FF00000u) < (1085u << 20);
                         range = range || !ok;
                         s_d[u][lane] = ok ? __double2ll_rn(d) : 0ll;
                     }
@@ -705,16 +723,21 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
         } else if (warp == 0) {
             // lane t holds markers t and 32 + t.  The loop below runs once per marker that
             // may change, on one warp, from instructions that the other phases have
-            // pushed out of the nearest instruction cache: its length is its cost.
-            float s0[2], boh[2], bol[2], zh[2], zl[2];
+            // pushed out of the nearest instruction cache: its length is its cost.  It only
+            // decides: num is carried in FP32 with a bound er on its error, which widens
+            // the certificates of the decisions; where they fail, the FP64 warp is
+            // asked for the marker's num.  (With num as a pair of FP32 words a change took
+            // 1.17k clk, so 0.97k; dense 2,000 x 5,000 in the burn-in, 27 changes a round: 1.63
+            // and 1.46 ms per sweep.)
+            float s0[2], bo[2], zf[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int t = lane + 32 * h;
                 const RoundRec &rc = rec[(start + (t < nb ? t : 0)) & Rm];
                 // num^2 above which the marker may change: always with an old effect
-                s0[h] = !(t < nb) ? INFINITY : rc.beta_old != 0.0 ? -1.f : rc.s0;
-                split_double(rc.beta_old, boh[h], bol[h]);
-                split_double(rc.z, zh[h], zl[h]);
+                bo[h] = double_hi(rc.beta_old);
+                zf[h] = double_hi(rc.z);
+                s0[h] = !(t < nb) ? INFINITY : nonzero(rc.beta_old) ? -1.f : rc.s0;
                 s_comp[t] = 0;
             }
             const double *gr = reinterpret_cast<const double *>(smem + plan.gram + (blk & 1u) * gslot);
@@ -724,21 +747,14 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             asm volatile("bar.sync 1, 96;" ::: "memory");
             mark(2);
             wstart();
-            float nh[2], nl[2], sx[2];
+            float x[2], er[2], sx[2];   // num, its error, the square of its largest magnitude
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float2 v = s_ndf[lane + 32 * h];
-                nh[h] = v.x;
-                nl[h] = v.y;
-                sx[h] = num_sq(v.x, v.y);
+                x[h] = v.x;
+                er[h] = __fmaf_rn(1e-10f, fabsf(v.x), 1.01f * fabsf(v.y));
+                sx[h] = (fabsf(x[h]) + er[h]) * (fabsf(x[h]) + er[h]);
             }
-            // The component of marker p (half h, this lane's) the guarded samplers choose.
-            auto slow = [&](int h, int p) {
-                const RoundRec &rc = rec[(start + p) & Rm];
-                const int g = (int)(rc.gm & 255u);
-                return decide_slow<KM>(h ? nh[1] : nh[0], h ? nl[1] : nl[0], a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
-                                       gcf + (size_t)g * kMaxK * 2, gk[g]);
-            };
             // A marker may change when its old effect is not zero or num^2 is not in
             // the range where component 0 is certain (s0; P(component 0) falls as
             // num^2 grows).  Only such a marker's component is worked out, when the
@@ -751,8 +767,12 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     const int t = lane + 32 * h;
                     int comp = 0;
                     const bool c = (h ? sx[1] : sx[0]) > (h ? s0[1] : s0[0]) && t < nb;
-                    if (c)
-                        comp = slow(h, t);
+                    if (c) {
+                        const RoundRec &rc = rec[(start + t) & Rm];
+                        const int g = (int)(rc.gm & 255u);
+                        comp = decide_slow<KM>(s_ndf[t].x, s_ndf[t].y, a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
+                                               gcf + (size_t)g * kMaxK * 2, gk[g]);
+                    }
                     __syncwarp();
                     const bool b = c && (comp > 0 || rec[(start + t) & Rm].beta_old != 0.0);
                     const unsigned kb = __ballot_sync(0xffffffffu, b);
@@ -786,17 +806,31 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                         gv1 = row[lane + 32];
                 }
                 const RoundRec &rc = rec[(start + p) & Rm];
-                const float ph = hi ? nh[1] : nh[0], pl = hi ? nl[1] : nl[0];
-                int comp = pick_lanes<KM>(lane, __shfl_sync(0xffffffffu, hi ? sx[1] : sx[0], p & 31), rc.uf,
-                                          gcf + (size_t)(rc.gm & 255u) * kMaxK * 2, gk[rc.gm & 255u]);
+                const unsigned g = rc.gm & 255u;
+                const float xp = hi ? x[1] : x[0], ep = hi ? er[1] : er[0];
+                const float px = __shfl_sync(0xffffffffu, xp, p & 31), pe = __shfl_sync(0xffffffffu, ep, p & 31);
+                // D_k moves by 2 h_k |num| er: 5e6 = 2 / 4e-7, in units of the samplers' own error
+                int comp = pick_lanes<KM>(lane, px * px, rc.uf,
+                                          reinterpret_cast<const float2 *>(gcf + (size_t)g * kMaxK * 2)[lane & (kMaxK - 1)],
+                                          gk[g], 5e6f * pe * (fabsf(px) + pe));
                 if (comp == -2) {
-                    if (own)
-                        comp = slow(hi, p);
+                    if (own) {
+                        s_ask = (nchg << 8) | (p + 1);
+                        unsigned spins = 0;
+                        while (s_ask != 0 && ++spins < (1u << 28))
+                            ;
+                        if (s_ask != 0)
+                            atomicCAS(a.err, kDevOk, kDevTimeout);
+                        float nh, nl;
+                        df_from_double(s_told, nh, nl);
+                        comp = decide_slow<KM>(nh, nl, a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
+                                               gcf + (size_t)g * kMaxK * 2, gk[g]);
+                    }
                     comp = __shfl_sync(0xffffffffu, comp, p & 31);
                 }
                 if (own)
                     s_comp[p] = comp;
-                if (comp <= 0 && rc.beta_old == 0.0)
+                if (comp <= 0 && !nonzero(rc.beta_old))
                     continue;
                 if (own)
                     s_ev[nchg] = 1 + p + ((comp + 1) << 8);
@@ -805,30 +839,28 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     fin = p + 1;   // a restart round ends at its first change, a pair round at one without a row
                     break;
                 }
-                // beta_old - beta_new in double-float, on the owner's lane
-                float bh = hi ? boh[1] : boh[0], bl = hi ? bol[1] : bol[0];
+                // beta_old - beta_new and its error, on the owner's lane
+                float d = hi ? bo[1] : bo[0], e = fabsf(d);
                 if (comp > 0) {
-                    const float4 k4 = gdf[(rc.gm & 255u) * kMaxK + comp];
-                    float ah, al, xh, xl;
-                    df_mul(hi ? zh[1] : zh[0], hi ? zl[1] : zl[0], k4.x, k4.y, ah, al);
-                    df_mul(ph, pl, k4.z, k4.w, xh, xl);
-                    df_add(ah, al, xh, xl);
-                    df_add(bh, bl, -ah, -al);
-                } else if (comp < 0) {
-                    bh = bl = 0.f;
+                    const float4 k4 = gdf[g * kMaxK + comp];   // {sdk hi, lo, invden hi, lo}
+                    const float zs = (hi ? zf[1] : zf[0]) * k4.x, xi = xp * k4.z;
+                    d -= zs + xi;
+                    e = __fmaf_rn(ep, k4.z, 5e-7f * (e + fabsf(zs) + fabsf(xi)));
+                } else {
+                    e *= 3e-7f;
+                    if (comp < 0)
+                        d = e = 0.f;
                 }
-                bh = __shfl_sync(0xffffffffu, bh, p & 31);
-                bl = __shfl_sync(0xffffffffu, bl, p & 31);
-                // the later markers' num
-                float vh, vl, ch, cl;
-                split_double(gv0, vh, vl);
-                df_mul(bh, bl, vh, vl, ch, cl);
-                df_add(nh[0], nl[0], ch, cl);
-                sx[0] = num_sq(nh[0], nl[0]);
-                split_double(gv1, vh, vl);
-                df_mul(bh, bl, vh, vl, ch, cl);
-                df_add(nh[1], nl[1], ch, cl);
-                sx[1] = num_sq(nh[1], nl[1]);
+                d = __shfl_sync(0xffffffffu, d, p & 31);
+                e = __shfl_sync(0xffffffffu, e, p & 31);
+                // the later markers' num; 7e-8 |num|: its rounding
+                const float g0 = double_hi(gv0), g1 = double_hi(gv1);
+                x[0] = __fmaf_rn(d, g0, x[0]);
+                x[1] = __fmaf_rn(d, g1, x[1]);
+                er[0] = __fmaf_rn(7e-8f, fabsf(x[0]), __fmaf_rn(e, fabsf(g0), er[0]));
+                er[1] = __fmaf_rn(7e-8f, fabsf(x[1]), __fmaf_rn(e, fabsf(g1), er[1]));
+                sx[0] = (fabsf(x[0]) + er[0]) * (fabsf(x[0]) + er[0]);
+                sx[1] = (fabsf(x[1]) + er[1]) * (fabsf(x[1]) + er[1]);
             }
             __syncwarp();
             if (lane == 0) {
@@ -856,7 +888,18 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             __syncwarp();
             int nchg = 0;
             for (;; ++nchg) {
-                const int ev = wait_event(&s_ev[nchg]);
+                int ev;
+                unsigned spins = 0;
+                while ((ev = s_ev[nchg]) == 0 && ++spins < (1u << 28)) {
+                    const int ask = s_ask;
+                    if (ask != 0 && ((ask - 1) & 31) == lane && ask >> 8 == nchg) {
+                        s_told = ((ask - 1) & 32) ? num[1] : num[0];
+                        __threadfence_block();
+                        s_ask = 0;
+                    }
+                }
+                if (ev == 0)
+                    atomicCAS(a.err, kDevOk, kDevTimeout);
                 if (ev <= 0)
                     break;
                 const int p = (ev - 1) & 63, comp = (ev - 1) / 256 - 1;
@@ -883,9 +926,9 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 if (!here && !a.rall)
                     continue;   // the round ends here
                 const double *row = (here ? gr : grow) + q * (2 * B - q - 1) / 2 - p - 1;
-                if (lane > p && lane < nb)
+                if (p < 31 && lane > p && lane < nb)
                     num[0] = fma(dB, row[lane], num[0]);
-                if (lane + 32 > p && lane + 32 < nb)
+                if (nb > 32 && lane + 32 > p && lane + 32 < nb)
                     num[1] = fma(dB, row[lane + 32], num[1]);
             }
             if (lane < nb)

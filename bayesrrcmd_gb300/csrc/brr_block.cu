@@ -136,6 +136,53 @@ __host__ __device__ inline size_t block_gram_entries(int B) { return (size_t)B *
 // previous one.
 __host__ __device__ inline size_t block_stage_entries(int B) { return block_gram_entries(B) + (size_t)B * B; }
 
+// Staged Gram entry e of block q from the packed Gram; ids: the ring of the blocks'
+// marker ids.  False where the block has no such entry.
+__device__ __forceinline__ bool gram_entry_of(const float2 *__restrict__ gram, const uint32_t *ids, unsigned q, unsigned Bu,
+                                              int lB, int nbq, unsigned npairs, unsigned e, float2 *out)
+{
+    const unsigned q0 = q * Bu;
+    unsigned pa, pb, qa;
+    if (e < npairs) {
+        // e = pb (pb - 1) / 2 + pa with pa < pb
+        pb = (unsigned)((1.f + __fsqrt_rn(8.f * (float)e + 1.f)) * 0.5f);
+        if (pb * (pb - 1u) / 2u > e)
+            --pb;
+        pa = e - pb * (pb - 1u) / 2u;
+        if ((int)pb >= nbq)
+            return false;
+        qa = q0 + pa;
+    } else {
+        // near (block q-1) or far (block q-2) entries; those blocks are full
+        const unsigned c = e - npairs;
+        const unsigned back = 1u + (c >> (2 * lB));
+        if (q < back)
+            return false;
+        pa = (c >> lB) & (Bu - 1u);
+        pb = c & (Bu - 1u);
+        if ((int)pb >= nbq)
+            return false;
+        qa = q0 - back * Bu + pa;
+    }
+    const int64_t ja = ids[((qa >> lB) % kIdSlots) * kMaxSpec + (qa & (Bu - 1u))], jb = ids[(q % kIdSlots) * kMaxSpec + pb];
+    const int64_t hi = ja > jb ? ja : jb, lw = ja > jb ? jb : ja;
+    *out = __ldg(&gram[hi * (hi - 1) / 2 + lw]);
+    return true;
+}
+
+// Entries e, e + step, ... of block q into its staging slot.  Out of line: the large
+// grids never come here.
+__device__ __noinline__ void gather_rest_of(const float2 *__restrict__ gram, const uint32_t *ids, float2 *slot, unsigned q,
+                                            unsigned Bu, int lB, int nbq, unsigned npairs, unsigned gst, unsigned e,
+                                            unsigned step)
+{
+    for (; e < gst; e += step) {
+        float2 v;
+        if (gram_entry_of(gram, ids, q, Bu, lB, nbq, npairs, e, &v))
+            slot[e] = v;
+    }
+}
+
 struct PipePlan {
     size_t planes;          // residual limb planes (FP16)
     size_t fix;             // residual in fixed point: one int64 per individual, in the planes' order
@@ -618,40 +665,15 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
     // e = s + G*(l + 32*i) from the packed Gram into staging slot q % 8.  The
     // first kGather entries of each thread are loaded one iteration before they
     // are stored, so that the random reads of the Gram never delay the
-    // signal before the barrier arrival (more than kGather entries per lane, on
-    // grids below 80 CTAs, are loaded when stored).
+    // signal before the barrier arrival.  What grids below 80 CTAs leave, the dot
+    // warps gather, a thread an entry (slices of few individuals keep them
+    // waiting): on the chore warp alone, 32 CTAs (2,000 individuals) spent 14.1k clk
+    // of an iteration, 5.9k now (0.63 and 0.31 ms per sweep of 5,000 markers).
     constexpr int kGather = 4;
     float2 gval[kGather];
     int gent_mine[kGather] = {-1, -1, -1, -1};
     auto gram_entry = [&](int q, unsigned e, float2 *out) -> bool {
-        const unsigned q0 = (unsigned)q * Bu;
-        const int nbq = nb_of(q);
-        unsigned pa, pb, qa;
-        if (e < (unsigned)npairs) {
-            // e = pb (pb - 1) / 2 + pa with pa < pb
-            pb = (unsigned)((1.f + __fsqrt_rn(8.f * (float)e + 1.f)) * 0.5f);
-            if (pb * (pb - 1u) / 2u > e)
-                --pb;
-            pa = e - pb * (pb - 1u) / 2u;
-            if ((int)pb >= nbq)
-                return false;
-            qa = q0 + pa;
-        } else {
-            // near (block q-1) or far (block q-2) entries; those blocks are full
-            const unsigned c = e - (unsigned)npairs;
-            const unsigned back = 1u + (c >> (2 * lB));
-            if ((unsigned)q < back)
-                return false;
-            pa = (c >> lB) & (Bu - 1u);
-            pb = c & (Bu - 1u);
-            if ((int)pb >= nbq)
-                return false;
-            qa = q0 - back * Bu + pa;
-        }
-        const int64_t ja = s_ids[(qa >> lB) % kIdSlots][qa & (Bu - 1u)], jb = s_ids[q % kIdSlots][pb];
-        const int64_t hi = ja > jb ? ja : jb, lw = ja > jb ? jb : ja;
-        *out = __ldg(&a.gram[hi * (hi - 1) / 2 + lw]);
-        return true;
+        return gram_entry_of(a.gram, &s_ids[0][0], (unsigned)q, Bu, lB, nb_of(q), (unsigned)npairs, e, out);
     };
     auto gather_load = [&](int q) {
 #pragma unroll
@@ -668,12 +690,12 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
         for (int k = 0; k < kGather; ++k)
             if (gent_mine[k] >= 0)
                 slot[gent_mine[k]] = gval[k];
-        for (unsigned e = (unsigned)sidx + (unsigned)(lane + 32 * kGather) * (unsigned)a.G; e < gst;
-             e += 32u * (unsigned)a.G) {
-            float2 v;
-            if (gram_entry(q, e, &v))
-                slot[e] = v;
-        }
+    };
+    const bool gather_rest = gst > 32u * kGather * (unsigned)a.G;
+    auto rest = [&](int q) {
+        gather_rest_of(a.gram, &s_ids[0][0], gstage + (size_t)(q % kStageSlots) * gst, (unsigned)q, Bu, lB, nb_of(q),
+                       (unsigned)npairs, gst, (unsigned)sidx + (unsigned)(32 * kGather + dtid) * (unsigned)a.G,
+                       (unsigned)(32 * kDotWarps) * (unsigned)a.G);
     };
 
     // ---- partial dot products of block q against the current residual (dot
@@ -962,6 +984,8 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
     cp_async_wait_all();
     __syncthreads();
     if (dw >= 0) {
+        for (int q = 0; q < 3 && q < nblk && gather_rest; ++q)
+            rest(q);
         dot_block(0);
         dot_warps_sync();
         if (nblk > 1)
@@ -1280,6 +1304,8 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
                 // ---- dot side: update of block r-1, the code slices of block r+3
                 // into the slot block r-1 held, dots of block r+2 and their
                 // publication
+                if (gather_rest && r + 3 < nblk)
+                    rest(r + 3);
                 if (r >= 1)
                     apply_update(r - 1);
                 mbar_arrive(&s_mb[(r + 1) & 1]);   // GO(r+1): block r-1's decisions applied

@@ -804,37 +804,45 @@ __global__ void __launch_bounds__(kBT, 1) k_sweep_batch(BatchArgs a)
     __syncthreads();
     tc_fence_after();
 
-    // ---- residuals back to HBM; per-slice sum(E) and sum(eps^2) per chain, a warp per pair of chains
+    // ---- residuals back to HBM; per-slice sum(E) and sum(eps^2) per chain, a warp per pair of chains.
+    // The squares are summed in the order that does not depend on who sums: eight
+    // groups of 32 individuals apart by 256, a butterfly per group, the groups in turn.
     for (int cp = warp; cp < C / 2; cp += kBW) {
         long long se[2] = {0, 0};
-        double sq[2] = {0.0, 0.0};
-        for (int i = lane; i < ns; i += 32) {
-            const uint4 w4 = *reinterpret_cast<const uint4 *>(e_t + (i >> 3) * pl.lbo_e + cp * 128 + (i & 7) * 16);
-            const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+        double total[2] = {0.0, 0.0};
+        for (int g = 0; g < 8; ++g) {
+            double sq[2] = {0.0, 0.0};
+            for (int i = 32 * g + lane; i < ns; i += 256) {
+                const uint4 w4 = *reinterpret_cast<const uint4 *>(e_t + (i >> 3) * pl.lbo_e + cp * 128 + (i & 7) * 16);
+                const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    int d[kBatchLimbs];
+#pragma unroll
+                    for (int l = 0; l < kBatchLimbs; ++l)
+                        d[l] = h_int((unsigned short)(w[2 * h + (l >> 1)] >> (16 * (l & 1))));
+                    const long long x = join4(d);
+                    a.E[(size_t)(2 * cp + h) * a.N + lo + i] = x;
+                    se[h] += x;
+                    const double e = (double)x * inv2f;
+                    sq[h] = fma(e, e, sq[h]);
+                }
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                int d[kBatchLimbs];
 #pragma unroll
-                for (int l = 0; l < kBatchLimbs; ++l)
-                    d[l] = h_int((unsigned short)(w[2 * h + (l >> 1)] >> (16 * (l & 1))));
-                const long long x = join4(d);
-                a.E[(size_t)(2 * cp + h) * a.N + lo + i] = x;
-                se[h] += x;
-                const double e = (double)x * inv2f;
-                sq[h] = fma(e, e, sq[h]);
+                for (int o = 16; o > 0; o >>= 1)
+                    sq[h] += __shfl_xor_sync(0xffffffffu, sq[h], o);
+                total[h] += sq[h];
             }
         }
-        // fixed-order reduction over the lanes
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             se[h] = warp_sum(se[h]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                sq[h] += __shfl_xor_sync(0xffffffffu, sq[h], o);
             if (lane == 0) {
                 double *pp = a.part + ((size_t)s * C + 2 * cp + h) * 2;
                 pp[0] = __longlong_as_double(se[h]);
-                pp[1] = sq[h];
+                pp[1] = total[h];
             }
         }
     }

@@ -27,15 +27,6 @@ __device__ __forceinline__ void cl_push16(unsigned raddr, unsigned long long w0,
                  : "memory");
 }
 
-// Bulk copy of shared memory (16-byte aligned, a multiple of 16 bytes) into another
-// CTA's, completing as that many transaction bytes on that CTA's mbarrier.
-__device__ __forceinline__ void cl_copy(unsigned rdst, unsigned src, unsigned bytes, unsigned rbar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(rdst),
-                 "r"(src), "r"(bytes), "r"(rbar)
-                 : "memory");
-}
-
 __device__ __forceinline__ void cl_bar_init(uint64_t *m)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_addr(m)) : "memory");

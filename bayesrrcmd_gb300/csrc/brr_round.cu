@@ -33,15 +33,15 @@
 // limb columns x one slice, far below a tcgen05 tile, and its operands are
 // decoded in registers straight from the 2-bit codes.
 //
-// Exchange: the partial sums of a round as two 64-bit integers per marker,
-// added in L2 with one grid-wide counter barrier per round, or stored into the
-// other CTAs' shared memory of one thread-block cluster (k_round_cl).
+// Exchange: the partial sums of a round as two 64-bit integers per marker, added
+// in L2 with the count of arrivals in their top byte (no barrier), or stored into
+// the other CTAs' shared memory of one thread-block cluster (k_round_cl).
 //
-// Sampling: one warp, marker t on lane t mod 32, identically in every CTA.  The
-// component is decided by the certified FP32 samplers of brr_pick.cuh with
-// their stability margins (FP64 where they cannot certify); num, beta and the
-// corrections are FP64.  P(component 0) is left to k_round_finish, one thread
-// per marker over the whole GPU, from the stored num.
+// Sampling: one warp walks the chain, markers t and 32 + t on lane t, identically
+// in every CTA, and only decides components, by the certified FP32 samplers of
+// brr_pick.cuh (FP64 where they cannot certify); num, beta and the corrections
+// are FP64, on a warp that follows it.  P(component 0) is left to k_round_finish,
+// one thread per marker over the whole GPU, from the stored num.
 #include "brr_cluster.cuh"
 #include "brr_device.cuh"
 #include "brr_internal.h"

@@ -291,10 +291,11 @@ def run_batched(lib, gpu, torch, device, steps, warmup):
     torch.cuda.empty_cache()
     nblocks = (B_M + 31) // 32
     # algorithmic tensor work per block: X_block^T E and X_block dB (2 * 32 * C * N
-    # each) plus the block Gram (32 * 32 * N); the kernel computes the residual
-    # as four 11-bit limbs, i.e. four times the dot and update products
-    alg_flop = nblocks * (2 * 2 * 32 * B_C * B_N + 2 * 32 * 32 * B_N)
-    issued_flop = nblocks * (2 * 2 * 32 * 4 * B_C * B_N + 2 * 128 * 32 * B_N)
+    # each) plus its Gram with itself and the block before (32 * 64 * N); the kernel
+    # computes the residual as four 11-bit limbs, i.e. four times the dot and update
+    # products, and the Gram in overlapping squares of 64 markers
+    alg_flop = nblocks * (2 * 2 * 32 * B_C * B_N + 2 * 32 * 64 * B_N)
+    issued_flop = nblocks * (2 * 2 * 32 * 4 * B_C * B_N + 2 * 64 * 64 * B_N)
     sweep_s = b_sweep / 1e3 / steps
     rate = B_C * B_M * steps / (b_total / 1e3)
     plain = B_M * p_steps / (p_total / 1e3)
@@ -527,7 +528,7 @@ def run_ragged(lib, gpu, torch, device, steps, warmup, cpu=True):
         "plain_fp64": {"value": f64["rate"], "ms_per_step": f64["ms_per_step"], "rounds_per_step": f64["rounds"]},
         "speedup_fp32c_vs_plain": f32["rate"] / f64["rate"],
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     "traffic": None, "kernel": "k_sweep_pr (ragged, FP32C, pair-resolved rounds)",
+                     "traffic": None, "kernel": "k_round (ragged, FP32C, pair-resolved rounds)",
                      "algorithmic_bytes_per_launch": idx_bytes,
                      "note": "4 bytes per listed genotype (ones, twos, missing) per sweep"},
         "matched_error": {"beta_max_abs_diff_vs_plain": float(np.abs(f32["beta"] - f64["beta"]).max()),

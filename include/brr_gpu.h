@@ -118,8 +118,8 @@ typedef struct brr_config {
                                   (src/parallelgraph.cpp:51-150): the T markers of a batch all read
                                   the residual before any of them updates it, acum is not written
                                   (src/BayesRBase.cpp:394-524); FP64 form only */
-    int32_t cluster;           /* 0: the restart sweep exchanges its partial sums through L2 across `grid`
-                                  CTAs with a grid-wide barrier; C in 2..16: the restart sweep runs as
+    int32_t cluster;           /* 0: the whole-round sweep exchanges its partial sums through L2 across
+                                  `grid` CTAs; C in 2..16: the whole-round sweep runs as
                                   one thread-block cluster of C CTAs, each holding its slice of the
                                   residual in shared memory and storing its partial sums into every
                                   CTA's shared memory (no Gram-blocked form; gram must not be 1) */
@@ -341,7 +341,11 @@ int brr_multi_get_timing(brr_multi *m, double *sweep_ms, double *total_ms, int32
 
 /* Per-phase SM cycles of the sweeps of the last brr_iterate / brr_sweep call,
  * measured on the first CTA (the counterpart of the reference's per-column
- * timing log, src/BayesRBase.cpp:381-389), 16 values.  Restart sweep: [0] ring
+ * timing log, src/BayesRBase.cpp:381-389), 16 values.  Whole-round sweep: [0]
+ * records and codes, [1] partial dot products and publication, [2] [3]
+ * exchange and resolve, [4] outputs and residual update, [5] rounds; on their own
+ * warps [6] before the wait, [7] the wait for the sums, [8] num, [10] the chain, [11]
+ * the FP64 warp behind it, [13] prefetching; [14] changes.  Restart sweep: [0] ring
  * prefetch and wait, [1] partial dot products, [2] grid barrier, [3]
  * component sampling, [4] outputs and residual update, [5] grid rounds.
  * Gram-blocked sweep: [0] ring wait and waiting for the other warps, [1] dot
@@ -352,7 +356,7 @@ int brr_multi_get_timing(brr_multi *m, double *sweep_ms, double *total_ms, int32
  * [3] in component picks, [10] cycles of [3] resolving steps, [11] assembling
  * the next block's inputs, [12]-[15] cycles from each iteration's start to the
  * end of the work of the dot warps, the Gram warp, the sampling warp and the
- * input warp.  The
+ * input warp (small grids' dot warps gather Gram entries too).  The
  * per-thread clock is read around long code regions, so the values are
  * indicative. */
 int brr_get_phase_cycles(brr_ctx *ctx, int64_t *cycles);

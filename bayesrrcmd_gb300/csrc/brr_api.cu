@@ -186,6 +186,8 @@ void free_all(brr_ctx *c)
     cudaFree(c->d_psum);
     cudaFree(c->d_rgram);
     cudaFree(c->d_num);
+    cudaFree(c->d_beta2);
+    cudaFree(c->d_comp2);
     cudaFree(c->d_emax);
     cudaFree(c->d_pstat);
     cudaFree(c->d_eps2);
@@ -383,6 +385,7 @@ int prepare_round(brr_ctx *c)
     const brr_config &cf = c->cfg;
     const size_t N = (size_t)cf.N, M = (size_t)cf.M;
     if (!c->d_rrec && (dalloc(&c->d_rrec, M) != cudaSuccess || dalloc(&c->d_rnz, (M + 255) / 256 * 8 + 2) != cudaSuccess || dalloc(&c->d_num, M) != cudaSuccess ||
+                       dalloc(&c->d_beta2, M) != cudaSuccess || dalloc(&c->d_comp2, M) != cudaSuccess ||
                        (cf.form == BRR_FORM_FP64
                             ? dalloc(&c->d_eps2, N) != cudaSuccess
                             : dalloc(&c->d_eps_hi2, N) != cudaSuccess || dalloc(&c->d_eps_lo2, N) != cudaSuccess))) {
@@ -390,6 +393,8 @@ int prepare_round(brr_ctx *c)
         drop_dev(c->d_rrec);
         drop_dev(c->d_rnz);
         drop_dev(c->d_num);
+        drop_dev(c->d_beta2);
+        drop_dev(c->d_comp2);
         drop_dev(c->d_eps2);
         drop_dev(c->d_eps_hi2);
         drop_dev(c->d_eps_lo2);
@@ -606,6 +611,8 @@ void brr::sweep_args(brr_ctx *c, double mu_new, double eps_total, SweepArgs &a, 
         a.rnz = c->d_rnz;
         a.rall = round_all_rows(c);
         a.num_out = c->d_num;
+        a.beta_out = c->d_beta2;
+        a.comp_out = c->d_comp2;
         a.eps_out = c->d_eps2;
         a.eps_hi_out = c->d_eps_hi2;
         a.eps_lo_out = c->d_eps_lo2;
@@ -702,18 +709,16 @@ int brr::sweep_finish(brr_ctx *c, brr_sweep_out *out)
     return sweep_collect(c, out);
 }
 
-// The whole-round sweep of the prepared inputs and its statistics.  A residual
-// that outgrows its fixed-point grid leaves the buffers of the last sweep as
-// they were (the records hold the old effects), and the sweep runs again on a
-// grid 12 bits coarser, four times at most.
+// The whole-round sweep of the prepared inputs and its statistics.  A sweep with a
+// status leaves the chain as it was: its residual, effects and components are in
+// buffers of their own until then.  After a residual that outgrows its fixed-point
+// grid it runs again on a grid 12 bits coarser, four times at most.
 int brr::round_sweep(brr_ctx *c, SweepArgs a, size_t smem, brr_sweep_out *out)
 {
     for (;;) {
         BRR_CUDA(launch_round(a, smem, c->st));
         BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
-        if (a.async_batch == 0)
-            BRR_CUDA(launch_round_finish(a.M, a.form, a.kmax, c->d_num, c->d_u, c->d_group, c->d_gconst, c->d_gK,
-                                         c->d_acum, c->st));
+        BRR_CUDA(launch_round_finish(a, c->d_group, c->st));
         const int rc = sweep_finish(c, out);
         if (rc != BRR_ERR_RANGE || a.headroom >= 48)
             return rc;

@@ -71,6 +71,8 @@ struct brr_ctx {
     double *d_rgram = nullptr;          // pair products of a sweep's rounds
     size_t psum_words = 0, rgram_doubles = 0;
     double *d_num = nullptr;            // the num every marker was decided on
+    double *d_beta2 = nullptr;          // effects and components of the sweep, until it ended well
+    int32_t *d_comp2 = nullptr;
     unsigned long long *d_pstat = nullptr;   // [4] totals of the packed counts, first marker that does not vary
     double *d_emax = nullptr;           // [kPartBlocks] partial maxima of |eps|
     double *d_eps2 = nullptr;           // the residual a sweep writes, swapped with d_eps when it ended well

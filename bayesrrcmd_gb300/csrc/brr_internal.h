@@ -133,6 +133,8 @@ struct SweepArgs {
     const uint32_t *rnz;         // one bit per sweep position: the marker is sure or likely to change
     int rall;                    // the products of every row are formed, not only those of rnz
     double *num_out;             // M: the num each marker was decided on
+    double *beta_out;            // M: effects, and components (-1: none chosen), by marker id; they
+    int32_t *comp_out;           // replace beta and comp when the sweep ended well (k_round_finish)
     double *eps_out;             // the residual after the sweep (not the input buffers)
     float *eps_hi_out, *eps_lo_out;
 };
@@ -319,8 +321,7 @@ cudaError_t launch_round_pairs(const uint32_t *order, int64_t M, int64_t N, int 
                                const uint8_t *codes, int64_t col_stride, const double *table, const double *scale,
                                const int64_t *counts, const uint32_t *nz, int all, int *sums, double *gram, int sms,
                                cudaStream_t st);
-cudaError_t launch_round_finish(int64_t M, int form, int kmax, const double *num, const double *u, const int32_t *group,
-                                const double *gconst, const int32_t *gK, double *acum, cudaStream_t st);
+cudaError_t launch_round_finish(const SweepArgs &a, const int32_t *group, cudaStream_t st);
 size_t sweep_block_smem_bytes(const SweepArgs &a);
 cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, const double *table,
                                 const double *scale, const double *beta, const double *u, const double *z,

@@ -205,11 +205,8 @@ int run_iteration(brr_multi *m)
     }
     cudaError_t e = m->round ? launch_round_multi(m->kmax, ma, smem, m->st)
                              : launch_sweep_multi(m->form, m->kmax, ma, smem, m->st);
-    for (int i = 0; m->round && i < n && e == cudaSuccess; ++i) {
-        const brr_ctx &c = *m->inst[i];
-        e = launch_round_finish(c.cfg.M, c.cfg.form, args[i].kmax, c.d_num, c.d_u, c.d_group, c.d_gconst, c.d_gK,
-                                c.d_acum, m->st);
-    }
+    for (int i = 0; m->round && i < n && e == cudaSuccess; ++i)
+        e = launch_round_finish(args[i], m->inst[i]->d_group, m->st);
     if (e != cudaSuccess)
         return abandon_capture(m, api_fail(BRR_ERR_CUDA, std::string("multi-instance sweep: ") + cudaGetErrorString(e)));
     for (int i = 0; i < n; ++i) {

@@ -954,11 +954,9 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
         if (tid < fin && turn == sidx) {
             const RoundRec &rc = rec[(start + tid) & Rm];
             const int c = s_comp[tid];
-            a.beta[rc.j] = s_beta[tid];
+            a.beta_out[rc.j] = s_beta[tid];
             a.num_out[rc.j] = s_num[tid];
-            a.chosen[rc.j] = c >= 0 ? 1 : 0;
-            if (c >= 0)
-                a.comp[rc.j] = c;
+            a.comp_out[rc.j] = c;
         }
         if (tid <= nchg)
             s_ev[tid] = s_ev2[tid] = 0;
@@ -1417,14 +1415,26 @@ __global__ void k_pair_gram(const uint32_t *__restrict__ order, int64_t M, int64
     }
 }
 
-// P(component 0) of every marker at its final num (src/BayesRBase.cpp:346).
+// The effects, components and chosen flags of a sweep that ended well, and P(component 0)
+// of every marker at its final num (src/BayesRBase.cpp:346; acum null: left as it
+// was).  A sweep with a status leaves the chain as it was.
 template <int KM>
-__global__ void k_round_finish(int64_t M, int form, const double *__restrict__ num, const double *__restrict__ u,
-                               const int32_t *__restrict__ group, const double *__restrict__ gconst,
-                               const int32_t *__restrict__ gK, double *__restrict__ acum)
+__global__ void k_round_finish(int64_t M, int form, const int *__restrict__ err, const double *__restrict__ beta_out,
+                               const int32_t *__restrict__ comp_out, const double *__restrict__ num,
+                               const double *__restrict__ u, const int32_t *__restrict__ group,
+                               const double *__restrict__ gconst, const int32_t *__restrict__ gK,
+                               double *__restrict__ beta, int32_t *__restrict__ comp, uint8_t *__restrict__ chosen,
+                               double *__restrict__ acum)
 {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= M)
+    if (j >= M || *err != kDevOk)
+        return;
+    const int c = comp_out[j];
+    beta[j] = beta_out[j];
+    chosen[j] = c >= 0 ? 1 : 0;
+    if (c >= 0)
+        comp[j] = c;
+    if (!acum)
         return;
     const int g = group[j];
     const double *gc = gconst + (size_t)g * kMaxK * 4;
@@ -1439,9 +1449,9 @@ __global__ void k_round_finish(int64_t M, int form, const double *__restrict__ n
         gcf[2 * k + 1] = k == 0 ? 0.f : __double2float_rn(gc[4 * k + 2]);
     }
     float h, l, a0;
-    int comp;
+    int picked;
     df_from_double(num[j], h, l);
-    if (pick_f32<KM>(h, l, __double2float_rn(u[j]), gcf, gK[g], comp, a0))
+    if (pick_f32<KM>(h, l, __double2float_rn(u[j]), gcf, gK[g], picked, a0))
         acum[j] = (double)a0;
     else
         acum[j] = pick_marker<true, KM>(num[j], u[j], 0.0, 0.0, gc, gK[g]).acum0;
@@ -1641,14 +1651,13 @@ cudaError_t launch_batch_pairs(const uint32_t *order, int64_t M, const uint8_t *
     return cudaSuccess;
 }
 
-cudaError_t launch_round_finish(int64_t M, int form, int kmax, const double *num, const double *u, const int32_t *group,
-                                const double *gconst, const int32_t *gK, double *acum, cudaStream_t st)
+cudaError_t launch_round_finish(const SweepArgs &a, const int32_t *group, cudaStream_t st)
 {
-    const unsigned nb = (unsigned)((M + 127) / 128);
-    if (kmax <= 4)
-        k_round_finish<4><<<nb, 128, 0, st>>>(M, form, num, u, group, gconst, gK, acum);
-    else
-        k_round_finish<kMaxK><<<nb, 128, 0, st>>>(M, form, num, u, group, gconst, gK, acum);
+    const unsigned nb = (unsigned)((a.M + 127) / 128);
+    double *acum = a.async_batch > 0 ? nullptr : a.acum;   // processColumnAsync leaves acum as it was
+    const auto f = a.kmax <= 4 ? k_round_finish<4> : k_round_finish<kMaxK>;
+    f<<<nb, 128, 0, st>>>(a.M, a.form, a.err, a.beta_out, a.comp_out, a.num_out, a.u, group, a.gconst, a.gK, a.beta,
+                          a.comp, a.chosen, acum);
     return cudaGetLastError();
 }
 

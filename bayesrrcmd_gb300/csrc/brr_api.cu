@@ -755,7 +755,7 @@ int run_sweep(brr_ctx *c, double mu_new, double eps_total, brr_sweep_out *out, f
         BRR_CUDA(launch_sweep(cf.form, c->kind, a, smem, c->st));
     BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
     if (c->blocked)
-        BRR_CUDA(launch_block_finish(cf.M, a.kmax, c->d_brec, a.num_df, a.code_pos, c->d_u, c->d_z, c->d_gconst,
+        BRR_CUDA(launch_block_finish(cf.M, a.kmax, a.err, c->d_brec, a.num_df, a.code_pos, c->d_u, c->d_z, c->d_gconst,
                                      c->d_gK, c->d_beta, c->d_acum, c->d_comp, c->d_chosen, c->st));
 
     rc = sweep_finish(c, out);

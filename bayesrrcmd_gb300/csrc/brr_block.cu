@@ -414,16 +414,17 @@ __global__ void k_gather_block(const uint32_t *__restrict__ order, int64_t M, in
 // component: z * sdk + num * invden in double-float, 0 for component 0), acum
 // (P(component 0) of the FP32 sampler at the final num, or of the FP64 evaluation
 // that decided), chosen flag and component, by marker id.  code: component & 0xFF |
-// FP64 decision << 8.
+// FP64 decision << 8.  A sweep that ended with a status has not written all of num
+// and code: the chain keeps what it had.
 template <int KM>
-__global__ void k_block_finish(int64_t M, const BlockRec *__restrict__ rec, const float2 *__restrict__ num,
-                               const int *__restrict__ code, const double *__restrict__ u,
+__global__ void k_block_finish(int64_t M, const int *__restrict__ err, const BlockRec *__restrict__ rec,
+                               const float2 *__restrict__ num, const int *__restrict__ code, const double *__restrict__ u,
                                const double *__restrict__ z, const double *__restrict__ gconst,
                                const int32_t *__restrict__ gK, double *__restrict__ beta, double *__restrict__ acum,
                                int32_t *__restrict__ comp, uint8_t *__restrict__ chosen)
 {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= M)
+    if (q >= M || *err != kDevOk)
         return;
     const BlockRec &r = rec[q];
     const int oc = code[q], K = gK[r.group];
@@ -1427,15 +1428,15 @@ cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, con
     return cudaGetLastError();
 }
 
-cudaError_t launch_block_finish(int64_t M, int kmax, const BlockRec *rec, const float2 *num, const int *code,
-                                const double *u, const double *z, const double *gconst, const int32_t *gK, double *beta,
+cudaError_t launch_block_finish(int64_t M, int kmax, const int *err, const BlockRec *rec, const float2 *num,
+                                const int *code, const double *u, const double *z, const double *gconst, const int32_t *gK, double *beta,
                                 double *acum, int32_t *comp, uint8_t *chosen, cudaStream_t st)
 {
     const unsigned nb = (unsigned)((M + 127) / 128);
     if (kmax <= 4)
-        k_block_finish<4><<<nb, 128, 0, st>>>(M, rec, num, code, u, z, gconst, gK, beta, acum, comp, chosen);
+        k_block_finish<4><<<nb, 128, 0, st>>>(M, err, rec, num, code, u, z, gconst, gK, beta, acum, comp, chosen);
     else
-        k_block_finish<kMaxK><<<nb, 128, 0, st>>>(M, rec, num, code, u, z, gconst, gK, beta, acum, comp, chosen);
+        k_block_finish<kMaxK><<<nb, 128, 0, st>>>(M, err, rec, num, code, u, z, gconst, gK, beta, acum, comp, chosen);
     return cudaGetLastError();
 }
 

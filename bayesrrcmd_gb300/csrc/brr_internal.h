@@ -327,8 +327,8 @@ cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, con
                                 const double *scale, const double *beta, const double *u, const double *z,
                                 const int32_t *group, double eps_total, int kmax, const double *gconst,
                                 const int32_t *gK, BlockRec *rec, cudaStream_t st);
-cudaError_t launch_block_finish(int64_t M, int kmax, const BlockRec *rec, const float2 *num, const int *code,
-                                const double *u, const double *z, const double *gconst, const int32_t *gK, double *beta,
+cudaError_t launch_block_finish(int64_t M, int kmax, const int *err, const BlockRec *rec, const float2 *num,
+                                const int *code, const double *u, const double *z, const double *gconst, const int32_t *gK, double *beta,
                                 double *acum, int32_t *comp, uint8_t *chosen, cudaStream_t st);
 cudaError_t launch_sweep_block(const SweepArgs &a, size_t smem, cudaStream_t st);
 size_t sweep_block_stage_bytes(int B);   // global Gram staging of the blocked sweep

@@ -9,7 +9,7 @@ from bayesrrcmd_gb300 import gpu, plink
 
 pytestmark = pytest.mark.gpu
 S1 = [[0.01, 0.001, 0.0001]]
-RANGE = -6
+RANGE, TIMEOUT = -6, -4
 
 
 def data(N, M, seed, miss=0.02):
@@ -53,4 +53,20 @@ def test_refused_residual_leaves_the_state(gpu_lib, kind, form):
         ch.sweep(order, u, z)
     assert e.value.code == RANGE
     unchanged(ch.state(), before, ("beta", "comp", "acum", "eps"))
+    ch.close()
+
+
+@pytest.mark.parametrize("miss", [0.0, 0.02])
+def test_blocked_sweep_that_ran_out_of_time_leaves_the_effects(gpu_lib, miss):
+    """The waits of the third sweep run out before its first block is decided."""
+    N, M = 1500, 300
+    bed, y = data(N, M, seed=11, miss=miss)
+    ch = chain(bed, N, y, form=gpu.FORM_FP32C, gram=1)
+    ch.iterate(2)
+    before = ch.state()
+    ch.set_wait_limit(50_000_000, 1)
+    with pytest.raises(gpu.BrrError) as e:
+        ch.iterate(1)
+    assert e.value.code == TIMEOUT
+    unchanged(ch.state(), before)
     ch.close()

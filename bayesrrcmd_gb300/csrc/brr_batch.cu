@@ -905,9 +905,11 @@ __global__ void k_batch_gather(const uint32_t *__restrict__ order, int64_t M, co
 // by sweep position, component counts per group and the exact fixed-point sum of the
 // squared non-zero betas per group over the markers whose component was drawn
 // (src/BayesRBase.cpp:200-202, :348-366).  P(component 0) is the FP32 sampler's where
-// that one could certify the decision, else the FP64 one's.
+// that one could certify the decision, else the FP64 one's.  A sweep that ended with a
+// status has not written all of pos and pcomp: the chains keep what they had.
 template <int KM>
-__global__ void __launch_bounds__(256) k_batch_finish(int64_t M, const BatchRec *__restrict__ rec,
+__global__ void __launch_bounds__(256) k_batch_finish(int64_t M, const int *__restrict__ err,
+                                                      const BatchRec *__restrict__ rec,
                                                       const ChainRec *__restrict__ crec, const float4 *__restrict__ pos,
                                                       const signed char *__restrict__ pcomp, int n_groups,
                                                       const double *__restrict__ gconst, const float *__restrict__ gcf,
@@ -917,6 +919,8 @@ __global__ void __launch_bounds__(256) k_batch_finish(int64_t M, const BatchRec 
 {
     __shared__ unsigned long long sv[kMaxGroups * kMaxK];
     __shared__ unsigned long long sb[kMaxGroups][2];
+    if (*err != kDevOk)
+        return;
     const int c = blockIdx.y;
     unsigned long long *o = out + (size_t)c * (n_groups * kMaxK + 2 * n_groups);
     for (int i = threadIdx.x; i < n_groups * kMaxK; i += blockDim.x)
@@ -1024,7 +1028,7 @@ cudaError_t launch_batch_finish(const BatchArgs &a, int kmax, unsigned long long
 {
     const dim3 grid((unsigned)((a.M + 255) / 256 < 64 ? (a.M + 255) / 256 : 64), (unsigned)a.C);
     auto go = [&](auto f) {
-        f<<<grid, 256, 0, st>>>(a.M, a.rec, a.crec, a.pos, a.pcomp, a.n_groups, a.gconst, a.gcf, a.gK, a.beta, a.acum,
+        f<<<grid, 256, 0, st>>>(a.M, a.err, a.rec, a.crec, a.pos, a.pcomp, a.n_groups, a.gconst, a.gcf, a.gK, a.beta, a.acum,
                                 a.comp, out);
     };
     if (kmax <= 4)

@@ -70,3 +70,23 @@ def test_blocked_sweep_that_ran_out_of_time_leaves_the_effects(gpu_lib, miss):
     assert e.value.code == TIMEOUT
     unchanged(ch.state(), before)
     ch.close()
+
+
+def test_batched_sweep_that_ran_out_of_time_leaves_the_effects(gpu_lib):
+    """The same for the chains of a batch."""
+    N, M, C = 1000, 96, 32
+    bed, y = data(N, M, seed=12, miss=0.0)
+    rng = np.random.default_rng(12)
+    b = gpu.Batch(gpu.ChainConfig(N=N, M=M, form=gpu.FORM_FP32C, S=S1, seed=4), C)
+    b.pack_bed(bed)
+    b.set_phenotypes(np.stack([y + 0.1 * rng.normal(size=N) for _ in range(C)]))
+    b.init()
+    b.iterate(2)
+    before = [b.state(c) for c in range(C)]
+    b.set_wait_limit(50_000_000, 1)
+    with pytest.raises(gpu.BrrError) as e:
+        b.iterate(1)
+    assert e.value.code == TIMEOUT
+    for c in range(C):
+        unchanged(b.state(c), before[c])
+    b.close()

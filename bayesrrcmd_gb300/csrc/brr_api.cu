@@ -486,6 +486,8 @@ static RoundMode round_mode(const brr_ctx *c)
 {
     if (c->cfg.async_batch > 0)
         return kRoundAsync;
+    if (c->no_grid)
+        return kRoundRestart;   // most likely refused again: no pair products for it
     if (c->cfg.form == BRR_FORM_FP64 || c->always_pairs)
         return c->d_rgram ? kRoundPairs : kRoundRestart;
     return use_pair_rounds(c) ? kRoundPairs : kRoundRestart;
@@ -709,24 +711,78 @@ int brr::sweep_finish(brr_ctx *c, brr_sweep_out *out)
     return sweep_collect(c, out);
 }
 
+// Widest round of the restart sweep, from the chain's own down, that fits its CTAs
+// (always_pairs: an instance of a multi-instance run).
+static int restart_width(const brr_ctx *c, SweepArgs a)
+{
+    for (a.B = c->B; a.B > 8; a.B /= 2) {
+        const size_t smem = sweep_smem_bytes(c->cfg.form, c->kind, a);
+        const int fit = a.cluster > 0        ? sweep_cluster_fits(c->cfg.form, c->kind, c->G, smem)
+                        : c->always_pairs ? sweep_multi_max_ctas_per_sm(c->cfg.form, kMaxK, smem)
+                                          : sweep_max_ctas_per_sm(c->cfg.form, c->kind, smem);
+        if (a.cluster > 0 ? fit >= 1 : (int64_t)fit * c->sms >= c->G)
+            break;
+    }
+    return a.B;
+}
+
+int brr::restart_prepare(brr_ctx *c, const SweepArgs &a, cudaStream_t st, SweepArgs &res, size_t &smem)
+{
+    const brr_config &cf = c->cfg;
+    res = a;
+    res.B = restart_width(c, a);
+    // the buffers of the sweep under way: the chain's own stay as they are until it ended well
+    if (cf.form == BRR_FORM_FP64) {
+        BRR_CUDA(cudaMemcpyAsync(c->d_eps2, c->d_eps, sizeof(double) * cf.N, cudaMemcpyDeviceToDevice, st));
+    } else {
+        BRR_CUDA(cudaMemcpyAsync(c->d_eps_hi2, c->d_eps_hi, sizeof(float) * cf.N, cudaMemcpyDeviceToDevice, st));
+        BRR_CUDA(cudaMemcpyAsync(c->d_eps_lo2, c->d_eps_lo, sizeof(float) * cf.N, cudaMemcpyDeviceToDevice, st));
+    }
+    BRR_CUDA(cudaMemsetAsync(c->d_comp2, 0xFF, sizeof(int32_t) * cf.M, st));   // -1: none chosen
+    res.eps = c->d_eps2;
+    res.eps_hi = c->d_eps_hi2;
+    res.eps_lo = c->d_eps_lo2;
+    res.beta = c->d_beta2;
+    res.comp = c->d_comp2;
+    res.acum = c->d_num;
+    BRR_CUDA(launch_gather(cf.form, c->kind, c->d_order, cf.M, c->d_table, c->d_scale, c->d_beta, c->d_u, c->d_z,
+                           c->d_group, c->d_colsum, c->d_rec, st));
+    smem = sweep_smem_bytes(cf.form, c->kind, res);
+    c->last_pair = false;
+    return sweep_reset(c, st);
+}
+
+int brr::restart_commit(brr_ctx *c, const SweepArgs &res, cudaStream_t st)
+{
+    SweepArgs f = res;
+    f.beta = c->d_beta;
+    f.comp = c->d_comp;
+    f.acum = c->d_acum;
+    BRR_CUDA(launch_round_finish(f, c->d_group, true, st));
+    return BRR_OK;
+}
+
 // The whole-round sweep of the prepared inputs and its statistics.  A sweep with a
 // status leaves the chain as it was: its residual, effects and components are in
-// buffers of their own until then.  After a residual that outgrows its fixed-point
-// grid it runs again on a grid 12 bits coarser, four times at most.
-int brr::round_sweep(brr_ctx *c, SweepArgs a, size_t smem, brr_sweep_out *out)
+// buffers of their own until then.  Where no fixed-point grid holds the residual as
+// finely as it is stored, or it outgrows its grid, the restart sweep takes its place.
+int brr::round_sweep(brr_ctx *c, const SweepArgs &a, size_t smem, brr_sweep_out *out)
 {
-    for (;;) {
-        BRR_CUDA(launch_round(a, smem, c->st));
-        BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
-        BRR_CUDA(launch_round_finish(a, c->d_group, c->st));
-        const int rc = sweep_finish(c, out);
-        if (rc != BRR_ERR_RANGE || a.headroom >= 48)
-            return rc;
-        a.headroom += 12;
-        const int rr = sweep_reset(c, c->st);
-        if (rr)
-            return rr;
-    }
+    BRR_CUDA(launch_round(a, smem, c->st));
+    BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
+    BRR_CUDA(launch_round_finish(a, c->d_group, false, c->st));
+    int rc = sweep_finish(c, out);
+    c->no_grid = rc == BRR_ERR_RANGE && c->h_misc[0] == 0;
+    if (rc != BRR_ERR_RANGE)
+        return rc;
+    SweepArgs res;
+    rc = restart_prepare(c, a, c->st, res, smem);
+    if (rc)
+        return rc;
+    BRR_CUDA(launch_sweep(c->cfg.form, c->kind, res, smem, c->st));
+    BRR_CUDA(cudaEventRecord(c->ev[1], c->st));
+    rc = restart_commit(c, res, c->st);
+    return rc ? rc : sweep_finish(c, out);
 }
 
 namespace {
@@ -1139,7 +1195,7 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
             dalloc(&c.d_stats, (size_t)cf.n_groups * kMaxK + cf.n_groups + 1) ||
             dalloc(&c.d_part, (size_t)std::max(2 * c.G, kPartBlocks)) || dalloc(&c.d_err, 1) ||
             dalloc(&c.d_rounds, 1) || dalloc(&c.d_prof, 16) || dalloc(&c.d_gstage, sweep_block_stage_bytes(kMaxSpec) / sizeof(double)) || dalloc(&c.d_group, (size_t)M) || dalloc(&c.d_ystd, (size_t)cf.N) ||
-            dalloc(&c.d_nzj, (size_t)M) || dalloc(&c.d_nzb, (size_t)M) || dalloc(&c.d_emax, (size_t)kPartBlocks) ||
+            dalloc(&c.d_nzj, (size_t)M) || dalloc(&c.d_nzb, (size_t)M) || dalloc(&c.d_emax, (size_t)2 * kPartBlocks) ||
             dalloc(&c.d_pstat, 4)) {
             release_pack_buffers(c);
             return fail(BRR_ERR_OOM, "device allocation failed");
@@ -1351,6 +1407,7 @@ int brr_init_chain(brr_ctx *ctx)
     c.iteration = 0;
     c.sweeps = 0;
     c.last_nnz = -1;
+    c.no_grid = false;
     c.inited = true;
     return BRR_OK;
 }
@@ -1480,6 +1537,7 @@ int brr_set_state(brr_ctx *ctx, const brr_state *st)
     std::memcpy(c.pi, st->pi, sizeof(c.pi));
     c.iteration = st->iteration;
     c.last_nnz = -1;
+    c.no_grid = false;
     int rb = prepare_blocked(&c);
     if (!rb)
         rb = prepare_round(&c);

@@ -74,9 +74,10 @@ struct brr_ctx {
     double *d_beta2 = nullptr;          // effects and components of the sweep, until it ended well
     int32_t *d_comp2 = nullptr;
     unsigned long long *d_pstat = nullptr;   // [4] totals of the packed counts, first marker that does not vary
-    double *d_emax = nullptr;           // [kPartBlocks] partial maxima of |eps|
+    double *d_emax = nullptr;           // [2][kPartBlocks] partial maxima and sums of |eps|
     double *d_eps2 = nullptr;           // the residual a sweep writes, swapped with d_eps when it ended well
     float *d_eps_hi2 = nullptr, *d_eps_lo2 = nullptr;
+    bool no_grid = false;               // no residual grid of the last sweep's start was fine enough (round_sweep)
     bool use_round() const { return round_ok && !blocked; }
     bool pair_rounds = false;   // FP32C without the marker Gram: pair-resolved rounds available
     bool last_pair = false;     // the last sweep took pair-resolved rounds
@@ -157,7 +158,11 @@ int sweep_enqueue_outputs(brr_ctx *c, cudaStream_t st);
 int sweep_collect(brr_ctx *c, brr_sweep_out *out);
 int iter_post(brr_ctx &c, const brr_sweep_out &so, uint32_t it);
 void choose_round(brr_ctx &c);
-int round_sweep(brr_ctx *c, SweepArgs a, size_t smem, brr_sweep_out *out);
+int round_sweep(brr_ctx *c, const SweepArgs &a, size_t smem, brr_sweep_out *out);
+// The restart sweep in place of a whole-round sweep (a) that was refused: its inputs
+// and arguments (res, with the shared memory), and, after the launch, the commit.
+int restart_prepare(brr_ctx *c, const SweepArgs &a, cudaStream_t st, SweepArgs &res, size_t &smem);
+int restart_commit(brr_ctx *c, const SweepArgs &res, cudaStream_t st);
 // New slicing (G CTAs) and, if B > 0, round width of a packed chain.
 int reslice(brr_ctx *c, int G, int B);
 

@@ -124,9 +124,8 @@ struct SweepArgs {
     int form;                    // BRR_FORM_*: how the residual is stored between sweeps
     int rkind;                   // BRR_KIND_DENSE, or any other value for the sparse kinds
     int rmode;                   // RoundMode
-    int headroom;                // bits of headroom of the fixed-point residual beyond the default 3
     int n_emax;
-    const double *emax;          // [n_emax] partial maxima of |eps| before mu_new is subtracted
+    const double *emax;          // [2][n_emax] partial maxima and sums of |eps| before mu_new is subtracted
     const RoundRec *rrec;        // M records in sweep order
     const double *rgram;         // [blocks of B][B (B-1) / 2] pair products in sweep order (pairs only)
     const double *u, *z;         // M: the markers' draws, by marker id (also the blocked sweep's)
@@ -321,7 +320,8 @@ cudaError_t launch_round_pairs(const uint32_t *order, int64_t M, int64_t N, int 
                                const uint8_t *codes, int64_t col_stride, const double *table, const double *scale,
                                const int64_t *counts, const uint32_t *nz, int all, int *sums, double *gram, int sms,
                                cudaStream_t st);
-cudaError_t launch_round_finish(const SweepArgs &a, const int32_t *group, cudaStream_t st);
+// acum_given: num_out holds P(component 0) (the restart sweep's).
+cudaError_t launch_round_finish(const SweepArgs &a, const int32_t *group, bool acum_given, cudaStream_t st);
 size_t sweep_block_smem_bytes(const SweepArgs &a);
 cudaError_t launch_gather_block(const uint32_t *order, int64_t M, int64_t N, const double *table,
                                 const double *scale, const double *beta, const double *u, const double *z,

@@ -150,6 +150,47 @@ int abandon_capture(brr_multi *m, int rc)
     return rc;
 }
 
+// The restart sweep of some instances, in one launch, in place of their whole-round
+// sweeps (args), and its statistics.
+int restart_again(brr_multi *m, const std::vector<int> &which, const std::vector<SweepArgs> &args,
+                  std::vector<brr_sweep_out> &so)
+{
+    MultiSweepArgs ma{};
+    size_t smem = 0;
+    for (const int i : which) {
+        brr_ctx &c = *m->inst[i];
+        size_t si = 0;
+        const int rc = restart_prepare(&c, args[i], m->st, ma.inst[ma.n], si);
+        if (rc)
+            return rc;
+        smem = std::max(smem, si);
+        ma.kind[ma.n] = c.kind == BRR_KIND_DENSE ? 0 : 1;
+        ma.cta_start[ma.n + 1] = ma.cta_start[ma.n] + c.G;
+        ++ma.n;
+    }
+    const int per_sm = sweep_multi_max_ctas_per_sm(m->form, m->kmax, smem);
+    if (per_sm < 1 || (int64_t)per_sm * m->sms < ma.cta_start[ma.n])
+        return api_fail(BRR_ERR_RANGE, "the residual left its fixed-point grid and the restart sweep does not fit");
+    MULTI_CUDA(launch_sweep_multi(m->form, m->kmax, ma, smem, m->st));
+    for (int k = 0; k < ma.n; ++k) {
+        brr_ctx *c = m->inst[which[k]];
+        int rc = restart_commit(c, ma.inst[k], m->st);
+        if (!rc)
+            rc = sweep_enqueue_outputs(c, m->st);
+        if (rc)
+            return rc;
+    }
+    MULTI_CUDA(cudaMemcpyAsync(m->h_t, m->d_t, sizeof(unsigned long long) * 2 * m->n, cudaMemcpyDeviceToHost, m->st));
+    MULTI_CUDA(cudaEventRecord(m->ev[1], m->st));
+    MULTI_CUDA(cudaStreamSynchronize(m->st));
+    for (const int i : which) {
+        const int rc = sweep_collect(m->inst[i], &so[i]);
+        if (rc)
+            return rc;
+    }
+    return BRR_OK;
+}
+
 // One iteration of every instance: the host parts of updateMu, then one CUDA
 // graph holding all instances' draws, sweep orders, constants and records,
 // the one launch of the multi-instance sweep, and all instances' statistics
@@ -206,7 +247,7 @@ int run_iteration(brr_multi *m)
     cudaError_t e = m->round ? launch_round_multi(m->kmax, ma, smem, m->st)
                              : launch_sweep_multi(m->form, m->kmax, ma, smem, m->st);
     for (int i = 0; m->round && i < n && e == cudaSuccess; ++i)
-        e = launch_round_finish(args[i], m->inst[i]->d_group, m->st);
+        e = launch_round_finish(args[i], m->inst[i]->d_group, false, m->st);
     if (e != cudaSuccess)
         return abandon_capture(m, api_fail(BRR_ERR_CUDA, std::string("multi-instance sweep: ") + cudaGetErrorString(e)));
     for (int i = 0; i < n; ++i) {
@@ -237,19 +278,22 @@ int run_iteration(brr_multi *m)
     MULTI_CUDA(cudaGraphLaunch(m->exec, m->st));
     MULTI_CUDA(cudaEventRecord(m->ev[1], m->st));
     MULTI_CUDA(cudaStreamSynchronize(m->st));
+    // instances whose residual no fixed-point grid holds (see round_sweep) run the restart sweep together
+    std::vector<int> again;
     for (int i = 0; i < n; ++i) {
         brr_ctx &c = *m->inst[i];
-        int rc = sweep_collect(&c, &so[i]);
-        if (rc == BRR_ERR_RANGE && m->round) {
-            // the residual outgrew its fixed-point grid: this instance's sweep again, alone, on a coarser one
-            args[i].headroom += 12;
-            rc = sweep_reset(&c, c.st);
-            if (!rc)
-                rc = round_sweep(&c, args[i], smem, &so[i]);
-        }
-        if (rc)
+        const int rc = sweep_collect(&c, &so[i]);
+        if (rc == BRR_ERR_RANGE && m->round)
+            again.push_back(i);
+        else if (rc)
             return rc;
-        rc = iter_post(c, so[i], its[i]);
+        c.no_grid = rc == BRR_ERR_RANGE && c.h_misc[0] == 0;
+    }
+    const int rr = again.empty() ? BRR_OK : restart_again(m, again, args, so);
+    if (rr)
+        return rr;
+    for (int i = 0; i < n; ++i) {
+        const int rc = iter_post(*m->inst[i], so[i], its[i]);
         if (rc)
             return rc;
     }

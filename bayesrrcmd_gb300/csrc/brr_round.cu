@@ -18,11 +18,16 @@
 // Residual.  Each CTA owns a slice of individuals.  Its residual is exact fixed
 // point E = eps 2^s (int64; s from the largest |eps| at the sweep start, 3 bits
 // of headroom below 2^62), so sums do not depend on their order and an update
-// adds the nearest integer of dBeta x 2^s.  At |eps| < 8 the grid is 2^-56,
-// finer than the FP64 spacing of values above 2^-4.  A value that outgrows
-// the headroom sets the range status and the host runs the sweep again with a
-// coarser grid; the residual in memory is only replaced by a sweep that ended
-// well.
+// adds the nearest integer of dBeta x 2^s.  The grid is one for all individuals,
+// where a stored value (FP64, or a pair of FP32 words) has a spacing of its own, so
+// it has to be no coarser than the spacing at a typical value, the mean of |eps|:
+// 2^-s <= 2^(floor(log2 mean) - 53) in the FP64 form, 2^(... - 49) in the FP32C form.
+// With normal residuals of variance 1 the largest of 100,000 is 4.5, 2^-s is 2^-56 and
+// 2^-54 would do; one bit of headroom instead of three allows for a largest |eps| of
+// 100 to 200 means.  Where no grid is fine enough (an outlier further out, values that
+// are not finite), and where a value outgrows the headroom during the sweep, the
+// sweep ends with the range status and the host runs the restart sweep instead; the
+// residual in memory is only replaced by a sweep that ended well.
 //
 // Dot products run on the tensor cores: E in seven balanced 10-bit limbs stored
 // as FP16 planes (|limb| <= 512) times the genotypes 0, 1, 2 in FP16 with FP32
@@ -328,14 +333,20 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     for (int i = tid; i < (kMaxSpec + 1) * 4; i += kRT)
         (&s_acc[0][0])[i] = 0ull;
     {
-        double mx = 0.0;
-        for (int i = tid; i < a.n_emax; i += kRT)
+        double mx = 0.0, sa = 0.0;
+        for (int i = tid; i < a.n_emax; i += kRT) {
             mx = fmax(mx, a.emax[i]);
+            sa += a.emax[a.n_emax + i];
+        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1) {
             mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0)
+            sa += __shfl_xor_sync(0xffffffffu, sa, o);
+        }
+        if (lane == 0) {
             s_red[warp][0] = mx;
+            s_red[warp][1] = sa;
+        }
     }
     if (tid == 0) {
         s_abort = 0;
@@ -358,18 +369,29 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
         issue_gram(1);
         cp_async_commit();
     }
-    double emax = fabs(a.mu_new);
+    // the residual's scale, the same in every CTA
+    int sc;
+    bool coarse;
     {
-        double mx = 0.0;
-        for (int w = 0; w < kRW; ++w)
+        double mx = 0.0, sa = 0.0;
+        for (int w = 0; w < kRW; ++w) {
             mx = fmax(mx, s_red[w][0]);
-        emax += mx;
+            sa += s_red[w][1];
+        }
+        // bounds of the residual after mu_new is subtracted: emax < 2^e2, and its mean
+        // magnitude from below
+        const double emax = fabs(a.mu_new) + mx, mean = sa / (double)a.N - fabs(a.mu_new);
+        auto exponent = [](double v) { return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7FF) - 1023; };
+        const int e2 = exponent(emax) + 1;
+        const int need = (a.form == BRR_FORM_FP64 ? 53 : 49) - exponent(mean);
+        const int most = min(61 - e2, 100);   // E below 2^61: one bit of headroom
+        sc = max(min(59 - e2, most), min(need, most));
+        coarse = !(mean > 0.0) || !(emax < 1e290) || sc < need;   // also where the sums are not finite
+        if (coarse)
+            sc = 0;
     }
-    // emax < 2^e2; E stays below 2^(59 - extra headroom) at the start
-    const int e2 = emax > 0.0 ? (int)(((unsigned long long)__double_as_longlong(emax) >> 52) & 0x7FF) - 1022 : 1;
-    const int sc = min(59 - e2 - a.headroom, 100);
     const double up = pow2d(sc), down = pow2d(-sc);
-    bool range = false;
+    bool range = coarse;
     for (int i = tid; i < a.slice_max; i += kRT) {
         const int ind = limb_individual(i);
         long long v = 0;
@@ -447,7 +469,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     const int mt = warp % nmt, kg = warp / nmt;
     const int fg = lane >> 2, fq = lane & 3;   // fragment row / column group
 
-    unsigned start = 0;
+    unsigned start = coarse ? M32 : 0u;
     long long r = 0;
     int turn = 0;   // r mod G: the CTA that writes the round's outputs
     while (start < M32) {
@@ -1417,11 +1439,11 @@ __global__ void k_pair_gram(const uint32_t *__restrict__ order, int64_t M, int64
 
 // The effects, components and chosen flags of a sweep that ended well, and P(component 0)
 // of every marker at its final num (src/BayesRBase.cpp:346; acum null: left as it
-// was).  A sweep with a status leaves the chain as it was.
+// was; acum_given: num holds it).  A sweep with a status leaves the chain as it was.
 template <int KM>
 __global__ void k_round_finish(int64_t M, int form, const int *__restrict__ err, const double *__restrict__ beta_out,
                                const int32_t *__restrict__ comp_out, const double *__restrict__ num,
-                               const double *__restrict__ u, const int32_t *__restrict__ group,
+                               bool acum_given, const double *__restrict__ u, const int32_t *__restrict__ group,
                                const double *__restrict__ gconst, const int32_t *__restrict__ gK,
                                double *__restrict__ beta, int32_t *__restrict__ comp, uint8_t *__restrict__ chosen,
                                double *__restrict__ acum)
@@ -1436,6 +1458,10 @@ __global__ void k_round_finish(int64_t M, int form, const int *__restrict__ err,
         comp[j] = c;
     if (!acum)
         return;
+    if (acum_given) {
+        acum[j] = num[j];
+        return;
+    }
     const int g = group[j];
     const double *gc = gconst + (size_t)g * kMaxK * 4;
     if (form == BRR_FORM_FP64) {
@@ -1651,13 +1677,13 @@ cudaError_t launch_batch_pairs(const uint32_t *order, int64_t M, const uint8_t *
     return cudaSuccess;
 }
 
-cudaError_t launch_round_finish(const SweepArgs &a, const int32_t *group, cudaStream_t st)
+cudaError_t launch_round_finish(const SweepArgs &a, const int32_t *group, bool acum_given, cudaStream_t st)
 {
     const unsigned nb = (unsigned)((a.M + 127) / 128);
     double *acum = a.async_batch > 0 ? nullptr : a.acum;   // processColumnAsync leaves acum as it was
     const auto f = a.kmax <= 4 ? k_round_finish<4> : k_round_finish<kMaxK>;
-    f<<<nb, 128, 0, st>>>(a.M, a.form, a.err, a.beta_out, a.comp_out, a.num_out, a.u, group, a.gconst, a.gK, a.beta,
-                          a.comp, a.chosen, acum);
+    f<<<nb, 128, 0, st>>>(a.M, a.form, a.err, a.beta_out, a.comp_out, a.num_out, acum_given, a.u, group, a.gconst,
+                          a.gK, a.beta, a.comp, a.chosen, acum);
     return cudaGetLastError();
 }
 

@@ -86,12 +86,13 @@ __global__ void k_gather(int form, int kind, const uint32_t *__restrict__ order,
     rec[q] = r;
 }
 
-// updateMu, first half: eps += mu_old, and per-block sum(eps) and max |eps| (src/DenseBayesRRmz.cpp:38-39).
+// updateMu, first half: eps += mu_old, and per-block sum(eps) (src/DenseBayesRRmz.cpp:38-39), max |eps|
+// and sum |eps| (emax, and nblocks further).
 __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, double mu_old, double *eps,
                                                       float *eps_hi, float *eps_lo, double *part, double *emax)
 {
-    __shared__ double red[kThreads / 32][2];
-    double s = 0.0, mx = 0.0;
+    __shared__ double red[kThreads / 32][3];
+    double s = 0.0, mx = 0.0, sa = 0.0;
     float mh, ml;
     df_from_double(mu_old, mh, ml);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
@@ -100,33 +101,40 @@ __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, doubl
             eps[i] = e;
             s += e;
             mx = fmax(mx, fabs(e));
+            sa += fabs(e);
         } else {
             float h = eps_hi[i], l = eps_lo[i];
             df_add(h, l, mh, ml);
             eps_hi[i] = h;
             eps_lo[i] = l;
-            s += (double)h + (double)l;
+            const double e = (double)h + (double)l;
+            s += e;
             mx = fmax(mx, fabs((double)h) + fabs((double)l));
+            sa += fabs(e);
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, o);
         mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
     }
     if ((threadIdx.x & 31) == 0) {
         red[threadIdx.x >> 5][0] = s;
         red[threadIdx.x >> 5][1] = mx;
+        red[threadIdx.x >> 5][2] = sa;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0.0, m = 0.0;
+        double t = 0.0, m = 0.0, ta = 0.0;
         for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
             t += red[q][0];
             m = fmax(m, red[q][1]);
+            ta += red[q][2];
         }
         part[blockIdx.x] = t;
         emax[blockIdx.x] = m;
+        emax[gridDim.x + blockIdx.x] = ta;
     }
 }
 

@@ -1258,7 +1258,7 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
         if (!c.round_ok)
             return fail(BRR_ERR_ARG, "the sweep kernel does not fit " + std::to_string(c.G) + " co-resident CTAs");
         c.packed = true;
-        return BRR_OK;
+        return c.inited ? prepare_round(&c) : BRR_OK;
     }
     // the sweep kernel must fit one CTA per slice on the GPU at once
     SweepArgs a{};
@@ -1274,7 +1274,7 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
                                          " bytes of shared memory each cannot be scheduled");
         choose_round(c);
         c.packed = true;
-        return BRR_OK;
+        return c.inited ? prepare_round(&c) : BRR_OK;
     }
     const int per_sm = sweep_max_ctas_per_sm(cf.form, c.kind, smem);
     if (per_sm < 1 || (int64_t)per_sm * c.sms < c.G)
@@ -1282,7 +1282,8 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
                                      " co-resident CTAs (shared memory " + std::to_string(smem) + " bytes)");
     choose_round(c);
     c.packed = true;
-    return BRR_OK;
+    // markers packed again under a running chain: its sweep's buffers follow them
+    return c.inited ? prepare_round(&c) : BRR_OK;
 }
 
 int brr_get_marker_table(brr_ctx *ctx, double *table, int64_t *counts)

@@ -139,6 +139,35 @@ bool allocate(const std::vector<double> &work, const std::vector<int> &mins, con
     return true;
 }
 
+// Dynamic shared memory a CTA may use beside the restart sweep's static arrays.
+int restart_smem_limit(const brr_multi *m, size_t &limit)
+{
+    int optin = 0;
+    MULTI_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->dev));
+    limit = (size_t)optin - sweep_multi_static_smem(m->form, m->kmax);
+    return BRR_OK;
+}
+
+// Every instance on the restart sweep from here on, each with the widest round of at
+// most 32 that fits its slices.  All sweeps of an iteration are one launch of one
+// kernel, so an instance that cannot run the whole-round sweep (no memory for its
+// buffers, slices that do not fit it) takes the others with it.
+int take_restart(brr_multi *m)
+{
+    const int rc = restart_smem_limit(m, m->smem_limit);
+    if (rc)
+        return rc;
+    m->round = false;
+    for (brr_ctx *c : m->inst) {
+        c->no_round = true;
+        c->always_pairs = false;
+        choose_round(*c);
+        for (c->B = std::min(c->B, 32); c->B > 8 && inst_smem(c, c->G, c->B, false) > m->smem_limit;)
+            c->B /= 2;
+    }
+    return BRR_OK;
+}
+
 // Ends a stream capture that failed part way, so the stream is usable again.
 int abandon_capture(brr_multi *m, int rc)
 {
@@ -199,6 +228,12 @@ int restart_again(brr_multi *m, const std::vector<int> &which, const std::vector
 int run_iteration(brr_multi *m)
 {
     const int n = m->n;
+    for (int i = 0; i < n && m->round; ++i)
+        if (!m->inst[i]->use_round()) {
+            const int rc = take_restart(m);
+            if (rc)
+                return rc;
+        }
     std::vector<SweepArgs> args(n);
     std::vector<brr_sweep_out> so(n);
     std::vector<uint32_t> its(n);
@@ -363,8 +398,12 @@ int brr_multi_create(const brr_config *cfgs, int32_t n, brr_multi **out)
     for (int pass = 0; pass < 4 && !split; ++pass) {
         m->round = pass < 2;
         // dynamic shared memory: what a CTA may use beside the kernel's static arrays
-        m->smem_limit = m->round ? kMaxRoundSmem
-                                 : prop.sharedMemPerBlockOptin - sweep_multi_static_smem(m->form, m->kmax);
+        m->smem_limit = kMaxRoundSmem;
+        if (!m->round) {
+            const int rc = restart_smem_limit(m, m->smem_limit);
+            if (rc)
+                return bail(rc);
+        }
         split = true;
         for (int i = 0; i < n; ++i) {
             const brr_ctx *c = m->inst[i];

@@ -364,7 +364,7 @@ void brr::choose_round(brr_ctx &c)
     for (int B = asked; B >= 8 && !c.round_ok && !c.no_round; B /= 2) {
         a.B = B;
         const size_t smem = round_smem_bytes(a);
-        const int fit = smem <= kMaxRoundSmem ? round_fits(c.G, smem, a.cluster > 0) : 0;
+        const int fit = smem <= round_smem_limit(c.dev) ? round_fits(c.G, smem, a.cluster > 0) : 0;
         c.round_ok = a.cluster > 0 ? fit >= 1 : (int64_t)fit * c.sms >= c.G;
         c.RB = B;
         if (cf.spec_width || cf.async_batch)

@@ -129,7 +129,6 @@ namespace brr {
 
 constexpr size_t kAccWords = 8 * 8 * kMaxSpec * 4;
 constexpr size_t kCounterWords = 2 * 8 * 16;
-constexpr size_t kMaxRoundSmem = 220 * 1024;   // dynamic shared memory of the whole-round sweep, beside its static arrays
 constexpr int kPartBlocks = 608;   // 4 x 152 SMs for the updateMu reduction
 
 // Phases of one iteration of a chain (BayesRBase::runGibbs loop body,

@@ -307,6 +307,8 @@ int sweep_cluster_fits(int form, int kind, int G, size_t smem);
 // Whole-round sweep (brr_round.cu).
 size_t round_smem_bytes(const SweepArgs &a);
 int round_fits(int G, size_t smem, bool cluster);
+// Dynamic shared memory that a CTA of every variant may use beside its static arrays.
+size_t round_smem_limit(int dev);
 cudaError_t launch_round(const SweepArgs &a, size_t smem, cudaStream_t st);
 // nz: room for M bits rounded up to 256.
 cudaError_t launch_round_gather(const uint32_t *order, int64_t M, int64_t N, int kind, int kmax, const double *table,

@@ -398,8 +398,9 @@ int brr_multi_create(const brr_config *cfgs, int32_t n, brr_multi **out)
     for (int pass = 0; pass < 4 && !split; ++pass) {
         m->round = pass < 2;
         // dynamic shared memory: what a CTA may use beside the kernel's static arrays
-        m->smem_limit = kMaxRoundSmem;
-        if (!m->round) {
+        if (m->round) {
+            m->smem_limit = round_smem_limit(m->dev);
+        } else {
             const int rc = restart_smem_limit(m, m->smem_limit);
             if (rc)
                 return bail(rc);

@@ -1531,6 +1531,29 @@ size_t round_smem_bytes(const SweepArgs &a)
     return round_plan(a.slice_max, a.B, a.n_groups, a.cluster, a.rmode == kRoundPairs, a.has_missing != 0).total;
 }
 
+size_t round_smem_limit(int dev)
+{
+    const void *fs[10] = {(const void *)k_round_multi<4>, (const void *)k_round_multi<kMaxK>};
+    int n = 2, optin = 0;
+    for (int km : {4, kMaxK})
+        for (int v = 0; v < 4; ++v)
+            fs[n++] = round_fn(km, (v & 1) != 0, (v & 2) != 0);
+    size_t used = 0;
+    for (const void *f : fs) {
+        cudaFuncAttributes fa{};
+        if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        used = fa.sharedSizeBytes > used ? fa.sharedSizeBytes : used;
+    }
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (size_t)optin - used;
+}
+
 // CTAs that can be resident at once: per SM without a cluster, else 1 when a
 // cluster of G CTAs can be scheduled (0: none).
 int round_fits(int G, size_t smem, bool cluster)

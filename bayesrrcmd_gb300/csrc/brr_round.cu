@@ -168,15 +168,28 @@ __device__ __forceinline__ float double_hi(double v)
 
 __device__ __forceinline__ bool nonzero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) != 0ull; }
 
-// A decision the margin sampler cannot certify: the guarded FP32 sampler, else
-// FP64.  Out of line: about one marker in a thousand.
+// The guarded FP32 sampler's decision on num as a pair of FP32 words, -2 where it cannot
+// certify one.
 template <int KM>
-__device__ __noinline__ int decide_slow(float nh, float nl, double u, const double *gc, const float *gcf, int K)
+__device__ __noinline__ int decide_pair(float nh, float nl, float uf, const float *gcf, int K)
 {
     int comp;
     float a0;
-    if (!pick_f32<KM>(nh, nl, __double2float_rn(u), gcf, K, comp, a0))
-        comp = pick_marker<true, KM>((double)nh + (double)nl, u, 0.0, 0.0, gc, K).comp;
+    return pick_f32<KM>(nh, nl, uf, gcf, K, comp, a0) ? comp : -2;
+}
+
+// A decision the margin sampler cannot certify: the guarded FP32 sampler, else
+// FP64 on the marker's FP64 num (a pair of FP32 words holds 48 bits of it, which
+// moves P(component 0) by up to 1e-12 of itself).  Out of line: about one marker in a
+// thousand.
+template <int KM>
+__device__ __noinline__ int decide_slow(double num, double u, const double *gc, const float *gcf, int K)
+{
+    float nh, nl;
+    df_from_double(num, nh, nl);
+    int comp = decide_pair<KM>(nh, nl, __double2float_rn(u), gcf, K);
+    if (comp == -2)
+        comp = pick_marker<true, KM>(num, u, 0.0, 0.0, gc, K).comp;
     return comp;
 }
 
@@ -782,6 +795,16 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             // num^2 grows).  Only such a marker's component is worked out, when the
             // chain reaches it; the markers before it stay in component 0.
             int nchg = 0, fin = nb, pos = 0;
+            // num of marker p after the changes so far, from the FP64 warp, on one lane
+            auto ask_num = [&](int p) -> double {
+                s_ask = (nchg << 8) | (p + 1);
+                unsigned spins = 0;
+                while (s_ask != 0 && ++spins < (1u << 28))
+                    ;
+                if (s_ask != 0)
+                    atomicCAS(a.err, kDevOk, kDevTimeout);
+                return s_told;
+            };
             if (a.rmode == kRoundAsync) {
                 // every marker is decided on the residual before the batch
 #pragma unroll 1
@@ -789,14 +812,17 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     const int t = lane + 32 * h;
                     int comp = 0;
                     const bool c = (h ? sx[1] : sx[0]) > (h ? s0[1] : s0[0]) && t < nb;
-                    if (c) {
-                        const RoundRec &rc = rec[(start + t) & Rm];
-                        const int g = (int)(rc.gm & 255u);
-                        comp = decide_slow<KM>(s_ndf[t].x, s_ndf[t].y, a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
-                                               gcf + (size_t)g * kMaxK * 2, gk[g]);
+                    const RoundRec &rc = rec[(start + (c ? t : 0)) & Rm];
+                    const unsigned g = rc.gm & 255u;
+                    if (c)
+                        comp = decide_pair<KM>(s_ndf[t].x, s_ndf[t].y, rc.uf, gcf + (size_t)g * kMaxK * 2, gk[g]);
+                    for (unsigned m = __ballot_sync(0xffffffffu, comp == -2); m; m &= m - 1u) {
+                        if (lane == __ffs(m) - 1)
+                            comp = decide_slow<KM>(ask_num(t), a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
+                                                   gcf + (size_t)g * kMaxK * 2, gk[g]);
+                        __syncwarp();
                     }
-                    __syncwarp();
-                    const bool b = c && (comp > 0 || rec[(start + t) & Rm].beta_old != 0.0);
+                    const bool b = c && (comp > 0 || rc.beta_old != 0.0);
                     const unsigned kb = __ballot_sync(0xffffffffu, b);
                     if (c)
                         s_comp[t] = comp;
@@ -836,18 +862,9 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                                           reinterpret_cast<const float2 *>(gcf + (size_t)g * kMaxK * 2)[lane & (kMaxK - 1)],
                                           gk[g], 5e6f * pe * (fabsf(px) + pe));
                 if (comp == -2) {
-                    if (own) {
-                        s_ask = (nchg << 8) | (p + 1);
-                        unsigned spins = 0;
-                        while (s_ask != 0 && ++spins < (1u << 28))
-                            ;
-                        if (s_ask != 0)
-                            atomicCAS(a.err, kDevOk, kDevTimeout);
-                        float nh, nl;
-                        df_from_double(s_told, nh, nl);
-                        comp = decide_slow<KM>(nh, nl, a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
+                    if (own)
+                        comp = decide_slow<KM>(ask_num(p), a.u[rc.j], gconst + (size_t)g * kMaxK * 4,
                                                gcf + (size_t)g * kMaxK * 2, gk[g]);
-                    }
                     comp = __shfl_sync(0xffffffffu, comp, p & 31);
                 }
                 if (own)

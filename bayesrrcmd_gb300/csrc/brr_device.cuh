@@ -55,6 +55,18 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
     return v;
 }
 
+// A shared-memory word that another warp of the CTA writes after a __threadfence_block:
+// what that warp wrote before is visible after this load has seen the word.
+__device__ __forceinline__ unsigned ld_acquire_shared(const volatile void *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];"
+                 : "=r"(v)
+                 : "r"((unsigned)__cvta_generic_to_shared(const_cast<const void *>(p)))
+                 : "memory");
+    return v;
+}
+
 __device__ __forceinline__ uint64_t global_timer_ns()
 {
     uint64_t t;

@@ -166,6 +166,14 @@ __device__ __forceinline__ float double_hi(double v)
                : __uint_as_float((top & 0x80000000u) | (((unsigned)(b >> 29) + 0x40000000u) & 0x7FFFFFFFu));
 }
 
+// Whether row q of a block's pair products is in shared memory: known before the round
+// (n0, n1), or, where rows are fetched during it (late), arrived since (nz, set after the row).
+__device__ __forceinline__ bool row_here(const uint32_t *nz, uint32_t n0, uint32_t n1, int q, bool late)
+{
+    const unsigned bit = 1u << (q & 31);
+    return ((q < 32 ? n0 : n1) & bit) != 0u || (late && (ld_acquire_shared(&nz[q >> 5]) & bit) != 0u);
+}
+
 __device__ __forceinline__ bool nonzero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) != 0ull; }
 
 // The guarded FP32 sampler's decision on num as a pair of FP32 words, -2 where it cannot
@@ -746,6 +754,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     const double x = up * (lane == 1 ? (dense ? rp.x : 0.0)
                                                      : __dmul_rn(__dsub_rn(lane == 0 ? 2.0 : lane == 2 ? 1.0 : 0.0, rp.m), rp.s));
                     wait_event(&s_ev2[u]);
+                    ld_acquire_shared(&s_ev2[u]);   // orders s_dB after the word
                     if (lane < 4) {
                         const double d = __dmul_rn(s_dB[u], x);   // up is a power of two
                         // |d| < 2^62, by its exponent
@@ -777,7 +786,10 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             }
             const double *gr = reinterpret_cast<const double *>(smem + plan.gram + (blk & 1u) * gslot);
             const double *grow = a.rgram + (size_t)blk * gn;
-            const volatile uint32_t *nz = s_nz[blk & 1u];
+            // rows that were in shared memory before the round, as bits; those that arrive
+            // during it are looked up
+            const uint32_t *nz = s_nz[blk & 1u];
+            const uint32_t nz0 = nz[0], nz1 = nz[1];
             __syncwarp();
             asm volatile("bar.sync 1, 96;" ::: "memory");
             mark(2);
@@ -801,7 +813,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 unsigned spins = 0;
                 while (s_ask != 0 && ++spins < (1u << 28))
                     ;
-                if (s_ask != 0)
+                if (ld_acquire_shared(&s_ask) != 0u)   // orders the answer after the word
                     atomicCAS(a.err, kDevOk, kDevTimeout);
                 return s_told;
             };
@@ -845,7 +857,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 bool last = !pairs;
                 if (pairs) {
                     const int q = off + p;
-                    const bool here = ((nz[q >> 5] >> (q & 31)) & 1u) != 0u;
+                    const bool here = row_here(nz, nz0, nz1, q, a.rall != 0);
                     last = !here && !a.rall;
                     const double *row = (here ? gr : grow) + q * (2 * B - q - 1) / 2 - p - 1;
                     if (!last && lane > p && lane < nb)
@@ -915,7 +927,8 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             // num, beta and the corrections in FP64, one change behind the chain
             const double *gr = reinterpret_cast<const double *>(smem + plan.gram + (blk & 1u) * gslot);
             const double *grow = a.rgram + (size_t)blk * gn;
-            const volatile uint32_t *nz = s_nz[blk & 1u];
+            const uint32_t *nz = s_nz[blk & 1u];
+            const uint32_t nz0 = nz[0], nz1 = nz[1];
             __syncwarp();
             asm volatile("bar.sync 2, 96;" ::: "memory");
             wstart();
@@ -929,7 +942,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             for (;; ++nchg) {
                 int ev;
                 unsigned spins = 0;
-                while ((ev = s_ev[nchg]) == 0 && ++spins < (1u << 28)) {
+                while ((ev = s_ev[nchg]) == 0 && ++spins < (1u << 28)) {   // the word is all it says
                     const int ask = s_ask;
                     if (ask != 0 && ((ask - 1) & 31) == lane && ask >> 8 == nchg) {
                         s_told = ((ask - 1) & 32) ? num[1] : num[0];
@@ -961,7 +974,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     continue;
                 dB = __shfl_sync(0xffffffffu, dB, p & 31);
                 const int q = off + p;
-                const bool here = ((nz[q >> 5] >> (q & 31)) & 1u) != 0u;
+                const bool here = row_here(nz, nz0, nz1, q, a.rall != 0);
                 if (!here && !a.rall)
                     continue;   // the round ends here
                 const double *row = (here ? gr : grow) + q * (2 * B - q - 1) / 2 - p - 1;

@@ -80,6 +80,7 @@ constexpr int kCountShift = 56;
 constexpr unsigned long long kAccBias = 1ull << 47;   // |value| < 2^47 of one CTA, 255 CTAs below 2^56
 constexpr unsigned long long kAccMask = (1ull << kCountShift) - 1;
 constexpr long long kLow30 = (1ll << 30) - 1;
+constexpr long long kNoChange = 0x7FF8000000000001ll;   // a NaN that no arithmetic returns
 
 struct RoundPlan {
     size_t E, planes, codes, rec, gram, ids, part, gconst, gk, gcf, gdf, xch, prev, total;
@@ -166,14 +167,6 @@ __device__ __forceinline__ float double_hi(double v)
                : __uint_as_float((top & 0x80000000u) | (((unsigned)(b >> 29) + 0x40000000u) & 0x7FFFFFFFu));
 }
 
-// Whether row q of a block's pair products is in shared memory: known before the round
-// (n0, n1), or, where rows are fetched during it (late), arrived since (nz, set after the row).
-__device__ __forceinline__ bool row_here(const uint32_t *nz, uint32_t n0, uint32_t n1, int q, bool late)
-{
-    const unsigned bit = 1u << (q & 31);
-    return ((q < 32 ? n0 : n1) & bit) != 0u || (late && (ld_acquire_shared(&nz[q >> 5]) & bit) != 0u);
-}
-
 __device__ __forceinline__ bool nonzero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) != 0ull; }
 
 // The guarded FP32 sampler's decision on num as a pair of FP32 words, -2 where it cannot
@@ -201,6 +194,19 @@ __device__ __noinline__ int decide_slow(double num, double u, const double *gc, 
     return comp;
 }
 
+// A question to the FP64 warp and its answer.  Out of line with decide_slow: an inlined
+// load that orders others made the chain's loop 4 % slower on 2,000 x 5,000.
+__device__ __noinline__ double ask_fp64_warp(volatile int *ask, const volatile double *told, int question, int *err)
+{
+    *ask = question;
+    unsigned spins = 0;
+    while (*ask != 0 && ++spins < (1u << 28))
+        ;
+    if (ld_acquire_shared(ask) != 0u)   // orders the answer after the word
+        atomicCAS(err, kDevOk, kDevTimeout);
+    return *told;
+}
+
 // --------------------------------------------------------------------------
 // The sweep of one chain over its G CTAs; sidx is this CTA's slice.
 template <int KM, bool PROF, bool CL>
@@ -212,13 +218,14 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     __shared__ int s_comp[kMaxSpec];
     __shared__ float2 s_ndf[kMaxSpec];    // num as a float pair
     __shared__ uint32_t s_nz[2][2];       // pair rounds: bits of the rows of the pair products in shared memory
-    __shared__ volatile int s_ev2[kMaxSpec + 1];  // the FP64 warp's progress over them
     __shared__ double s_Td;               // dense: the residual total
     __shared__ float2 s_Tf;               // the residual total or the running sum as a float pair
     __shared__ volatile int s_ask;        // the chain's question to the FP64 warp: events before it << 8, marker + 1
     __shared__ volatile double s_told;    // and its answer: the marker's num
     __shared__ volatile int s_ev[kMaxSpec + 1];   // changes of the round in order, for the FP64 warp
-    __shared__ double s_dB[kMaxSpec];
+    // beta_old - beta_new of the changes from the FP64 warp, kNoChange until then: the word
+    // is the value, so its reader needs no other
+    __shared__ volatile long long s_dB[kMaxSpec];
     __shared__ int s_ci[kMaxSpec];
     __shared__ __align__(16) long long s_d[kMaxSpec][4];
     __shared__ long long s_T[2];          // dense: the residual total, T = s_T[1] 2^30 + s_T[0]
@@ -297,9 +304,12 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     };
     const int nblocks = (int)((a.M + B - 1) / B);
     // pair products: only the rows of markers that are sure or likely to change are
-    // fetched ahead; another marker's row is fetched when its num is known, or
-    // read from L2 when it changes.  All rows would be 16 KB per CTA and round, half
-    // of what 152 CTAs then read from L2 during the exchange.
+    // fetched, ahead of their round; another marker's row is read from L2 when it
+    // changes.  All rows would be 16 KB per CTA and round, half of what 152 CTAs then read
+    // from L2 during the exchange.  (Fetching the rows of the markers that may change
+    // once their num is known, during the round, was 0.2 % faster at 2,000 x 5,000 and 0.8 %
+    // slower at 100,000 x 100,000, before the loads that its arrival needs to be ordered,
+    // which cost 5 % and 1 %.)
     auto issue_gram = [&](int upto) {
         if (!pairs)
             return;
@@ -345,7 +355,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
         gdf[i] = v;
     }
     for (int i = tid; i <= kMaxSpec; i += kRT)
-        s_ev[i] = s_ev2[i] = 0;
+        s_ev[i] = 0;
     if (tid == 0)
         s_ask = 0;
     if (!CL)
@@ -496,6 +506,8 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     while (start < M32) {
         cp_async_wait_all();
         __syncthreads();
+        if (tid < kMaxSpec)
+            s_dB[tid] = kNoChange;
         // pair rounds stay inside a block of B positions, whose products they use: blk, from
         // position off (not 0 after a change whose row was not formed)
         const unsigned blk = start / (unsigned)B;
@@ -689,7 +701,6 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 }
             }
             long long L = 0, H2 = 0, mL = 0, mH = 0;
-            bool cand = false;
             if (m < nb) {
                 fetch(m, 0, L, H2);
                 if (msum)
@@ -708,22 +719,11 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 }
                 df_add(nh, nl, ch, cl);
                 s_ndf[m] = make_float2(nh, nl);
-                cand = rc.beta_old == 0.0 && num_sq(nh, nl) > rc.s0;
                 if (warp == 2)
                     wmark(8);
             }
             __syncwarp();
             asm volatile("bar.sync 1, 96;" ::: "memory");
-            // the rows of the pair products of the markers that may change now
-            const unsigned rows = pairs && a.rall ? __ballot_sync(0xffffffffu, cand) : 0u;
-            const double *grow = a.rgram + (size_t)blk * gn;
-            double *gr = reinterpret_cast<double *>(smem + plan.gram + (blk & 1u) * gslot);
-            for (unsigned k = rows; k; k &= k - 1u) {
-                const int p = off + __ffs(k) - 1 + 32 * (warp - 2), base = p * (2 * B - p - 1) / 2;
-                for (int t = lane; t < B - 1 - p; t += 32)
-                    cp_async8(gr + base + t, grow + base + t);
-            }
-            cp_async_commit();
             // num in FP64, for the warp that follows the chain
             if (m < nb) {
                 const double at = -(rc.s * rc.m);
@@ -735,14 +735,6 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             }
             __syncwarp();
             asm volatile("bar.sync 2, 96;" ::: "memory");
-            cp_async_wait_all();
-            __syncwarp();
-            if (lane == 0 && rows) {
-                __threadfence_block();
-                const unsigned long long m = (unsigned long long)rows << (off + 32 * (warp - 2));
-                atomicOr(&s_nz[blk & 1u][0], (unsigned)m);
-                atomicOr(&s_nz[blk & 1u][1], (unsigned)(m >> 32));
-            }
             if (warp == 3) {
                 // the moves of every change per 2-bit code, as the FP64 warp finishes them
                 for (int u = 0;; ++u) {
@@ -753,10 +745,14 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     // (genotype - mean) scale; missing genotypes apart
                     const double x = up * (lane == 1 ? (dense ? rp.x : 0.0)
                                                      : __dmul_rn(__dsub_rn(lane == 0 ? 2.0 : lane == 2 ? 1.0 : 0.0, rp.m), rp.s));
-                    wait_event(&s_ev2[u]);
-                    ld_acquire_shared(&s_ev2[u]);   // orders s_dB after the word
+                    long long dB;
+                    unsigned spins = 0;
+                    while ((dB = s_dB[u]) == kNoChange && ++spins < (1u << 28))
+                        ;
+                    if (dB == kNoChange)
+                        atomicCAS(a.err, kDevOk, kDevTimeout);
                     if (lane < 4) {
-                        const double d = __dmul_rn(s_dB[u], x);   // up is a power of two
+                        const double d = __dmul_rn(__longlong_as_double(dB), x);   // up is a power of two
                         // |d| < 2^62, by its exponent
                         const bool ok = ((unsigned)__double2hiint(d) & 0x7FF00000u) < (1085u << 20);
                         range = range || !ok;
@@ -786,10 +782,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             }
             const double *gr = reinterpret_cast<const double *>(smem + plan.gram + (blk & 1u) * gslot);
             const double *grow = a.rgram + (size_t)blk * gn;
-            // rows that were in shared memory before the round, as bits; those that arrive
-            // during it are looked up
             const uint32_t *nz = s_nz[blk & 1u];
-            const uint32_t nz0 = nz[0], nz1 = nz[1];
             __syncwarp();
             asm volatile("bar.sync 1, 96;" ::: "memory");
             mark(2);
@@ -808,15 +801,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             // chain reaches it; the markers before it stay in component 0.
             int nchg = 0, fin = nb, pos = 0;
             // num of marker p after the changes so far, from the FP64 warp, on one lane
-            auto ask_num = [&](int p) -> double {
-                s_ask = (nchg << 8) | (p + 1);
-                unsigned spins = 0;
-                while (s_ask != 0 && ++spins < (1u << 28))
-                    ;
-                if (ld_acquire_shared(&s_ask) != 0u)   // orders the answer after the word
-                    atomicCAS(a.err, kDevOk, kDevTimeout);
-                return s_told;
-            };
+            auto ask_num = [&](int p) { return ask_fp64_warp(&s_ask, &s_told, (nchg << 8) | (p + 1), a.err); };
             if (a.rmode == kRoundAsync) {
                 // every marker is decided on the residual before the batch
 #pragma unroll 1
@@ -857,7 +842,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 bool last = !pairs;
                 if (pairs) {
                     const int q = off + p;
-                    const bool here = row_here(nz, nz0, nz1, q, a.rall != 0);
+                    const bool here = ((nz[q >> 5] >> (q & 31)) & 1u) != 0u;
                     last = !here && !a.rall;
                     const double *row = (here ? gr : grow) + q * (2 * B - q - 1) / 2 - p - 1;
                     if (!last && lane > p && lane < nb)
@@ -928,7 +913,6 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             const double *gr = reinterpret_cast<const double *>(smem + plan.gram + (blk & 1u) * gslot);
             const double *grow = a.rgram + (size_t)blk * gn;
             const uint32_t *nz = s_nz[blk & 1u];
-            const uint32_t nz0 = nz[0], nz1 = nz[1];
             __syncwarp();
             asm volatile("bar.sync 2, 96;" ::: "memory");
             wstart();
@@ -942,7 +926,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             for (;; ++nchg) {
                 int ev;
                 unsigned spins = 0;
-                while ((ev = s_ev[nchg]) == 0 && ++spins < (1u << 28)) {   // the word is all it says
+                while ((ev = s_ev[nchg]) == 0 && ++spins < (1u << 28)) {
                     const int ask = s_ask;
                     if (ask != 0 && ((ask - 1) & 31) == lane && ask >> 8 == nchg) {
                         s_told = ((ask - 1) & 32) ? num[1] : num[0];
@@ -965,16 +949,14 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                                               : comp == 0 ? 0.0 : rc.beta_old;
                     dB = rc.beta_old - b;
                     s_beta[p] = b;
-                    s_dB[nchg] = dB;
+                    s_dB[nchg] = __double_as_longlong(dB);
                     s_ci[nchg] = p;
-                    __threadfence_block();
-                    s_ev2[nchg] = 1;
                 }
                 if (!pairs)
                     continue;
                 dB = __shfl_sync(0xffffffffu, dB, p & 31);
                 const int q = off + p;
-                const bool here = row_here(nz, nz0, nz1, q, a.rall != 0);
+                const bool here = ((nz[q >> 5] >> (q & 31)) & 1u) != 0u;
                 if (!here && !a.rall)
                     continue;   // the round ends here
                 const double *row = (here ? gr : grow) + q * (2 * B - q - 1) / 2 - p - 1;
@@ -1011,7 +993,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
             a.comp_out[rc.j] = c;
         }
         if (tid <= nchg)
-            s_ev[tid] = s_ev2[tid] = 0;
+            s_ev[tid] = 0;
         if (nchg) {
             if (dense && warp == kRW - 1) {
                 // the residual total, exactly: individuals per code times the code's move
@@ -1043,7 +1025,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                 double es = s_es;
                 for (int u = 0; u < nchg; ++u) {
                     const RoundRec &rc = rec[(start + s_ci[u]) & Rm];
-                    es += s_dB[u] * ((rc.x - rc.m * (double)a.N) * rc.s);
+                    es += __longlong_as_double(s_dB[u]) * ((rc.x - rc.m * (double)a.N) * rc.s);
                 }
                 s_es = es;
                 float fh, fl;

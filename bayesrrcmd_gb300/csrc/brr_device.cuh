@@ -187,6 +187,24 @@ __device__ __forceinline__ void df_add(float &hi, float &lo, float bh, float bl)
     lo = __fsub_rn(e, __fsub_rn(hi, s));
 }
 
+// Magnitude of v as the FP32 value next to it towards zero, by integer operations (an
+// FP64 instruction takes 16 clocks of an SM); zero below 2^-126, infinity from 2^127 on
+// and where v is not finite.
+__device__ __forceinline__ float float_below(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned top = (unsigned)(b >> 32) & 0x7FF00000u;
+    return top < (897u << 20)    ? 0.f
+           : top >= (1150u << 20) ? __int_as_float(0x7F800000)
+                                  : __uint_as_float(((unsigned)(b >> 29) + 0x40000000u) & 0x7FFFFFFFu);
+}
+
+// Bits of a magnitude: they order as the values do.
+__device__ __forceinline__ unsigned long long magnitude_bits(double v)
+{
+    return (unsigned long long)__double_as_longlong(v) & ~(1ull << 63);
+}
+
 // Split an FP64 value into a normalised double-float pair.
 __device__ __forceinline__ void df_from_double(double v, float &hi, float &lo)
 {

@@ -186,10 +186,10 @@ __device__ __noinline__ int decide_pair(float nh, float nl, float uf, const floa
 template <int KM>
 __device__ __noinline__ int decide_slow(double num, double u, const double *gc, const float *gcf, int K)
 {
-    float nh, nl;
+    float nh, nl, a0;
+    int comp;
     df_from_double(num, nh, nl);
-    int comp = decide_pair<KM>(nh, nl, __double2float_rn(u), gcf, K);
-    if (comp == -2)
+    if (!pick_f32<KM>(nh, nl, __double2float_rn(u), gcf, K, comp, a0))
         comp = pick_marker<true, KM>(num, u, 0.0, 0.0, gc, K).comp;
     return comp;
 }
@@ -231,6 +231,7 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     __shared__ long long s_T[2];          // dense: the residual total, T = s_T[1] 2^30 + s_T[0]
     __shared__ double s_es;               // sparse: the running residual sum
     __shared__ double s_red[kRW][2];
+    __shared__ float s_sum[kRW];
     __shared__ int s_nchg, s_fin, s_abort;
     __shared__ unsigned long long s_acc[kMaxSpec + 1][4];   // one CTA: the round's sums
     __shared__ __align__(8) uint64_t s_xbar[2];
@@ -364,19 +365,22 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     for (int i = tid; i < (kMaxSpec + 1) * 4; i += kRT)
         (&s_acc[0][0])[i] = 0ull;
     {
-        double mx = 0.0, sa = 0.0;
+        unsigned long long mx = 0ull;
+        float sa = 0.f;
         for (int i = tid; i < a.n_emax; i += kRT) {
-            mx = fmax(mx, a.emax[i]);
-            sa += a.emax[a.n_emax + i];
+            const unsigned long long b = magnitude_bits(a.emax[i]);
+            mx = b > mx ? b : mx;
+            sa += float_below(a.emax[a.n_emax + i]);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const unsigned long long b = __shfl_xor_sync(0xffffffffu, mx, o);
+            mx = b > mx ? b : mx;
             sa += __shfl_xor_sync(0xffffffffu, sa, o);
         }
         if (lane == 0) {
-            s_red[warp][0] = mx;
-            s_red[warp][1] = sa;
+            s_red[warp][0] = __longlong_as_double((long long)mx);
+            s_sum[warp] = sa;
         }
     }
     if (tid == 0) {
@@ -404,20 +408,22 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
     int sc;
     bool coarse;
     {
-        double mx = 0.0, sa = 0.0;
+        unsigned long long mx = 0ull;
+        float sa = 0.f;
         for (int w = 0; w < kRW; ++w) {
-            mx = fmax(mx, s_red[w][0]);
-            sa += s_red[w][1];
+            const unsigned long long b = magnitude_bits(s_red[w][0]);
+            mx = b > mx ? b : mx;
+            sa += s_sum[w];
         }
-        // bounds of the residual after mu_new is subtracted: emax < 2^e2, and its mean
-        // magnitude from below
-        const double emax = fabs(a.mu_new) + mx, mean = sa / (double)a.N - fabs(a.mu_new);
-        auto exponent = [](double v) { return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7FF) - 1023; };
-        const int e2 = exponent(emax) + 1;
-        const int need = (a.form == BRR_FORM_FP64 ? 53 : 49) - exponent(mean);
+        // bounds of the residual after mu_new is subtracted: its largest magnitude, below
+        // 2^e2, and its mean magnitude
+        const double emax = fabs(a.mu_new) + __longlong_as_double((long long)mx);
+        const float mean = __fdividef(sa, (float)a.N) - float_below(a.mu_new);
+        const int e2 = (int)(magnitude_bits(emax) >> 52) - 1022;
+        const int need = (a.form == BRR_FORM_FP64 ? 53 : 49) - ((int)(__float_as_uint(mean) >> 23) - 127);
         const int most = min(61 - e2, 100);   // E below 2^61: one bit of headroom
         sc = max(min(59 - e2, most), min(need, most));
-        coarse = !(mean > 0.0) || !(emax < 1e290) || sc < need;   // also where the sums are not finite
+        coarse = !(mean > 0.f && mean < INFINITY) || sc < need;
         if (coarse)
             sc = 0;
     }

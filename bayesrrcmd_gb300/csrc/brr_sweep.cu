@@ -87,12 +87,21 @@ __global__ void k_gather(int form, int kind, const uint32_t *__restrict__ order,
 }
 
 // updateMu, first half: eps += mu_old, and per-block sum(eps) (src/DenseBayesRRmz.cpp:38-39), max |eps|
-// and sum |eps| (emax, and nblocks further).
+// and sum |eps| (emax, and nblocks further; the sum in FP32 from below).
 __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, double mu_old, double *eps,
                                                       float *eps_hi, float *eps_lo, double *part, double *emax)
 {
-    __shared__ double red[kThreads / 32][3];
-    double s = 0.0, mx = 0.0, sa = 0.0;
+    __shared__ double red[kThreads / 32];
+    __shared__ unsigned long long red_mx[kThreads / 32];
+    __shared__ float red_sa[kThreads / 32];
+    double s = 0.0;
+    unsigned long long mx = 0ull;
+    float sa = 0.f;
+    auto magnitude = [&](double e) {
+        const unsigned long long b = magnitude_bits(e);
+        mx = b > mx ? b : mx;
+        sa += float_below(e);
+    };
     float mh, ml;
     df_from_double(mu_old, mh, ml);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
@@ -100,8 +109,7 @@ __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, doubl
             const double e = __dadd_rn(eps[i], mu_old);
             eps[i] = e;
             s += e;
-            mx = fmax(mx, fabs(e));
-            sa += fabs(e);
+            magnitude(e);
         } else {
             float h = eps_hi[i], l = eps_lo[i];
             df_add(h, l, mh, ml);
@@ -109,32 +117,32 @@ __global__ void __launch_bounds__(kThreads) k_mu_prep(int form, int64_t N, doubl
             eps_lo[i] = l;
             const double e = (double)h + (double)l;
             s += e;
-            mx = fmax(mx, fabs((double)h) + fabs((double)l));
-            sa += fabs(e);
+            magnitude(e);
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, o);
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const unsigned long long b = __shfl_xor_sync(0xffffffffu, mx, o);
+        mx = b > mx ? b : mx;
         sa += __shfl_xor_sync(0xffffffffu, sa, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        red[threadIdx.x >> 5][0] = s;
-        red[threadIdx.x >> 5][1] = mx;
-        red[threadIdx.x >> 5][2] = sa;
+        red[threadIdx.x >> 5] = s;
+        red_mx[threadIdx.x >> 5] = mx;
+        red_sa[threadIdx.x >> 5] = sa;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0.0, m = 0.0, ta = 0.0;
+        double t = 0.0;
         for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-            t += red[q][0];
-            m = fmax(m, red[q][1]);
-            ta += red[q][2];
+            t += red[q];
+            mx = red_mx[q] > mx ? red_mx[q] : mx;
+            sa = q ? sa + red_sa[q] : red_sa[q];
         }
         part[blockIdx.x] = t;
-        emax[blockIdx.x] = m;
-        emax[gridDim.x + blockIdx.x] = ta;
+        emax[blockIdx.x] = __longlong_as_double((long long)mx);
+        emax[gridDim.x + blockIdx.x] = (double)sa;
     }
 }
 

@@ -205,13 +205,6 @@ __device__ __forceinline__ int limb_row(int c, int l) { return 4 * c + l; }
 __device__ __forceinline__ unsigned short h_bits(int v) { return __half_as_ushort(__int2half_rn(v)); }
 __device__ __forceinline__ int h_int(unsigned short b) { return __half2int_rn(__ushort_as_half(b)); }
 
-// Genotype of a 2-bit BED code {0: 2, 1: missing, 2: 1, 3: 0}.
-__device__ __forceinline__ unsigned short g_half(unsigned code)
-{
-    // FP16 bit patterns of 2.0, 0.0 (missing genotypes are rejected before), 1.0, 0.0
-    return code == 0u ? (unsigned short)0x4000 : (code == 2u ? (unsigned short)0x3C00 : (unsigned short)0);
-}
-
 struct BatchPlan {
     unsigned off_g, off_e, off_w, off_p, total;
     unsigned sbo_g;      // stride between 8-marker groups of g (= kext/8 * 128)

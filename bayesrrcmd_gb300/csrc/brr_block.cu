@@ -469,32 +469,6 @@ __global__ void k_block_finish(int64_t M, const int *__restrict__ err, const Blo
         comp[r.j] = c;
 }
 
-// One halving exchange of a warp's reduce-scatter over double-float sums:
-// lanes of the lower half (upper false) keep entries [0, H), the others
-// [H, 2H), each adding the partner's copy; the kept sums move to [0, H).
-template <int H>
-__device__ __forceinline__ void df_rs_step(float (&h)[kMaxSpec / 8], float (&l)[kMaxSpec / 8], bool upper, int off)
-{
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-        const float kh = upper ? h[i + H] : h[i], kl = upper ? l[i + H] : l[i];
-        const float sh = upper ? h[i] : h[i + H], sl = upper ? l[i] : l[i + H];
-        const float rh = __shfl_xor_sync(0xffffffffu, sh, off);
-        const float rl = __shfl_xor_sync(0xffffffffu, sl, off);
-        h[i] = kh;
-        l[i] = kl;
-        df_add(h[i], l[i], rh, rl);
-    }
-}
-
-// Butterfly step of a double-float all-reduce (both partners get the same sum).
-__device__ __forceinline__ void df_xor_add(float &h, float &l, int off)
-{
-    const float rh = __shfl_xor_sync(0xffffffffu, h, off);
-    const float rl = __shfl_xor_sync(0xffffffffu, l, off);
-    df_add(h, l, rh, rl);
-}
-
 // One CTA of 15 warps per SM (12 dot warps, the resolve, input and chore warps) at
 // 128 registers a thread.  PROF: the variant that counts phase cycles on the first
 // CTA (the clock reads constrain the code's scheduling, so the plain variant has

@@ -338,11 +338,14 @@ int build_ragged_lists(brr_ctx &c)
 }  // namespace
 
 // FP32C chains of at least this many markers take pair-resolved rounds of 64 (see
-// use_pair_rounds).  Measured, ragged, ms per iteration with 64 markers and pair
-// products / 32 and pair products / 32 and rounds that end at a change: N 2,000 x
-// M 4,000 0.49 / 0.65 / 0.85 past the burn-in and 1.58 / 1.75 / 6.6 in it, N 20,000 x
-// M 50,000 4.6 / 6.8 / 8.2, N 100,000 x M 8,000 1.08 / 1.37 / 1.44.  Below it the
-// three differ by about a tenth of a millisecond and keep the rounds of 32.
+// use_pair_rounds).  Measured, ragged, ms per sweep with 64 markers and pair
+// products / 32 and pair products / 32 and rounds that end at a change: N 20,000 x
+// M 50,000 4.6 / 6.8 / 8.2, N 100,000 x M 8,000 1.08 / 1.37 / 1.44, both past the
+// burn-in.  The line is where the form's documented widths change, not where the curves
+// cross: below it the order is the same, N 2,000 x M 4,000 1.60 / 1.78 / 7.9 in the
+// burn-in and 0.94 / 1.12 / 4.0 with 570 effects, N 20,000 x M 1,000 0.46 / 0.49 / 2.1
+// and 0.20 / 0.24 / 0.39 (36 effects), N 2,000 x M 500 0.26 / 0.27 / 1.05; dense markers
+// without the Gram-blocked sweep 1.40 / 1.58 / 8.4 at N 2,000 x M 4,000.
 constexpr int64_t kWidePairM = 4096;
 
 // Whether the whole-round sweep fits this chain's slices at its round width

@@ -3,8 +3,8 @@
 //
 // Replaces BayesRBase::processColumn (src/BayesRBase.cpp:287-392) over the
 // dense kernel (src/densebayesrkernel.cpp:10-20) for whole sweeps, like the
-// restart sweep of brr_sweep.cu, with the precomputed marker Gram matrix
-// (packed lower triangle, FP64, brr_gram.cu).
+// whole-round sweep of brr_round.cu, with the precomputed marker Gram matrix
+// (packed lower triangle, double-float pairs, brr_gram.cu).
 //
 // The sweep order is cut into blocks of B consecutive markers.  One CTA per SM
 // owns a slice of individuals and keeps its residual slice in shared memory in
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
     __shared__ int s_cp_issued;
     // resolve warp <-> other warps: GO(q) on s_mb[q & 1] (one arrival per thread: the dot
     // threads after block q-2's update, the input warp after block q's inputs,
-    // the chore warp after block q-2's outputs), RESOLVED(q) on s_mb[2 + (q & 1)]
+    // the chore warp after its Gram loads), RESOLVED(q) on s_mb[2 + (q & 1)]
     // (the resolve warp's 32 lanes after block q's decisions)
     __shared__ __align__(8) uint64_t s_mb[4];
 
@@ -1232,7 +1232,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
                 // Gram entries of block r+3 (loaded in the previous iteration) and
                 // the zeroed accumulators of block r+4, signalled to the dot warps
                 // before their arrival at barrier r+2; then the Gram loads of
-                // block r+4 and the outputs of block r-1
+                // block r+4
                 auto issue_bulk_next = [&]() {
                     if (lane == 0 && r + 1 < nblk) {
                         const int q = r + 1;
@@ -1307,7 +1307,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_sweep_block(SweepArgs a)
         }
     }
     __syncthreads();
-    // the last block: residual update and outputs
+    // the last block's residual update
     if (!s_abort && r == nblk) {
         if (dw >= 0)
             apply_update(nblk - 1);

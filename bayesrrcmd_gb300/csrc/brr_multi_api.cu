@@ -1,13 +1,14 @@
 // C ABI of the uneven batch: independent regressions of different sizes
 // (each its own genotypes, phenotype, seed, marker kind) swept together by one
-// cooperative launch of k_sweep_multi per iteration, each instance on its own
-// group of CTAs.  Per instance the iteration is the single-chain one
-// (BayesRBase::runGibbs loop body, src/BayesRBase.cpp:186-247) through the
-// phases of brr_ctx.h.
+// cooperative launch per iteration, of k_round_multi or, where an instance cannot run
+// the whole-round sweep, k_sweep_multi, each instance on its own group of CTAs.  Per
+// instance the iteration is the single-chain one (BayesRBase::runGibbs loop body,
+// src/BayesRBase.cpp:186-247) through the phases of brr_ctx.h.
 //
 // The autotuner chooses, per instance, the round width (markers resolved per
 // grid round) and the number of CTAs: it runs real iterations, reads each
 // instance's sweep time from the device timer, keeps the fastest round width
+// of 8, 16 and 32 (64, with which a whole-round instance starts, is not tried again)
 // and then moves CTAs to the instances that finish last until the times are
 // balanced (an instance's slices must fit shared memory, which bounds its
 // CTAs from below).  Slicing and round width change only the order of
@@ -390,7 +391,10 @@ int brr_multi_create(const brr_config *cfgs, int32_t n, brr_multi **out)
     // first split of the SMs: at least what the slices need, the rest by N*M.
     // The whole-round sweep where every instance fits it, else the restart sweep;
     // when the default round widths need more CTAs than there are SMs, every
-    // instance starts at the narrowest width (the smallest code ring)
+    // instance starts at the narrowest width (the smallest code ring).  Narrow whole
+    // rounds come before the restart sweep: one chain on all SMs, 1,500 markers, ms
+    // per sweep of the two, N 750,000 (rounds of 32) dense 1.5 / 17 FP64 and ragged 1.6 /
+    // 39 FP64, 1.6 / 58 FP32C; N 900,000 (rounds of 16) dense FP64 1.6 / 18
     std::vector<double> work(n);
     std::vector<int> mins(n), maxs(n), G, widths(n);
     const int narrowest = 8;

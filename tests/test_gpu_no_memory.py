@@ -55,6 +55,55 @@ CHAIN = """
             ch.close()
 """
 
+TIMEOUT = """
+    N, M = 1_500, 150
+    bed, y = data(N, M, 3)
+    for kw in (dict(), dict(cluster=8)):
+        ch = gpu.Chain(gpu.ChainConfig(N=N, M=M, S=S1, seed=7, **kw))
+        ch.pack_bed(bed)
+        ch.set_phenotype(y)
+        budget(0)
+        ch.init()
+        budget(-1)
+        ch.set_wait_limit(50_000_000, 1)
+        try:
+            ch.iterate(1)
+            raise SystemExit("no timeout")
+        except gpu.BrrError as e:
+            assert e.code == -4
+        ch.set_wait_limit(2_000_000_000, 0)
+        ch.init()
+        oc = O.OracleChain(bed, N, y, S1, kind=0, seed=7)
+        for it in range(2):
+            ch.iterate(1)
+            oc.iterate(it)
+        compare(ch.state(), oc.state(), 1e-10)
+        assert ch.timing()[2] > -(-M // 64) + 10
+        ch.close()
+    m = gpu.Multi([gpu.ChainConfig(N=N, M=M, S=S1, seed=3, chain=k) for k in range(2)])
+    for k in range(2):
+        m.pack_bed(k, bed)
+        m.set_phenotype(k, y)
+    budget(0)
+    m.init()
+    budget(-1)
+    m.set_wait_limit(50_000_000, 1, instance=1)
+    try:
+        m.iterate(1)
+        raise SystemExit("no timeout")
+    except gpu.BrrError as e:
+        assert e.code == -4
+    m.set_wait_limit(2_000_000_000, 0)
+    m.init()
+    m.iterate(2)
+    for k in range(2):
+        oc = O.OracleChain(bed, N, y, S1, kind=0, seed=3, chain=k)
+        oc.iterate(0)
+        oc.iterate(1)
+        compare(m.state(k), oc.state(), 1e-10)
+    m.close()
+"""
+
 MULTI = """
     shapes = [(2_500, 300, gpu.KIND_DENSE), (1_203, 150, gpu.KIND_RAGGED), (5_000, 100, gpu.KIND_EIGEN)]
     probs = [(N, M, kind) + data(N, M, 40 + k) for k, (N, M, kind) in enumerate(shapes)]
@@ -107,3 +156,7 @@ def test_fp32c_chain(gpu_lib, lib, calls):
 @pytest.mark.parametrize("calls", [0, 3, 6, 11, 17])
 def test_multi(gpu_lib, lib, calls, form, rtol):
     run(MULTI, lib, calls=calls, form=form, rtol=rtol)
+
+
+def test_waits_of_the_restart_sweep_run_out_and_the_chain_recovers(gpu_lib, lib):
+    run(TIMEOUT, lib)

@@ -24,7 +24,7 @@
 // 2^-s <= 2^(floor(log2 mean) - 53) in the FP64 form, 2^(... - 49) in the FP32C form.
 // With normal residuals of variance 1 the largest of 100,000 is 4.5, 2^-s is 2^-56 and
 // 2^-54 would do; one bit of headroom instead of three allows for a largest |eps| of
-// 100 to 200 means.  Where no grid is fine enough (an outlier further out, values that
+// 128 to 256 means (FP32C: 2,048 to 4,096).  Where no grid is fine enough (an outlier further out, values that
 // are not finite), and where a value outgrows the headroom during the sweep, the
 // sweep ends with the range status and the host runs the restart sweep instead; the
 // residual in memory is only replaced by a sweep that ended well.

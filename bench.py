@@ -336,10 +336,9 @@ def run_uneven(lib, gpu, torch, device, steps, tune_rounds, scale=1.0):
     seed = SEED + 11
     N, M, h2 = uneven_instances(seed, scale)
     # each instance's genotypes and phenotype; its kind, dense or ragged, from
-    # its own packed genotype counts: the ragged sweep reads 2 bytes (a
-    # slice-local index) per listed genotype (ones, twos, missing), the dense
-    # sweep N/4 bytes per marker, so ragged storage is chosen when fewer than one
-    # genotype in eight is listed
+    # its own packed genotype counts: ragged where fewer than one genotype in
+    # eight is listed (one, two or missing), so that a list of 2-byte indices is
+    # smaller than the N/4 bytes of codes
     rng = np.random.default_rng(seed + 2)
     beds, ys, kinds, listed = [], [], [], []
     for i in range(len(N)):
@@ -490,11 +489,11 @@ def cpu_rate(bed, N, y, kind, iters):
 
 def run_ragged(lib, gpu, torch, device, steps, warmup, cpu=True):
     """C2: the FP64 and FP32C ragged chains, their rates and the roofline on
-    the index bytes; C1: the plain FP64 dense chain; the CPU restatement's
+    the code bytes; C1: the plain FP64 dense chain; the CPU restatement's
     rate on both beside them."""
     d_bed = synth_parts(torch, gpu, lib, device, R_N, [(R_RARE, 0.001, 0.05), (R_M - R_RARE, 0.05, 0.5)], SEED + 21,
                         0.01)
-    y, counts = synth_phenotype(gpu, lib, device, d_bed, R_N, R_M, 500, 0.5, SEED + 21)
+    y, _ = synth_phenotype(gpu, lib, device, d_bed, R_N, R_M, 500, 0.5, SEED + 21)
     f64 = time_chain(gpu, lib, device, d_bed, R_N, R_M, y, gpu.KIND_RAGGED, gpu.FORM_FP64, steps, warmup, SEED)
     # the first timed iterations lie in the chain's burn-in, where about one
     # marker in six changes its effect; the late ones in its stationary phase
@@ -502,10 +501,10 @@ def run_ragged(lib, gpu, torch, device, steps, warmup, cpu=True):
                      late=R_LATE, phases=True)
     f32r = time_chain(gpu, lib, device, d_bed, R_N, R_M, y, gpu.KIND_RAGGED, gpu.FORM_FP32C, steps, warmup, SEED,
                       pair_rounds=-1, late=R_LATE)
-    # algorithmic bytes of a sweep: 4 bytes per listed genotype (ones, twos, missing)
-    idx_bytes = 4.0 * float(counts[:, 1:4].sum())
+    # algorithmic bytes of a sweep: the 2-bit codes of every marker
+    code_bytes = R_M * (R_N / 4.0)
     hbm, _ = peaks()
-    achieved = idx_bytes / (f32["sweep_ms"] / 1e3) / 1e9
+    achieved = code_bytes / (f32["sweep_ms"] / 1e3) / 1e9
     host_bed = d_bed.cpu().numpy().reshape(R_M, -1)
     del d_bed
     c1_bed = synth_parts(torch, gpu, lib, device, C1_N, [(C1_M, 0.05, 0.5)], SEED + 31, 0.0)
@@ -529,8 +528,8 @@ def run_ragged(lib, gpu, torch, device, steps, warmup, cpu=True):
         "speedup_fp32c_vs_plain": f32["rate"] / f64["rate"],
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": None, "kernel": "k_round (ragged, FP32C, pair-resolved rounds)",
-                     "algorithmic_bytes_per_launch": idx_bytes,
-                     "note": "4 bytes per listed genotype (ones, twos, missing) per sweep"},
+                     "algorithmic_bytes_per_launch": code_bytes,
+                     "note": "2-bit codes of every marker, once per sweep"},
         "matched_error": {"beta_max_abs_diff_vs_plain": float(np.abs(f32["beta"] - f64["beta"]).max()),
                           "component_mismatches_vs_plain": int(np.count_nonzero(f32["comp"] != f64["comp"])),
                           "sigmaE_rel_diff_vs_plain": abs(f32["sigmaE"] / f64["sigmaE"] - 1),

@@ -92,6 +92,15 @@ extern "C" {
 
 #define BRR_FORM_FP64 0      /* plain FP64 sweep: the drop-in */
 #define BRR_FORM_FP32C 1     /* FP32 compensated dots and residual, FP64 refresh */
+/* Between sweeps the residual is FP64 (FP32C: a pair of FP32 words).  The whole-round
+ * sweep of either form holds it in 64-bit fixed point, on one grid for all individuals
+ * that is no coarser than 2^(e - 53) (FP32C: 2^(e - 49)), e = floor(log2 of the mean of
+ * |eps|): the stored spacing there or finer.  That takes a largest |eps| below 128 to
+ * 256 means (FP32C: 2,048 to 4,096).  A sweep whose residual has no such grid, or outgrows
+ * it, runs as the restart sweep, which keeps it as stored: the same chain, one round
+ * per marker that changes.  BRR_ERR_RANGE then means that dot products left its
+ * range too, or a residual that is not finite; effects, components and residual are
+ * those before the sweep. */
 
 #define BRR_MAX_GROUPS 64
 #define BRR_MAX_K 16

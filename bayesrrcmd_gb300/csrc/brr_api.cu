@@ -981,6 +981,21 @@ int refresh_eps_impl(brr_ctx *c)
     return BRR_OK;
 }
 
+// The markers are packed.  Packed again under a running chain, the marker Gram and the
+// whole-round sweep's buffers follow them.
+int packed_markers(brr_ctx &c, bool running)
+{
+    c.packed = true;
+    drop_dev(c.d_gram);
+    if (!running)
+        return BRR_OK;
+    int rc = prepare_blocked(&c);
+    if (!rc)
+        rc = prepare_round(&c);
+    c.inited = rc == BRR_OK;
+    return rc;
+}
+
 }  // namespace
 
 // FP64 refresh when due, updateMu (dense src/DenseBayesRRmz.cpp:36-42, ragged
@@ -1229,6 +1244,9 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
         BRR_CUDA(cudaMemset(c.d_group, 0, sizeof(int32_t) * M));
         c.group.assign(M, 0);
     }
+    // until the markers are whole, a running chain is not
+    const bool running = c.inited;
+    c.inited = false;
     BRR_CUDA(cudaMemcpy(c.d_slice_lo, c.slice_lo.data(), sizeof(int32_t) * (c.G + 1), cudaMemcpyHostToDevice));
     BRR_CUDA(launch_pack_counts(d_bed, cf.N, M, c.d_codes, c.col_stride, c.d_counts, c.st));
     // totals of the counts, and the first marker that does not vary (0x7F7F7F7F: none)
@@ -1260,8 +1278,7 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
         choose_round(c);
         if (!c.round_ok)
             return fail(BRR_ERR_ARG, "the sweep kernel does not fit " + std::to_string(c.G) + " co-resident CTAs");
-        c.packed = true;
-        return c.inited ? prepare_round(&c) : BRR_OK;
+        return packed_markers(c, running);
     }
     // the sweep kernel must fit one CTA per slice on the GPU at once
     SweepArgs a{};
@@ -1276,17 +1293,14 @@ int brr_pack_bed_device(brr_ctx *ctx, const uint8_t *d_bed, int64_t nbytes)
             return fail(BRR_ERR_ARG, "a cluster of " + std::to_string(c.G) + " CTAs with " + std::to_string(smem) +
                                          " bytes of shared memory each cannot be scheduled");
         choose_round(c);
-        c.packed = true;
-        return c.inited ? prepare_round(&c) : BRR_OK;
+        return packed_markers(c, running);
     }
     const int per_sm = sweep_max_ctas_per_sm(cf.form, c.kind, smem);
     if (per_sm < 1 || (int64_t)per_sm * c.sms < c.G)
         return fail(BRR_ERR_ARG, "the sweep kernel does not fit " + std::to_string(c.G) +
                                      " co-resident CTAs (shared memory " + std::to_string(smem) + " bytes)");
     choose_round(c);
-    c.packed = true;
-    // markers packed again under a running chain: its sweep's buffers follow them
-    return c.inited ? prepare_round(&c) : BRR_OK;
+    return packed_markers(c, running);
 }
 
 int brr_get_marker_table(brr_ctx *ctx, double *table, int64_t *counts)

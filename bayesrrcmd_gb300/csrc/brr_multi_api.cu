@@ -229,6 +229,9 @@ int restart_again(brr_multi *m, const std::vector<int> &which, const std::vector
 int run_iteration(brr_multi *m)
 {
     const int n = m->n;
+    for (int i = 0; i < n; ++i)
+        if (!m->inst[i]->inited)
+            return api_fail(BRR_ERR_ARG, "instance " + std::to_string(i) + " is not initialised");
     for (int i = 0; i < n && m->round; ++i)
         if (!m->inst[i]->use_round()) {
             const int rc = take_restart(m);

@@ -881,7 +881,10 @@ __device__ __forceinline__ void round_body(const SweepArgs &a, const int sidx)
                     fin = p + 1;   // a restart round ends at its first change, a pair round at one without a row
                     break;
                 }
-                // beta_old - beta_new and its error, on the owner's lane
+                // beta_old - beta_new and its error, on the owner's lane.  With the truncation of
+                // G the roundings come to 3.0e-7 of the old effect, 4.8e-7 of z sd and 3.6e-7 of
+                // num / den; those of er itself, 2e-7 of it a change, stay inside the 1 % that its
+                // first term has over
                 float d = hi ? bo[1] : bo[0], e = fabsf(d);
                 if (comp > 0) {
                     const float4 k4 = gdf[g * kMaxK + comp];   // {sdk hi, lo, invden hi, lo}

@@ -175,7 +175,9 @@ int brr_ctx_destroy(brr_ctx *ctx);
 
 /* Pack a PLINK SNP-major BED payload (M columns of ceil(N/4) bytes, the 3-byte
  * magic header already removed) from host memory; the decode, genotype counts,
- * standardisation or ragged index lists all run on the device. */
+ * standardisation or ragged index lists all run on the device.  Packing again
+ * replaces the markers under a running chain, whose state stays; a packing that
+ * fails after its arguments were checked leaves the chain to be initialised again. */
 int brr_pack_bed(brr_ctx *ctx, const uint8_t *bed, int64_t nbytes);
 /* Same, from a device pointer: device or managed memory of the context's GPU
  * with nbytes to the end of its allocation, else BRR_ERR_ARG before any launch. */
